@@ -73,50 +73,58 @@ constexpr unsigned FULL = 0xffffffffu;
 /* one group-exchange buffer: two values per unit of the largest group
  * (128 units) and one flag word per warp, padded to 16-byte multiples */
 constexpr int XCH_BUF = 2 * 128 + 8;
-
+/* one buffer of warp_sum32 / warp_sum32x2: the 16 even and the 16 odd units'
+ * values of one or two vectors, each run padded by one double2 so that the
+ * runs a load reads at once start in different banks */
+constexpr int RED_RUN = 18, RED_BUF = 4 * RED_RUN;
 /* Shared-memory doubles per system (G warps, U units per lane, NMAX = 32 U G
- * units): one NMAX x (NMAX+1) matrix region (the operator W with the
- * shared-memory operator, the system's coupling matrix C with the
- * register-resident operator), six broadcast vectors, the group's exchange
- * buffers (G > 1), the system-scope arrays, the unit parameters when each
- * lane owns one unit (U = 1: in registers they crowd out the BiCG state) and
- * for the register-resident operator (U = G = 1) the operator W itself
- * (column-major, ld NMAX+1: its columns feed the transposed product). */
+ * units): one NMAX x (NMAX+1) matrix region (the operator W; with the
+ * register-resident operator, U = G = 1, the system's coupling matrix C and
+ * the part of W that A^T v reads), six broadcast vectors, the group's exchange buffers
+ * (G > 1) or the warp's reduction buffers, the system-scope arrays, and the unit
+ * parameters when each lane owns one unit (U = 1: in registers they crowd out
+ * the BiCG state). */
 template <int U, int G = 1>
 struct WarpSmem {
     static constexpr int NMAX = 32 * U * G;
+    static constexpr bool ONE = U == 1 && G == 1;   /* one warp, one unit per lane */
     static constexpr int LDW = NMAX + 1;
     static constexpr int W_DOUBLES = NMAX * LDW;
     static constexpr int VEC_DOUBLES = 6 * NMAX;
     static constexpr int XCH_DOUBLES = G > 1 ? 2 * XCH_BUF + 8 : 0; /* two buffers of two values per unit, vote words */
     static constexpr int SYS_DOUBLES = NSPa + NSAa + NISAa;  /* ints stored in double slots */
+    static constexpr int RED_DOUBLES = ONE ? 3 * RED_BUF : 0;   /* warp_sum32's buffers, two vectors by parity */
     static constexpr int UP_DOUBLES = U == 1 ? NMAX * NUPa : 0; /* unit parameters (one unit per lane) */
-    static constexpr int WT_DOUBLES = U == 1 && G == 1 ? NMAX * LDW : 0;  /* operator W of the register variants */
+    static constexpr int WT_DOUBLES = ONE ? NMAX * NMAX : 0;  /* each lane's column share of W */
     /* per-system stride rounded up to 256 bytes: every system's vectors stay
      * 16-byte aligned for the double2 broadcast loads */
+    static constexpr int K_DOUBLES = U == 1 ? 6 * UD * NMAX : 0;   /* stage derivatives (one unit per lane) */
     static constexpr int DOUBLES =
-        (W_DOUBLES + WT_DOUBLES + VEC_DOUBLES + XCH_DOUBLES + SYS_DOUBLES + UP_DOUBLES + 31) / 32 * 32;
+        (W_DOUBLES + WT_DOUBLES + VEC_DOUBLES + XCH_DOUBLES + RED_DOUBLES + SYS_DOUBLES + UP_DOUBLES + K_DOUBLES + 31) / 32 * 32;
     static constexpr int BYTES = DOUBLES * 8;
     static_assert(DOUBLES % 2 == 0 && W_DOUBLES % 2 == 0 && NMAX % 2 == 0,
                   "broadcast vectors must start on 16-byte boundaries");
 };
 
 /* Shared-memory layout of the shared-matrix variant (RHS = 3): one padded
- * copy of the launch's coupling matrix per CTA (leading dimension NMAX+2:
- * rows are read lane-consecutive, each lane's column is 16-byte aligned and
- * its double2 reads are conflict-free), then per system five broadcast
+ * copy of the launch's coupling matrix per CTA (one unit per lane: leading
+ * dimension NMAX+1 for the quads; more: NMAX+2, rows are read lane-consecutive,
+ * each lane's column is 16-byte aligned and its double2 reads are
+ * conflict-free), then per system five broadcast
  * vectors, the group's exchange buffers and the system-scope arrays. */
 template <int U, int G = 1>
 struct SharedCSmem {
     static constexpr int NMAX = 32 * U * G;
-    static constexpr int LDC = NMAX + 2;
+    static constexpr int LDC = U == 1 ? NMAX + 1 : NMAX + 2;   /* odd for the quads' 64-bit reads */
     static constexpr int C_DOUBLES = NMAX * LDC;
     static constexpr int XCH_DOUBLES = G > 1 ? 2 * XCH_BUF + 8 : 0;
     static constexpr int UP_DOUBLES = U == 1 ? NMAX * NUPa : 0; /* unit parameters (one unit per lane) */
-    static constexpr int WARP_DOUBLES = (5 * NMAX + XCH_DOUBLES + NSPa + NSAa + NISAa + UP_DOUBLES + 31) / 32 * 32;
+    static constexpr int K_DOUBLES = U == 1 ? 6 * UD * NMAX : 0;    /* stage derivatives (one unit per lane) */
+    static constexpr int WARP_DOUBLES =
+        (5 * NMAX + XCH_DOUBLES + NSPa + NSAa + NISAa + UP_DOUBLES + K_DOUBLES + 31) / 32 * 32;
     static constexpr int C_BYTES = C_DOUBLES * 8;
     static constexpr int WARP_BYTES = WARP_DOUBLES * 8;
-    static_assert(LDC % 2 == 0 && C_DOUBLES % 2 == 0 && WARP_DOUBLES % 2 == 0, "16-byte alignment");
+    static_assert(C_DOUBLES % 2 == 0 && WARP_DOUBLES % 2 == 0, "16-byte alignment");
 };
 
 /* Shared-memory layout of the banded variant (RHS = 7, one unit per lane, G
@@ -129,10 +137,18 @@ template <int G>
 struct BandSmem {
     static constexpr int NMAX = 32 * G;
     static constexpr int XCH_DOUBLES = G > 1 ? 2 * XCH_BUF + 8 : 0;
+    static constexpr int RED_DOUBLES = G == 1 ? 2 * RED_BUF : 0;   /* warp_sum32's buffers */
     __host__ __device__ static constexpr int diagonals(int bw) { return 2 * bw + 1 < NMAX ? 2 * bw + 1 : NMAX; }
     __host__ __device__ static constexpr int doubles(int bw) {
-        return (2 * diagonals(bw) * NMAX + 6 * NMAX + XCH_DOUBLES + NSPa + NSAa + NISAa + NMAX * NUPa + 31) / 32 * 32;
+        return (2 * diagonals(bw) * NMAX + 6 * NMAX + XCH_DOUBLES + RED_DOUBLES + NSPa + NSAa + NISAa + NMAX * NUPa + 6 * UD * NMAX + 31) /
+               32 * 32;
     }
+};
+
+/* a compile-time constant as a function argument */
+template <int V>
+struct Const {
+    static constexpr int value = V;
 };
 
 /* halving-tree sum S(L, i) = S(2L, i) + S(2L, i + L), S(P, i) = leaf(i) */
@@ -165,10 +181,19 @@ __device__ __forceinline__ double warp_tree_sum(const double (&v)[U]) {
     return s;
 }
 
+/* Minimum over the warp, NaN ignored unless every value is NaN (as a tree of fmin): the bits
+ * as unsigned integers in the doubles' order, the high words' minimum first, then the low words'
+ * among the lanes that hold it -- two integer reductions (22 cycles each on a B200) for five
+ * levels of shuffles and fmin (56 each). */
 __device__ __forceinline__ double warp_min(double s) {
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) s = fmin(s, __shfl_xor_sync(FULL, s, o));
-    return s;
+    const unsigned hi = (unsigned)__double2hiint(s), lo = (unsigned)__double2loint(s);
+    const unsigned flip = (unsigned)((int)hi >> 31);
+    const bool nan = s != s;
+    const unsigned kh = nan ? 0xffffffffu : hi ^ (flip | 0x80000000u), kl = nan ? 0xffffffffu : lo ^ flip;
+    const unsigned mh = __reduce_min_sync(FULL, kh);
+    const unsigned ml = __reduce_min_sync(FULL, kh == mh ? kl : 0xffffffffu);
+    const unsigned back = mh & 0x80000000u ? 0u : 0xffffffffu;
+    return __hiloint2double((int)(mh ^ (back | 0x80000000u)), (int)(ml ^ back));
 }
 
 /* one warp's view of its system: the system runs on G warps (wis = this
@@ -182,9 +207,11 @@ struct Sys {
     double* W;         /* matrix region in shared memory: W, or a padded copy of C */
     double *vp, *vpt, *vcpt, *vx1, *vxu, *vrd;
     double* upsh;      /* unit parameters of the register-operator variant: unit i at upsh[i * NUP] */
-    double* xch;       /* the group's exchange buffers (G > 1) */
+    double* xch;       /* the group's exchange buffers (G > 1), or warp_sum32's (U = G = 1) */
+    double *tpar, *rdpar;   /* vectors split by parity (register-operator variants): entry i at par_slot(i) */
     double* flag;      /* the group's exit-vote words, one per warp (G > 1) */
-    mutable int xsel;  /* which exchange buffer the next group exchange uses */
+    mutable int xsel;  /* which of the two exchange (or warp_sum32) buffers is next */
+    double* ks;        /* stage derivatives (U = 1): entry j, component c of unit i at ks[(j * UD + c) * 32 U G + i] */
     double* sPAR;
     double* sACC;
     int* isACC;
@@ -215,6 +242,60 @@ __device__ __forceinline__ double* grp_buffer(const Sys<U, G>& S) {
     return b;
 }
 
+/* slot of unit i in a vector split by parity: 16 even entries, then 16 odd ones */
+__device__ __forceinline__ int par_slot(int i) { return (i & 1) * RED_RUN + (i >> 1); }
+
+/* Sum over the 32 units of a one-warp system in halving-tree order, every lane
+ * gets it.  The tree splits into its even and its odd lanes' subtrees until its
+ * last addition, so lane l reads the 16 values of its own parity from shared
+ * memory (8 double2 loads, two addresses a load), adds them in tree order and
+ * meets the other parity in one shuffle: 144 cycles against the five-level
+ * butterfly's 176 on a B200 (a 64-bit shuffle and its addition take 35).  The
+ * two buffers alternate: one is rewritten only after a later call's barrier,
+ * which every reader of its previous contents has reached. */
+__device__ __forceinline__ double warp_sum32(const Sys<1, 1>& S, double v) {
+    double* buf = S.xch + (S.xsel & 1) * RED_BUF;
+    S.xsel++;
+    buf[par_slot(S.lane)] = v;
+    __syncwarp();
+    const double2* mine = reinterpret_cast<const double2*>(buf + (S.lane & 1) * RED_RUN);
+    double a[16];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const double2 t = mine[k];
+        a[2 * k] = t.x;
+        a[2 * k + 1] = t.y;
+    }
+    auto leaf = [&](int k) -> double { return a[k]; };
+    const double s = TreeSum<1, 16>::run(0, leaf);
+    return s + __shfl_xor_sync(FULL, s, 1);
+}
+
+/* The sums of two vectors at once, each as warp_sum32 forms it: a quarter of the
+ * warp adds one parity of one vector, so both cost the loads and additions of
+ * one and a second shuffle (a paired butterfly: 196 cycles and twenty shuffles). */
+__device__ __forceinline__ void warp_sum32x2(const Sys<1, 1>& S, double v, double w, double& sv, double& sw) {
+    double* buf = S.xch + (S.xsel & 1) * RED_BUF;
+    S.xsel++;
+    buf[par_slot(S.lane)] = v;
+    buf[2 * RED_RUN + par_slot(S.lane)] = w;
+    __syncwarp();
+    const double2* mine = reinterpret_cast<const double2*>(buf + (S.lane >> 3) * RED_RUN);
+    double a[16];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const double2 t = mine[k];
+        a[2 * k] = t.x;
+        a[2 * k + 1] = t.y;
+    }
+    auto leaf = [&](int k) -> double { return a[k]; };
+    double s = TreeSum<1, 16>::run(0, leaf);
+    s = s + __shfl_xor_sync(FULL, s, 8);
+    const double o = __shfl_xor_sync(FULL, s, 16);
+    sv = S.lane & 16 ? o : s;
+    sw = S.lane & 16 ? s : o;
+}
+
 /* a[k][b]: value k of this lane's unit in block b = G m + wis, for all U G blocks */
 template <int U, int G, int K>
 __device__ __forceinline__ void grp_gather(const Sys<U, G>& S, const double (&v)[K][U], double (&a)[K][U * G]) {
@@ -241,11 +322,15 @@ __device__ __forceinline__ void grp_gather(const Sys<U, G>& S, const double (&v)
  * then the lanes); every lane of every warp of the system gets it. */
 template <int U, int G>
 __device__ __forceinline__ double grp_tree_sum(const Sys<U, G>& S, const double (&v)[U]) {
-    double in[1][U], a[1][U * G];
+    if constexpr (U == 1 && G == 1) {
+        return warp_sum32(S, v[0]);
+    } else {
+        double in[1][U], a[1][U * G];
 #pragma unroll
-    for (int m = 0; m < U; m++) in[0][m] = v[m];
-    grp_gather<U, G, 1>(S, in, a);
-    return warp_tree_sum<U * G>(a[0]);
+        for (int m = 0; m < U; m++) in[0][m] = v[m];
+        grp_gather<U, G, 1>(S, in, a);
+        return warp_tree_sum<U * G>(a[0]);
+    }
 }
 
 /* BiCG exit test and next rho in one exchange: returns whether the fmax-tree
@@ -264,7 +349,7 @@ __device__ __forceinline__ bool grp_sum_max_below(const Sys<U, G>& S, const doub
     }
     const bool wok = __all_sync(FULL, ok), wseen = __any_sync(FULL, seen);
     if constexpr (G == 1) {
-        ysum = warp_tree_sum<U>(y);
+        ysum = grp_tree_sum<U, G>(S, y);
         return wok && wseen;
     } else {
         /* the sum's blocks and one flag word per warp share one exchange buffer */
@@ -285,7 +370,7 @@ __device__ __forceinline__ bool grp_sum_max_below(const Sys<U, G>& S, const doub
             all_ok = all_ok && (f == 1.0 || f == 3.0);
             any_seen = any_seen || f >= 2.0;
         }
-        return all_ok && any_seen;
+        return __all_sync(FULL, all_ok && any_seen);
     }
 }
 
@@ -313,24 +398,59 @@ __device__ __forceinline__ double grp_min(const Sys<U, G>& S, double s) {
     return w[0];
 }
 
+/* What the step controller needs of all units, in one exchange: whether every
+ * a and every b holds, whether any c does, and the minimum of s. */
+template <int U, int G>
+__device__ __forceinline__ void grp_step_votes(const Sys<U, G>& S, bool& a, bool& b, bool& c, double& s) {
+    a = __all_sync(FULL, a);
+    b = __all_sync(FULL, b);
+    c = __any_sync(FULL, c);
+    s = warp_min(s);
+    if constexpr (G > 1) {
+        double* buf = grp_buffer(S);
+        if (S.lane == 0) {
+            buf[2 * S.wis] = __hiloint2double(0, (a ? 0 : 1) + (b ? 0 : 2) + (c ? 4 : 0));
+            buf[2 * S.wis + 1] = s;
+        }
+        grp_sync(S);
+        int f = 0;
+#pragma unroll
+        for (int w = 0; w < G; w++) {
+            f |= __double2loint(buf[2 * w]);
+            s = w == 0 ? buf[1] : fmin(s, buf[2 * w + 1]);
+        }
+        a = __all_sync(FULL, (f & 1) == 0);
+        b = __all_sync(FULL, (f & 2) == 0);
+        c = __all_sync(FULL, (f & 4) != 0);
+    }
+}
+
 template <int U, int G>
 __device__ __forceinline__ bool grp_all(const Sys<U, G>& S, bool p) {
-    double w[G];
-    grp_share(S, __all_sync(FULL, p) ? 1.0 : 0.0, w);
-    bool r = true;
+    if constexpr (G == 1) {
+        return __all_sync(FULL, p);
+    } else {
+        double w[G];
+        grp_share(S, __all_sync(FULL, p) ? 1.0 : 0.0, w);
+        bool r = true;
 #pragma unroll
-    for (int k = 0; k < G; k++) r = r && w[k] != 0.0;
-    return r;
+        for (int k = 0; k < G; k++) r = r && w[k] != 0.0;
+        return __all_sync(FULL, r);
+    }
 }
 
 template <int U, int G>
 __device__ __forceinline__ bool grp_any(const Sys<U, G>& S, bool p) {
-    double w[G];
-    grp_share(S, __any_sync(FULL, p) ? 1.0 : 0.0, w);
-    bool r = false;
+    if constexpr (G == 1) {
+        return __any_sync(FULL, p);
+    } else {
+        double w[G];
+        grp_share(S, __any_sync(FULL, p) ? 1.0 : 0.0, w);
+        bool r = false;
 #pragma unroll
-    for (int k = 0; k < G; k++) r = r || w[k] != 0.0;
-    return r;
+        for (int k = 0; k < G; k++) r = r || w[k] != 0.0;
+        return __all_sync(FULL, r);
+    }
 }
 
 /* A callback may change a system-scope scalar through its reference argument
@@ -382,7 +502,9 @@ __device__ __forceinline__ void warp_tree_sum2(const double (&v)[U], const doubl
 template <int U, int G>
 __device__ __forceinline__ void grp_tree_sum2(const Sys<U, G>& S, const double (&v)[U], const double (&w)[U],
                                               double& sv, double& sw) {
-    if constexpr (G == 1) {
+    if constexpr (U == 1 && G == 1) {
+        warp_sum32x2(S, v[0], w[0], sv, sw);
+    } else if constexpr (G == 1) {
         warp_tree_sum2<U>(v, w, sv, sw);
     } else {
         double in[2][U], a[2][U * G];
@@ -419,12 +541,13 @@ __device__ __forceinline__ bool grp_max_below(const Sys<U, G>& S, const double (
     }
 }
 
-/* The exit test of a multi-warp group, posted before a barrier: each warp's
- * votes go to its flag word, the group crosses one barrier, every warp reads
- * all flags.  The flag words are rewritten only after a later group exchange,
- * which every reader of the current flags passes after reading them. */
+/* The exit test of a multi-warp group, folded into a barrier the group crosses
+ * anyway: each warp posts its votes in its flag word before that barrier, and
+ * after it every warp reads all flags.  The flag words are rewritten only
+ * after a later group exchange, which every reader of the current flags passes
+ * after reading them. */
 template <int U, int G>
-__device__ __forceinline__ bool grp_flags_max_below(const Sys<U, G>& S, const double (&x)[U], double lim) {
+__device__ __forceinline__ void grp_post_max_below(const Sys<U, G>& S, const double (&x)[U], double lim) {
     bool ok = true, seen = false;
 #pragma unroll
     for (int m = 0; m < U; m++) {
@@ -433,7 +556,10 @@ __device__ __forceinline__ bool grp_flags_max_below(const Sys<U, G>& S, const do
     }
     const bool wok = __all_sync(FULL, ok), wseen = __any_sync(FULL, seen);
     if (S.lane == 0) S.flag[S.wis] = (wok ? 1.0 : 0.0) + (wseen ? 2.0 : 0.0);
-    grp_sync(S);
+}
+
+template <int U, int G>
+__device__ __forceinline__ bool grp_read_max_below(const Sys<U, G>& S) {
     bool all_ok = true, any_seen = false;
 #pragma unroll
     for (int w = 0; w < G; w++) {
@@ -441,78 +567,114 @@ __device__ __forceinline__ bool grp_flags_max_below(const Sys<U, G>& S, const do
         all_ok = all_ok && (f == 1.0 || f == 3.0);
         any_seen = any_seen || f >= 2.0;
     }
-    return all_ok && any_seen;
+    return __all_sync(FULL, all_ok && any_seen);
 }
 
 /* ---------------------------------------------------------------------------
  * BiCG iterations (Steppers.cuh:508-561) on a system whose residual r
- * (r~ = r) and start x are set.  apply(v, vt, q, qt) forms q = A v and
- * q~ = A^T vt, zero for slots beyond the system's units.
+ * (r~ = r) and start x are set.  put(v, vt) posts this lane's entries of v and
+ * vt for the other lanes, mul(v, vt, q, qt) -- after a grp_sync -- forms
+ * q = A v and q~ = A^T vt, zero for slots beyond the system's units.  A put
+ * needs no barrier before it when a group exchange lies between it and the last
+ * read of the posted vectors (every reader is past its reads there); a single
+ * warp's __syncwarp costs nothing and stays.
  *
  * REC = 0: the reference's recurrence -- per iteration the products of the
  * search directions, then alpha from one reduction and the exit test with the
  * next rho from a second.
  * REC = 1: the single-reduction form of the same iterates.  The products of
- * the residuals w = A r, w~ = A^T r~ come first; one reduction gives
- * rho = r.r~ and mu = r~.w together; then
+ * the residuals w = A r, w~ = A^T r~ come first; rho = r.r~ needs no product
+ * and mu = r~.w does; then
  *   beta = rho / rho_prev, sigma = mu - beta^2 sigma_prev,
  *   p = r + beta p, p~ = r~ + beta p~, q = w + beta q, q~ = w~ + beta q~,
  *   alpha = rho / sigma,
  * so q = A p, q~ = A^T p~ and sigma = p~.A p (its cross terms equal
  * -rho/alpha_prev = -beta sigma_prev each, by the biorthogonality of the
  * residuals).  Same exits as the reference (|rho| < 1e-6 before the first
- * update, max |r| < 1e-6 after each, at most bicg_max_iter updates); a
- * single warp tests by votes right after the update, a group posts each warp's
- * votes before the barrier that opens the next product phase (the test sees
- * the same r, and no barrier or product is added).  Returns the completed
+ * update, max |r| < 1e-6 after each, at most bicg_max_iter updates).  A single
+ * warp tests the exit by votes right after the update; a group posts each
+ * warp's votes with the residuals it puts for the next product, so the test
+ * costs no barrier of its own.
+ *
+ * An iteration is one dependency chain on one warp and is bound by its length
+ * and its instruction count.  Both quotients of either recurrence go on as
+ * Markstein's and are proven at the end of the iteration, together with the
+ * exit test, so the loop has one branch (a proof's comparison and branch on the
+ * chain cost 60 cycles each, twice an iteration); an unproven one drops the
+ * iteration, which is then done with IEEE divisions.  Returns the completed
  * iterations; sets capped when the cap ended the loop. */
-template <int U, int G, int REC, class Apply>
+template <int U, int G, int REC, class Put, class Mul>
 __device__ __forceinline__ int bicg_iterate(const Sys<U, G>& S, const DeviceProblem& P, const double (&b)[U],
-                                            double (&r)[U], double (&x)[U], Apply&& apply, bool& capped) {
-    double rt[U], p[U], pt[U], q[U], qt[U], prod[U], ar[U];
+                                            double (&r)[U], double (&x)[U], Put&& put, Mul&& mul, bool& capped) {
+    double rt[U], p[U], pt[U], ar[U];
+    const int max_iter = P.bicg_max_iter;
 #pragma unroll
     for (int m = 0; m < U; m++) { rt[m] = r[m]; p[m] = 0.0; pt[m] = 0.0; ar[m] = 0.0; }
     int done = 0;
     bool exited = false;
     auto reference_recurrence = [&]() {
+        double prod[U], q[U], qt[U];
 #pragma unroll
         for (int m = 0; m < U; m++) prod[m] = r[m] * rt[m];
         double rho1 = grp_tree_sum<U, G>(S, prod);
-        double rho2 = 0.0, y2 = 0.0;   /* y2: reciprocal estimate of rho2, formed an iteration early */
-        for (int iter = 1; iter <= P.bicg_max_iter; iter++) {
-            if (iter == 1) {
-#pragma unroll
-                for (int m = 0; m < U; m++) { p[m] = r[m]; pt[m] = rt[m]; }
-                if (fabs(rho1) < 1e-6) { exited = true; break; }
-            } else {
-                const double beta = math::div_known(rho1, rho2, y2);   /* = rho1 / rho2 */
-#pragma unroll
-                for (int m = 0; m < U; m++) {
-                    p[m] = fma(beta, p[m], r[m]);
-                    pt[m] = fma(beta, pt[m], rt[m]);
-                }
-            }
-            const double y1 = math::recip_estimate(rho1);   /* becomes y2 at the end of the iteration */
-            apply(p, pt, q, qt, false);
-#pragma unroll
-            for (int m = 0; m < U; m++) prod[m] = pt[m] * q[m];
-            const double sig = grp_tree_sum<U, G>(S, prod);
-            const double alpha = math::div_known(rho1, sig, math::recip_estimate(sig));   /* = rho1 / sig */
+        if (max_iter < 1) return;
+        if (__all_sync(FULL, fabs(rho1) < 1e-6)) { exited = true; return; }
+        double rho2 = 1.0, y2 = 1.0;   /* y2: reciprocal estimate of rho2, formed an iteration early */
+        double pn[U], ptn[U], xn[U], rn[U], rtn[U], rho_next, y1;
+        bool small, proven;
+        int it = 0;   /* committed iterations of this solve (done counts a redone solve's too) */
+        /* one iteration into pn .. rtn, rho_next and small: nothing is committed */
+        auto iteration = [&](auto ieee) {
+            bool beta_ok, alpha_ok;
+            double beta = decltype(ieee)::value ? math::div_ieee(rho1, rho2)
+                                                : math::div_markstein(rho1, rho2, y2, beta_ok);   /* = rho1 / rho2 */
+            if (it == 0) { beta = 0.0; beta_ok = true; }   /* p = r */
 #pragma unroll
             for (int m = 0; m < U; m++) {
-                x[m] = fma(alpha, p[m], x[m]);
-                r[m] = fma(-alpha, q[m], r[m]);
-                rt[m] = fma(-alpha, qt[m], rt[m]);
-                ar[m] = fabs(r[m]);
-                prod[m] = r[m] * rt[m];
+                pn[m] = fma(beta, p[m], r[m]);
+                ptn[m] = fma(beta, pt[m], rt[m]);
             }
-            double rho_next;
-            const bool small = grp_sum_max_below<U, G>(S, ar, prod, 1e-6, rho_next);
+            if constexpr (G == 1) __syncwarp();
+            put(pn, ptn);
+            grp_sync(S);
+            y1 = math::recip_estimate(rho1);   /* becomes y2 with the commit */
+            mul(pn, ptn, q, qt);
+#pragma unroll
+            for (int m = 0; m < U; m++) prod[m] = ptn[m] * q[m];
+            const double sig = grp_tree_sum<U, G>(S, prod);
+            const double alpha = decltype(ieee)::value
+                                     ? math::div_ieee(rho1, sig)
+                                     : math::div_markstein(rho1, sig, math::recip_estimate(sig), alpha_ok);   /* = rho1 / sig */
+#pragma unroll
+            for (int m = 0; m < U; m++) {
+                xn[m] = fma(alpha, pn[m], x[m]);
+                rn[m] = fma(-alpha, q[m], r[m]);
+                rtn[m] = fma(-alpha, qt[m], rt[m]);
+                ar[m] = fabs(rn[m]);
+                prod[m] = rn[m] * rtn[m];
+            }
+            small = grp_sum_max_below<U, G>(S, ar, prod, 1e-6, rho_next);
+            proven = decltype(ieee)::value || __all_sync(FULL, beta_ok && alpha_ok);
+        };
+        auto commit = [&]() {
+#pragma unroll
+            for (int m = 0; m < U; m++) { p[m] = pn[m]; pt[m] = ptn[m]; x[m] = xn[m]; r[m] = rn[m]; rt[m] = rtn[m]; }
             rho2 = rho1;
             y2 = y1;
-            done++;
-            if (small) { exited = true; break; }
             rho1 = rho_next;
+            it++;
+            done++;
+        };
+        for (;;) {
+            for (;;) {
+                iteration(Const<0>{});
+                if (!proven || small || it + 1 >= max_iter) break;
+                commit();
+            }
+            if (!proven) iteration(Const<1>{});
+            commit();
+            exited = small;
+            if (small || it >= max_iter) break;
         }
     };
     if constexpr (REC == 0) {
@@ -521,71 +683,86 @@ __device__ __forceinline__ int bicg_iterate(const Sys<U, G>& S, const DeviceProb
         double r0[U], x0[U];
 #pragma unroll
         for (int m = 0; m < U; m++) { r0[m] = r[m]; x0[m] = x[m]; }
-        double w[U], wt[U], rw[U];
-        double sigma = 0.0, rho_prev = 0.0, y_prev = 0.0;   /* y_prev: reciprocal estimate of rho_prev */
-        for (int iter = 1; iter <= P.bicg_max_iter; iter++) {
+        double w[U], wt[U], rw[U], prod[U], q[U], qt[U];
+#pragma unroll
+        for (int m = 0; m < U; m++) { q[m] = 0.0; qt[m] = 0.0; }
+        double sigma = 0.0, rho_prev = 1.0, y_prev = 1.0;   /* y_prev: reciprocal estimate of rho_prev */
+        double rho, sg, y1, pn[U], ptn[U], qn[U], qtn[U], xn[U], rn[U], rtn[U];
+        bool small = false, proven = true, early = false;
+        /* one iteration into pn .. rtn and sg: nothing is committed */
+        auto iteration = [&](auto ieee) {
+            if (G == 1 || done == 0) grp_sync(S);
+            put(r, rt);
             if constexpr (G > 1) {
-                if (iter > 1) {
-                    /* the exit test of the previous update: every warp posts its vote
-                     * before the barrier the product phase needs anyway */
-                    if (grp_flags_max_below<U, G>(S, ar, 1e-6)) { exited = true; break; }
-                    apply(r, rt, w, wt, true);
-                } else {
-                    apply(r, rt, w, wt, false);
-                }
-            } else {
-                apply(r, rt, w, wt, false);
+                if (done > 0 && !decltype(ieee)::value) grp_post_max_below<U, G>(S, ar, 1e-6);
             }
+            grp_sync(S);
+            if constexpr (G > 1) {
+                early = done > 0 && !decltype(ieee)::value && grp_read_max_below<U, G>(S);
+                if (early) return;
+            }
+            double mu;
 #pragma unroll
-            for (int m = 0; m < U; m++) { prod[m] = r[m] * rt[m]; rw[m] = rt[m] * w[m]; }
-            double rho, mu;
+            for (int m = 0; m < U; m++) prod[m] = r[m] * rt[m];
+            mul(r, rt, w, wt);
+#pragma unroll
+            for (int m = 0; m < U; m++) rw[m] = rt[m] * w[m];
             grp_tree_sum2<U, G>(S, prod, rw, rho, mu);
-            double alpha;
-            if (iter == 1) {
-                if (fabs(rho) < 1e-6) { exited = true; break; }
-#pragma unroll
-                for (int m = 0; m < U; m++) { p[m] = r[m]; pt[m] = rt[m]; q[m] = w[m]; qt[m] = wt[m]; }
-                sigma = mu;
-                alpha = math::div_known(rho, sigma, math::recip_estimate(sigma));   /* = rho / sigma */
-            } else {
-                /* beta = rho / rho_prev: sigma and alpha go on from Markstein's quotient
-                 * while its proof runs; an unproven quotient redoes them from the IEEE
-                 * one, so both are always the correctly rounded values */
-                bool beta_ok;
-                double beta = math::div_markstein(rho, rho_prev, y_prev, beta_ok);
-                double sg = fma(-(beta * beta), sigma, mu);
-                alpha = math::div_known(rho, sg, math::recip_estimate(sg));   /* = rho / sigma */
-                if (__builtin_expect(!beta_ok, 0)) {
-                    beta = math::div_ieee(rho, rho_prev);
-                    sg = fma(-(beta * beta), sigma, mu);
-                    alpha = math::div_known(rho, sg, math::recip_estimate(sg));
-                }
-                sigma = sg;
-#pragma unroll
-                for (int m = 0; m < U; m++) {
-                    p[m] = fma(beta, p[m], r[m]);
-                    pt[m] = fma(beta, pt[m], rt[m]);
-                    q[m] = fma(beta, q[m], w[m]);
-                    qt[m] = fma(beta, qt[m], wt[m]);
-                }
-            }
-            rho_prev = rho;
-            y_prev = math::recip_estimate(rho);
+            bool beta_ok, alpha_ok;
+            double beta = decltype(ieee)::value ? math::div_ieee(rho, rho_prev)
+                                                : math::div_markstein(rho, rho_prev, y_prev, beta_ok);   /* = rho / rho_prev */
+            if (done == 0) { beta = 0.0; beta_ok = true; }   /* p = r */
+            sg = fma(-(beta * beta), sigma, mu);
+            const double alpha = decltype(ieee)::value
+                                     ? math::div_ieee(rho, sg)
+                                     : math::div_markstein(rho, sg, math::recip_estimate(sg), alpha_ok);   /* = rho / sigma */
+            y1 = math::recip_estimate(rho);
 #pragma unroll
             for (int m = 0; m < U; m++) {
-                x[m] = fma(alpha, p[m], x[m]);
-                r[m] = fma(-alpha, q[m], r[m]);
-                rt[m] = fma(-alpha, qt[m], rt[m]);
-                ar[m] = fabs(r[m]);
+                pn[m] = fma(beta, p[m], r[m]);
+                ptn[m] = fma(beta, pt[m], rt[m]);
+                qn[m] = fma(beta, q[m], w[m]);
+                qtn[m] = fma(beta, qt[m], wt[m]);
+                xn[m] = fma(alpha, pn[m], x[m]);
+                rn[m] = fma(-alpha, qn[m], r[m]);
+                rtn[m] = fma(-alpha, qtn[m], rt[m]);
+                ar[m] = fabs(rn[m]);
             }
+            if constexpr (G == 1) small = grp_max_below<U, G>(S, ar, 1e-6);
+            proven = decltype(ieee)::value || __all_sync(FULL, beta_ok && alpha_ok);
+            early = done == 0 && __all_sync(FULL, fabs(rho) < 1e-6);   /* the first rho test: the update is dropped */
+        };
+        auto commit = [&]() {
+#pragma unroll
+            for (int m = 0; m < U; m++) {
+                p[m] = pn[m]; pt[m] = ptn[m]; q[m] = qn[m]; qt[m] = qtn[m];
+                x[m] = xn[m]; r[m] = rn[m]; rt[m] = rtn[m];
+            }
+            sigma = sg;
+            rho_prev = rho;
+            y_prev = y1;
             done++;
-            if constexpr (G == 1) {
-                if (grp_max_below<U, G>(S, ar, 1e-6)) { exited = true; break; }
+        };
+        if (max_iter >= 1) {
+            for (;;) {
+                for (;;) {
+                    iteration(Const<0>{});
+                    if (early || !proven || small || done + 1 >= max_iter) break;
+                    commit();
+                }
+                if (early) { exited = true; break; }
+                if (!proven) {
+                    iteration(Const<1>{});   /* the previous update's exit test is not repeated */
+                    if (early) { exited = true; break; }
+                }
+                commit();
+                exited = small;
+                if (small || done >= max_iter) break;
             }
         }
         if constexpr (G > 1) {
             /* the update that used up the cap has not been tested yet */
-            if (!exited && done > 0 && done == P.bicg_max_iter && grp_max_below<U, G>(S, ar, 1e-6)) exited = true;
+            if (!exited && done > 0 && done == max_iter && grp_max_below<U, G>(S, ar, 1e-6)) exited = true;
         }
         /* Safeguard: q is a recurrence, not a product, so r can drift from the
          * true residual (and sigma can collapse).  The solution stands when every
@@ -604,7 +781,10 @@ __device__ __forceinline__ int bicg_iterate(const Sys<U, G>& S, const DeviceProb
             double ax[U], unused[U], zero[U], tr[U];
 #pragma unroll
             for (int m = 0; m < U; m++) zero[m] = 0.0;
-            apply(x, zero, ax, unused, false);
+            if constexpr (G == 1) __syncwarp();
+            put(x, zero);
+            grp_sync(S);
+            mul(x, zero, ax, unused);
 #pragma unroll
             for (int m = 0; m < U; m++) tr[m] = fabs(b[m] - ax[m]);
             accept = grp_max_below<U, G>(S, tr, 1e-6);
@@ -621,7 +801,190 @@ __device__ __forceinline__ int bicg_iterate(const Sys<U, G>& S, const DeviceProb
 }
 
 /* ---------------------------------------------------------------------------
- * Coupled right-hand side of the whole system (Steppers.cuh:432-562). */
+ * Work split of the products of multi-warp systems (one unit per lane, matrix in
+ * shared memory, M[i][j] at i + j LD with LD odd).  Warp w owns 32 rows; lane
+ * l = 4r + c of it takes the four rows 4r .. 4r + 3 and of each the columns of
+ * chain c (j = 4t + c), so an entry of a posted vector is loaded for four rows.
+ * The four lanes of a quad then exchange their partial sums (three shuffles a
+ * vector) and lane l keeps row l.  Both directions read 64-bit words of 32
+ * different banks: 4r + c LD along rows, c + 4r LD along columns.
+ *
+ * A sub-partition fills registers from shared memory at 64 to 80 bytes a clock,
+ * which bounds these products; with one row a lane the posted vectors were two
+ * thirds of those bytes (N = 128, two vectors: 128 + 2 x 128 words a lane and
+ * product, now 128 + 2 x 32), and loops of four guarded columns exposed every
+ * load's latency.  Cycles per BiCG iteration of a lone system
+ * on a B200: own matrix, N = 101: 7710 -> 3610, N = 48: 4130 -> 1780; shared
+ * symmetric matrix, N = 128: 3840 -> 2900, N = 51: 1950 -> 1740. */
+
+/* s[i]: this lane's chain of row i.  Returns (s0 + s1) + (s2 + s3) of its own row. */
+__device__ __forceinline__ double quad_chains(int c, const double (&s)[4]) {
+    const bool odd = c & 1, high = c & 2;
+    const double k0 = odd ? s[1] : s[0], k2 = odd ? s[3] : s[2], g0 = odd ? s[0] : s[1], g2 = odd ? s[2] : s[3];
+    const double a0 = k0 + __shfl_xor_sync(FULL, g0, 1), a2 = k2 + __shfl_xor_sync(FULL, g2, 1);
+    return (high ? a2 : a0) + __shfl_xor_sync(FULL, high ? a0 : a2, 2);
+}
+
+/* s[i]: the halving subtree over the rows k = c (mod 4) of column i.  Returns the
+ * whole tree (s0 + s2) + (s1 + s3) of this lane's own column. */
+__device__ __forceinline__ double quad_subtrees(int c, const double (&s)[4]) {
+    const bool odd = c & 1, high = c & 2;
+    const double k0 = high ? s[2] : s[0], k1 = high ? s[3] : s[1], g0 = high ? s[0] : s[2], g1 = high ? s[1] : s[3];
+    const double a0 = k0 + __shfl_xor_sync(FULL, g0, 2), a1 = k1 + __shfl_xor_sync(FULL, g1, 2);
+    return (odd ? a1 : a0) + __shfl_xor_sync(FULL, odd ? a0 : a1, 1);
+}
+
+/* sums of this lane's row of M against K posted vectors (columns j < N) */
+template <int LD, int K>
+__device__ __forceinline__ void quad_row_sums(const double* M, int row0, int c, int N, const double* const (&v)[K],
+                                              double (&out)[K]) {
+    double s[K][4];
+#pragma unroll
+    for (int k = 0; k < K; k++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) s[k][i] = 0.0;
+    const double* m = M + row0 + c * LD;
+    auto group = [&](int t) {
+        double w[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) w[i] = m[4 * t * LD + i];
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            const double x = v[k][4 * t + c];
+#pragma unroll
+            for (int i = 0; i < 4; i++) s[k][i] = fma(w[i], x, s[k][i]);
+        }
+    };
+    const int full = N >> 2;
+#pragma unroll 8
+    for (int t = 0; t < full; t++) group(t);
+    if (c < (N & 3)) group(full);
+#pragma unroll
+    for (int k = 0; k < K; k++) out[k] = quad_chains(c, s[k]);
+}
+
+/* sum of this lane's column of M against a posted vector, halving tree over the NMAX rows (zero-padded) */
+template <int NMAX, int LD>
+__device__ __forceinline__ double quad_column_tree(const double* M, int col0, int c, const double* v) {
+    double s[4];
+    const double* m = M + col0 * LD + c;
+    double x[NMAX / 4];
+#pragma unroll
+    for (int t = 0; t < NMAX / 4; t++) x[t] = v[4 * t + c];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        auto leaf = [&](int t) -> double { return m[i * LD + 4 * t] * x[t]; };
+        s[i] = TreeSum<1, NMAX / 4>::run(0, leaf);
+    }
+    return quad_subtrees(c, s);
+}
+
+/* ---------------------------------------------------------------------------
+ * Coupled right-hand side with the operator W in shared memory and one unit
+ * per lane on G warps (Steppers.cuh:432-562): W_ij = (rD_i C_ij) X1sq_j formed
+ * once per right-hand side from the system's matrix in HBM (L2), products as
+ * quads. */
+template <int G, int REC>
+__device__ __forceinline__ int coupled_rhs_quad(const Sys<1, G>& S, const DeviceProblem& P, double T,
+                                                double (&Xs)[1][UD], double (&F)[1][UD], double (&ua)[1][NUAa],
+                                                int (&iua)[1][NIUAa], bool& capped) {
+    constexpr int NMAX = WarpSmem<1, G>::NMAX;
+    constexpr int LD = WarpSmem<1, G>::LDW;
+    const int N = S.N;
+    const int i = S.unit(0);
+    const bool valid = i < N;
+    const int c = S.lane & 3, row0 = i & ~3;
+    double xu = 0.0, rd = 0.0;
+    grp_sync(S);
+    if (valid) {
+        double Fl[UD], cpt, cpf;
+        CoupledSystems_PerBlock_OdeFunction<double>(S.sid, i, Fl, Xs[0], T, S.upsh + i * NUPa, S.sPAR, S.gPAR,
+                                                    S.igPAR, ua[0], iua[0], S.sACC, S.isACC, &cpt, &cpf);
+#pragma unroll
+        for (int k = 0; k < UD; k++) F[0][k] = Fl[k];
+        xu = Fl[IC];
+        rd = cpf;
+        S.vcpt[i] = cpt;
+        S.vx1[i] = Xs[0][0] * Xs[0][0];
+        S.vxu[i] = xu;
+    } else {
+#pragma unroll
+        for (int k = 0; k < UD; k++) F[0][k] = 0.0;
+    }
+    S.vrd[i] = rd;
+    grp_sync(S);
+    /* b = rD (C CPT) + x_u, r = b - A x_u, and W */
+    double bs[4] = {0.0, 0.0, 0.0, 0.0}, as[4] = {0.0, 0.0, 0.0, 0.0}, rd4[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) rd4[k] = S.vrd[row0 + k];
+    const double* Cg = S.C + row0 + (int64_t)c * N;
+    double* Wq = S.W + row0 + c * LD;
+    const bool in[4] = {row0 < N, row0 + 1 < N, row0 + 2 < N, row0 + 3 < N};
+    auto load = [&](int t, double (&w)[4]) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) w[k] = in[k] ? __ldg(Cg + (int64_t)4 * t * N + k) : 0.0;
+    };
+    auto form = [&](int t, const double (&w)[4]) {
+        const int j = 4 * t + c;
+        const double x1 = S.vx1[j], cp = S.vcpt[j], xj = S.vxu[j];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            bs[k] = fma(w[k], cp, bs[k]);
+            as[k] = fma(w[k] * x1, xj, as[k]);
+            Wq[4 * t * LD + k] = (rd4[k] * w[k]) * x1;
+        }
+    };
+    const int full = N >> 2;
+    int t = 0;
+    for (; t + 3 < full; t += 4) {
+        /* sixteen loads from L2 in flight */
+        double w[4][4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) load(t + e, w[e]);
+#pragma unroll
+        for (int e = 0; e < 4; e++) form(t + e, w[e]);
+    }
+    for (; t < full; t++) {
+        double w[4];
+        load(t, w);
+        form(t, w);
+    }
+    if (c < (N & 3)) {
+        double w[4];
+        load(full, w);
+        form(full, w);
+    }
+    const double bsum = quad_chains(c, bs), asum = quad_chains(c, as);
+    double r = 0.0, bval = 0.0;
+    if (valid) {
+        const double b = fma(rd, bsum, xu);
+        const double ax = fma(rd, asum, xu);
+        r = b - ax;
+        bval = b;
+    }
+    auto put = [&](const double (&v)[1], const double (&vt)[1]) {
+        S.vp[i] = v[0];
+        S.vpt[i] = vt[0];
+    };
+    /* q = A v (row sums of W), q~ = A^T vt (column tree of W) */
+    auto mul = [&](const double (&v)[1], const double (&vt)[1], double (&q)[1], double (&qt)[1]) {
+        double qs[1];
+        const double* const vec[1] = {S.vp};
+        quad_row_sums<LD, 1>(S.W, row0, c, N, vec, qs);
+        const double qts = quad_column_tree<NMAX, LD>(S.W, row0, c, S.vpt);
+        q[0] = valid ? v[0] + qs[0] : 0.0;
+        qt[0] = valid ? vt[0] + qts : 0.0;
+    };
+    double rr[1] = {r}, xx[1] = {xu};
+    const double bb[1] = {bval};
+    const int done = bicg_iterate<1, G, REC>(S, P, bb, rr, xx, put, mul, capped);
+    F[0][IC] = xx[0];
+    return done;
+}
+
+/* ---------------------------------------------------------------------------
+ * Coupled right-hand side with the operator W in shared memory and two or four
+ * units per lane of one warp (Steppers.cuh:432-562). */
 template <int U, int G, int REC>
 __device__ __forceinline__ int coupled_rhs(const Sys<U, G>& S, const DeviceProblem& P, double T,
                                            double (&Xs)[U][UD], double (&F)[U][UD],
@@ -693,15 +1056,15 @@ __device__ __forceinline__ int coupled_rhs(const Sys<U, G>& S, const DeviceProbl
         x[m] = xu[m];
     }
     /* q = A v (row sums of W), q~ = A^T vt (column tree of W) */
-    auto apply = [&](const double (&v)[U], const double (&vt)[U], double (&q)[U], double (&qt)[U], bool presynced) {
-        if (!presynced) grp_sync(S);
+    auto put = [&](const double (&v)[U], const double (&vt)[U]) {
 #pragma unroll
         for (int m = 0; m < U; m++) {
             const int i = S.unit(m);
             S.vp[i] = v[m];
             S.vpt[i] = vt[m];
         }
-        grp_sync(S);
+    };
+    auto mul = [&](const double (&v)[U], const double (&vt)[U], double (&q)[U], double (&qt)[U]) {
 #pragma unroll
         for (int m = 0; m < U; m++) {
             const int i = S.unit(m);
@@ -729,21 +1092,54 @@ __device__ __forceinline__ int coupled_rhs(const Sys<U, G>& S, const DeviceProbl
             }
         }
     };
-    const int done = bicg_iterate<U, G, REC>(S, P, bv, r, x, apply, capped);
+    const int done = bicg_iterate<U, G, REC>(S, P, bv, r, x, put, mul, capped);
 #pragma unroll
     for (int m = 0; m < U; m++) F[m][IC] = x[m];
     return done;
 }
 
 /* ---------------------------------------------------------------------------
+ * Work split of the one-warp products (N <= 32).  Lane l owns unit l, but a
+ * product gives lane l = 2r + h two rows, 2r and 2r + 1, and of each the columns
+ * of chains 2h and 2h + 1 (j = 4t + 2h + e, e < 2): the lane pair then exchanges
+ * one partial sum a vector, and lane l keeps row l.  With a whole row per lane
+ * every entry of a broadcast vector is loaded for one fma, and a sub-partition
+ * fills registers from shared memory at 64 bytes a clock: 32 double2 loads a
+ * product took 270 cycles against 160 for the fmas.  Two rows a lane halve the
+ * loads; the sums are the same chains in the same order. */
+__device__ __forceinline__ double pair_exchange(int h, double own0, double own1) {
+    const double keep = h ? own1 : own0, give = h ? own0 : own1;
+    return keep + __shfl_xor_sync(FULL, give, 1);
+}
+
+/* f(t) for the column groups t < ceil(N / 4), unrolled, in three runs so that
+ * systems of up to 8 and up to 16 units skip the rest */
+template <int NFIX, class Fn>
+__device__ __forceinline__ void column_groups(int N, Fn&& f) {
+#pragma unroll
+    for (int t = 0; t < 2; t++) f(t);
+    if (NFIX != 0 || N > 8) {
+#pragma unroll
+        for (int t = 2; t < 4; t++) f(t);
+    }
+    if (NFIX != 0 || N > 16) {
+#pragma unroll
+        for (int t = 4; t < 8; t++) f(t);
+    }
+}
+
+/* ---------------------------------------------------------------------------
  * Coupled right-hand side with the operator in registers (N <= 32, one unit
- * per lane).  Lane i holds row i of W (for A p) in 32 registers and writes it
- * to shared memory, from where it reads column i of W (for A^T p~; holding
- * the column in registers as well cost 27 % of the step time on the B200 at
- * 254 registers per thread); the system's coupling matrix sits in shared memory
- * (padded, leading dimension 33: row and column reads are conflict-free),
- * staged once per system.  NFIX = 32 drops the N guards for full warps.
- * Same arithmetic, in the same order, as the shared-memory variant. */
+ * per lane).  A lane holds the entries of W that its share of A v reads (two
+ * rows, two chains: 32 doubles in registers) and those its share of A^T vt
+ * reads: for the two columns 2r and 2r + 1 the rows of parity h, because the
+ * halving tree over the rows splits into its even and its odd subtree until its
+ * last addition (32 doubles of its own in shared memory, lane-consecutive
+ * double2; in registers as well they spill).  The system's coupling matrix is
+ * staged once per system, zero-padded (leading dimension 33); the vector of the
+ * transposed product is posted split by parity.
+ * NFIX = 32 drops the N guards for full warps.  Same arithmetic, in the same
+ * order, as the shared-memory variant. */
 template <int NFIX, int REC>
 __device__ __forceinline__ int coupled_rhs_regw(const Sys<1>& S, const DeviceProblem& P, double T,
                                                 double (&Xs)[1][UD], double (&F)[1][UD],
@@ -752,6 +1148,7 @@ __device__ __forceinline__ int coupled_rhs_regw(const Sys<1>& S, const DevicePro
     constexpr int LDC = WarpSmem<1>::LDW;
     const int N = NFIX ? NFIX : S.N;
     const int i = S.lane;
+    const int h = i & 1, r0 = i & ~1;   /* rows (and columns) r0, r0 + 1; chains 2h, 2h + 1; row parity h */
     const bool valid = i < N;
     double xu = 0.0, rd = 0.0, x1 = 0.0;
     __syncwarp();
@@ -773,76 +1170,85 @@ __device__ __forceinline__ int coupled_rhs_regw(const Sys<1>& S, const DevicePro
     S.vx1[i] = x1;
     S.vxu[i] = xu;
     S.vrd[i] = rd;
+    S.rdpar[par_slot(i)] = rd;
     __syncwarp();
-    double wr[32];
-    double bs[4] = {0.0, 0.0, 0.0, 0.0}, as[4] = {0.0, 0.0, 0.0, 0.0};
-    const double* Crow = S.W + i;        /* C[i][j] at i + j*LDC */
-    double* Wt = S.W + 32 * LDC;         /* W[i][j] at i + j*LDC, after the staged C */
-    /* the broadcast vectors are read two entries at a time (16-byte aligned) */
+    double wr[2][16];
+    double2* wc = reinterpret_cast<double2*>(S.W + 32 * LDC) + i;   /* entry k of columns r0, r0 + 1 at wc[32 k] */
+    double bs[2][2] = {{0.0, 0.0}, {0.0, 0.0}}, as[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+    const double* C = S.W;   /* C[i][j] at i + j * LDC */
     const double2* vx1_2 = reinterpret_cast<const double2*>(S.vx1);
     const double2* vcpt2 = reinterpret_cast<const double2*>(S.vcpt);
     const double2* vxu2 = reinterpret_cast<const double2*>(S.vxu);
+    const double2* rdp2 = reinterpret_cast<const double2*>(S.rdpar + h * RED_RUN);
+    const double2 rd2 = reinterpret_cast<const double2*>(S.vrd)[i >> 1], x12 = vx1_2[i >> 1];
 #pragma unroll
-    for (int j = 0; j < 32; j += 2) {
-        const double2 x1p = vx1_2[j / 2], cpp = vcpt2[j / 2], xup = vxu2[j / 2];
+    for (int t = 0; t < 16; t++) wr[0][t] = wr[1][t] = 0.0;
+    column_groups<NFIX>(N, [&](int t) {
+        const double2 x1p = vx1_2[2 * t + h], cpp = vcpt2[2 * t + h], xup = vxu2[2 * t + h];
+        const double2 rdk = rdp2[t];   /* rows k = 4t + h and 4t + 2 + h */
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int jj = j + h;
-            const double cij = Crow[jj * LDC];
-            const double x1j = h ? x1p.y : x1p.x;
-            const bool in = NFIX != 0 || jj < N;
-            if (in) {
-                bs[jj & 3] = fma(cij, h ? cpp.y : cpp.x, bs[jj & 3]);
-                as[jj & 3] = fma(cij * x1j, h ? xup.y : xup.x, as[jj & 3]);
-            }
-            wr[jj] = in ? (rd * cij) * x1j : 0.0;
+        for (int e = 0; e < 2; e++) {
+            const int j = 4 * t + 2 * h + e;
+            const double c0 = C[r0 + j * LDC], c1 = C[r0 + 1 + j * LDC];
+            const double x1j = e ? x1p.y : x1p.x, cpj = e ? cpp.y : cpp.x, xuj = e ? xup.y : xup.x;
+            /* columns beyond N hold zeros in C and in every vector: their terms are +0 */
+            bs[0][e] = fma(c0, cpj, bs[0][e]);
+            bs[1][e] = fma(c1, cpj, bs[1][e]);
+            as[0][e] = fma(c0 * x1j, xuj, as[0][e]);
+            as[1][e] = fma(c1 * x1j, xuj, as[1][e]);
+            wr[0][2 * t + e] = (rd2.x * c0) * x1j;
+            wr[1][2 * t + e] = (rd2.y * c1) * x1j;
+            const int k = 4 * t + 2 * e + h;   /* the row with index 2t + e among those of parity h */
+            const double rk = e ? rdk.y : rdk.x;
+            wc[32 * (2 * t + e)] = make_double2((rk * C[k + r0 * LDC]) * x12.x, (rk * C[k + (r0 + 1) * LDC]) * x12.y);
         }
-    }
-#pragma unroll
-    for (int j = 0; j < 32; j++) Wt[j * LDC + i] = wr[j];
-    __syncwarp();
+    });
     double r = 0.0, bval = 0.0;
-    if (valid) {
-        const double b = fma(rd, (bs[0] + bs[1]) + (bs[2] + bs[3]), xu);
-        const double ax = fma(rd, (as[0] + as[1]) + (as[2] + as[3]), xu);
-        r = b - ax;
-        bval = b;
+    {
+        const double bsum = pair_exchange(h, bs[0][0] + bs[0][1], bs[1][0] + bs[1][1]);
+        const double asum = pair_exchange(h, as[0][0] + as[0][1], as[1][0] + as[1][1]);
+        if (valid) {
+            const double b = fma(rd, bsum, xu);
+            const double ax = fma(rd, asum, xu);
+            r = b - ax;
+            bval = b;
+        }
     }
     const double2* vp2 = reinterpret_cast<const double2*>(S.vp);
-    const double2* vpt2 = reinterpret_cast<const double2*>(S.vpt);
-    /* q = A v (row of W in registers), q~ = A^T vt (column of W from shared memory) */
-    auto apply = [&](const double (&v)[1], const double (&vt)[1], double (&qo)[1], double (&qto)[1], bool presynced) {
-        if (!presynced) __syncwarp();
+    const double2* tp2 = reinterpret_cast<const double2*>(S.tpar + h * RED_RUN);
+    const int tslot = par_slot(i);
+    auto put = [&](const double (&v)[1], const double (&vt)[1]) {
         S.vp[i] = v[0];
-        S.vpt[i] = vt[0];
-        __syncwarp();
-        double qs[4] = {0.0, 0.0, 0.0, 0.0};
+        S.tpar[tslot] = vt[0];
+    };
+    /* q = A v (this lane's chains of two rows), q~ = A^T vt (this lane's subtree of two columns) */
+    auto mul = [&](const double (&v)[1], const double (&vt)[1], double (&qo)[1], double (&qto)[1]) {
+        double qs[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+        double u[2][16];
 #pragma unroll
-        for (int j = 0; j < 32; j += 2) {
-            const double2 a = vp2[j / 2];
-            if (NFIX != 0 || j < N) qs[j & 3] = fma(wr[j], a.x, qs[j & 3]);
-            if (NFIX != 0 || j + 1 < N) qs[(j + 1) & 3] = fma(wr[j + 1], a.y, qs[(j + 1) & 3]);
-        }
-        double q = v[0] + ((qs[0] + qs[1]) + (qs[2] + qs[3]));
-        /* column i of W from shared memory (lane-consecutive rows, conflict-free);
-         * first tree level t_k + t_{k+16} on the loads, then the halving tree over 16 */
-        const double* Wc = Wt + i * LDC;
-        double u[16];
-#pragma unroll
-        for (int k = 0; k < 16; k += 2) {
-            const double2 lo = vpt2[k / 2], hi = vpt2[(k + 16) / 2];
-            u[k] = Wc[k] * lo.x + Wc[k + 16] * hi.x;
-            u[k + 1] = Wc[k + 1] * lo.y + Wc[k + 17] * hi.y;
-        }
-        auto leaf = [&](int k) -> double { return u[k]; };
-        double qt = vt[0] + TreeSum<1, 16>::run(0, leaf);
-        if (!valid) { q = 0.0; qt = 0.0; }
-        qo[0] = q;
-        qto[0] = qt;
+        for (int k = 0; k < 16; k++) u[0][k] = u[1][k] = 0.0;
+        column_groups<NFIX>(N, [&](int t) {
+            const double2 a = vp2[2 * t + h], c = tp2[t];
+            qs[0][0] = fma(wr[0][2 * t], a.x, qs[0][0]);
+            qs[1][0] = fma(wr[1][2 * t], a.x, qs[1][0]);
+            qs[0][1] = fma(wr[0][2 * t + 1], a.y, qs[0][1]);
+            qs[1][1] = fma(wr[1][2 * t + 1], a.y, qs[1][1]);
+            const double2 w0 = wc[32 * (2 * t)], w1 = wc[32 * (2 * t + 1)];
+            u[0][2 * t] = w0.x * c.x;
+            u[1][2 * t] = w0.y * c.x;
+            u[0][2 * t + 1] = w1.x * c.y;
+            u[1][2 * t + 1] = w1.y * c.y;
+        });
+        const double q = v[0] + pair_exchange(h, qs[0][0] + qs[0][1], qs[1][0] + qs[1][1]);
+        auto leaf0 = [&](int k) -> double { return u[0][k]; };
+        auto leaf1 = [&](int k) -> double { return u[1][k]; };
+        const double qt = vt[0] + pair_exchange(h, TreeSum<1, 16>::run(0, leaf0), TreeSum<1, 16>::run(0, leaf1));
+        qo[0] = valid ? q : 0.0;
+        qto[0] = valid ? qt : 0.0;
     };
     double rr[1] = {r}, xx[1] = {xu};
     const double bb[1] = {bval};
-    const int done = bicg_iterate<1, 1, REC>(S, P, bb, rr, xx, apply, capped);
+    const int done = bicg_iterate<1, 1, REC>(S, P, bb, rr, xx, put, mul, capped);
     const double x = xx[0];
     F[0][IC] = x;
     return done;
@@ -901,8 +1307,14 @@ __device__ __forceinline__ int coupled_rhs_sharedc(const Sys<U, G>& S, const Dev
     const double2* cpt2 = reinterpret_cast<const double2*>(S.vcpt);
     const double2* z2 = reinterpret_cast<const double2*>(S.vp);
     const double2* zt2 = reinterpret_cast<const double2*>(S.vpt);
+    const int c = S.lane & 3, row0 = S.unit(0) & ~3;   /* the quad's rows (U = 1) */
     /* rowsum_m = sum_j C[i_m][j] v[j], four interleaved chains */
     auto row_sums = [&](const double2* v2, double (&out)[U]) {
+        if constexpr (U == 1) {
+            const double* const vec[1] = {reinterpret_cast<const double*>(v2)};
+            quad_row_sums<LDC, 1>(S.W, row0, c, N, vec, out);
+            return;
+        }
         double a0[U], a1[U], a2[U], a3[U];
 #pragma unroll
         for (int m = 0; m < U; m++) { a0[m] = 0.0; a1[m] = 0.0; a2[m] = 0.0; a3[m] = 0.0; }
@@ -925,6 +1337,14 @@ __device__ __forceinline__ int coupled_rhs_sharedc(const Sys<U, G>& S, const Dev
      * shared memory once (the kernel is bound by shared-memory reads), the
      * chains and their order per vector as in row_sums */
     auto row_sums2 = [&](const double2* v2, const double2* w2, double (&outv)[U], double (&outw)[U]) {
+        if constexpr (U == 1) {
+            const double* const vec[2] = {reinterpret_cast<const double*>(v2), reinterpret_cast<const double*>(w2)};
+            double o[2];
+            quad_row_sums<LDC, 2>(S.W, row0, c, N, vec, o);
+            outv[0] = o[0];
+            outw[0] = o[1];
+            return;
+        }
         double a0[U], a1[U], a2[U], a3[U], b0[U], b1[U], b2[U], b3[U];
 #pragma unroll
         for (int m = 0; m < U; m++) {
@@ -978,19 +1398,22 @@ __device__ __forceinline__ int coupled_rhs_sharedc(const Sys<U, G>& S, const Dev
         x[m] = xu[m];
     }
     /* q = A v = v + rD a (G (b X1sq v)), q~ = A^T vt = vt + b X1sq (G^T (rD a vt)) */
-    auto apply = [&](const double (&v)[U], const double (&vt)[U], double (&q)[U], double (&qt)[U], bool presynced) {
-        if (!presynced) grp_sync(S);
+    auto put = [&](const double (&v)[U], const double (&vt)[U]) {
 #pragma unroll
         for (int m = 0; m < U; m++) {
             const int i = S.unit(m);
             S.vp[i] = x1[m] * v[m];    /* z  = X1sq v  */
             S.vpt[i] = rd[m] * vt[m];  /* z~ = rD vt   */
         }
-        grp_sync(S);
+    };
+    auto mul = [&](const double (&v)[U], const double (&vt)[U], double (&q)[U], double (&qt)[U]) {
         double qs[U], qts[U];
         if constexpr (SYM) {
             /* C = C^T: the transposed product is a row sum too, from the same reads */
             row_sums2(z2, zt2, qs, qts);
+        } else if constexpr (U == 1) {
+            row_sums(z2, qs);
+            qts[0] = quad_column_tree<NMAX, LDC>(S.W, row0, c, S.vpt);
         } else {
         row_sums(z2, qs);
 #pragma unroll
@@ -1028,7 +1451,7 @@ __device__ __forceinline__ int coupled_rhs_sharedc(const Sys<U, G>& S, const Dev
             qt[m] = vld ? fma(x1[m], qts[m], vt[m]) : 0.0;
         }
     };
-    const int done = bicg_iterate<U, G, REC>(S, P, bv, r, x, apply, capped);
+    const int done = bicg_iterate<U, G, REC>(S, P, bv, r, x, put, mul, capped);
 #pragma unroll
     for (int m = 0; m < U; m++) F[m][IC] = x[m];
     return done;
@@ -1037,10 +1460,11 @@ __device__ __forceinline__ int coupled_rhs_sharedc(const Sys<U, G>& S, const Dev
 /* ---------------------------------------------------------------------------
  * Coupled right-hand side for N <= 32 when the launch shares one symmetric
  * matrix G (RHS = 5; 6 drops the N guards when every system has 32 units):
- * lane i keeps row i of G in registers for the whole system -- nothing is
- * formed per right-hand side -- and both BiCG products are row sums of that
- * row against broadcast vectors, with the unit factors a, b as in
- * coupled_rhs_sharedc<.., SYM = true> and the same arithmetic order. */
+ * a lane keeps its share of G (two rows, two chains: 32 entries) in registers
+ * for the whole system -- nothing is formed per right-hand side -- and both BiCG
+ * products are row sums of those entries against posted vectors, with the unit
+ * factors a, b as in coupled_rhs_sharedc<.., SYM = true> and the same arithmetic
+ * order. */
 template <int NFIX, int REC>
 __device__ __forceinline__ int coupled_rhs_regsym(const Sys<1>& S, const DeviceProblem& P, double T,
                                                   double (&Xs)[1][UD], double (&F)[1][UD], double (&ua)[1][NUAa],
@@ -1048,6 +1472,7 @@ __device__ __forceinline__ int coupled_rhs_regsym(const Sys<1>& S, const DeviceP
                                                   const double (&g)[32], bool& capped) {
     const int N = NFIX ? NFIX : S.N;
     const int i = S.lane;
+    const int h = i & 1;
     const bool valid = i < N;
     double xu = 0.0, rd = 0.0, x1 = 0.0;
     __syncwarp();
@@ -1069,22 +1494,26 @@ __device__ __forceinline__ int coupled_rhs_regsym(const Sys<1>& S, const DeviceP
         S.vp[i] = 0.0;
     }
     __syncwarp();
-    /* row sums of G against two broadcast vectors, four interleaved chains each */
+    /* row sums of G against two posted vectors: this lane's chains of two rows, g = their entries
+     * (columns beyond N hold zeros in G and in the vectors: their terms are +0) */
     auto row_sums2 = [&](const double* v, const double* w, double& outv, double& outw) {
-        const double2* v2 = reinterpret_cast<const double2*>(v);
-        const double2* w2 = reinterpret_cast<const double2*>(w);
-        double a[4] = {0.0, 0.0, 0.0, 0.0}, b[4] = {0.0, 0.0, 0.0, 0.0};
+        const double2* v2 = reinterpret_cast<const double2*>(v) + h;
+        const double2* w2 = reinterpret_cast<const double2*>(w) + h;
+        double a[2][2] = {{0.0, 0.0}, {0.0, 0.0}}, b[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+        column_groups<NFIX>(N, [&](int t) {
+            const double2 vv = v2[2 * t], ww = w2[2 * t];
 #pragma unroll
-        for (int j = 0; j < 32; j += 2) {
-            const double2 vv = v2[j / 2], ww = w2[j / 2];
-            if (NFIX != 0 || j < N) { a[j & 3] = fma(g[j], vv.x, a[j & 3]); b[j & 3] = fma(g[j], ww.x, b[j & 3]); }
-            if (NFIX != 0 || j + 1 < N) {
-                a[(j + 1) & 3] = fma(g[j + 1], vv.y, a[(j + 1) & 3]);
-                b[(j + 1) & 3] = fma(g[j + 1], ww.y, b[(j + 1) & 3]);
+            for (int e = 0; e < 2; e++) {
+                const double vj = e ? vv.y : vv.x, wj = e ? ww.y : ww.x;
+#pragma unroll
+                for (int m = 0; m < 2; m++) {
+                    a[m][e] = fma(g[16 * m + 2 * t + e], vj, a[m][e]);
+                    b[m][e] = fma(g[16 * m + 2 * t + e], wj, b[m][e]);
+                }
             }
-        }
-        outv = (a[0] + a[1]) + (a[2] + a[3]);
-        outw = (b[0] + b[1]) + (b[2] + b[3]);
+        });
+        outv = pair_exchange(h, a[0][0] + a[0][1], a[1][0] + a[1][1]);
+        outw = pair_exchange(h, b[0][0] + b[0][1], b[1][0] + b[1][1]);
     };
     double bsum, asum;
     row_sums2(S.vcpt, S.vp, bsum, asum);
@@ -1096,11 +1525,11 @@ __device__ __forceinline__ int coupled_rhs_regsym(const Sys<1>& S, const DeviceP
         bval = b;
     }
     /* q = A v = v + v_f (G (u v)), q~ = A^T vt = vt + u (G (v_f vt)) with u = b X1sq, v_f = rD a */
-    auto apply = [&](const double (&v)[1], const double (&vt)[1], double (&qo)[1], double (&qto)[1], bool presynced) {
-        if (!presynced) __syncwarp();
-        S.vp[i] = x1 * v[0];     /* z  = u v  */
-        S.vpt[i] = rd * vt[0];   /* z~ = v_f vt */
-        __syncwarp();
+    auto put = [&](const double (&v)[1], const double (&vt)[1]) {
+        S.vp[i] = valid ? x1 * v[0] : 0.0;     /* z  = u v  */
+        S.vpt[i] = valid ? rd * vt[0] : 0.0;   /* z~ = v_f vt */
+    };
+    auto mul = [&](const double (&v)[1], const double (&vt)[1], double (&qo)[1], double (&qto)[1]) {
         double qs, qts;
         row_sums2(S.vp, S.vpt, qs, qts);
         qo[0] = valid ? fma(rd, qs, v[0]) : 0.0;
@@ -1108,7 +1537,7 @@ __device__ __forceinline__ int coupled_rhs_regsym(const Sys<1>& S, const DeviceP
     };
     double rr[1] = {r}, xx[1] = {xu};
     const double bb[1] = {bval};
-    const int done = bicg_iterate<1, 1, REC>(S, P, bb, rr, xx, apply, capped);
+    const int done = bicg_iterate<1, 1, REC>(S, P, bb, rr, xx, put, mul, capped);
     const double x = xx[0];
     F[0][IC] = x;
     return done;
@@ -1200,11 +1629,11 @@ __device__ __forceinline__ int coupled_rhs_band(const Sys<1, G>& S, const Device
     grp_sync(S);
 #pragma unroll
     for (int d = 0; d < BAND_REGS; d++) wt[d] = valid && d < nd ? Wb[d * NMAX + row(d)] : 0.0;
-    auto apply = [&](const double (&v)[1], const double (&vt)[1], double (&qo)[1], double (&qto)[1], bool presynced) {
-        if (!presynced) grp_sync(S);
+    auto put = [&](const double (&v)[1], const double (&vt)[1]) {
         S.vp[i] = v[0];
         S.vpt[i] = vt[0];
-        grp_sync(S);
+    };
+    auto mul = [&](const double (&v)[1], const double (&vt)[1], double (&qo)[1], double (&qto)[1]) {
         double q = 0.0, qt = 0.0;
         if (valid) {
             double qs[4] = {0.0, 0.0, 0.0, 0.0}, ts[4] = {0.0, 0.0, 0.0, 0.0};
@@ -1231,7 +1660,7 @@ __device__ __forceinline__ int coupled_rhs_band(const Sys<1, G>& S, const Device
     };
     double rr[1] = {r}, xx[1] = {xu};
     const double bb[1] = {bval};
-    const int done = bicg_iterate<1, G, REC>(S, P, bb, rr, xx, apply, capped);
+    const int done = bicg_iterate<1, G, REC>(S, P, bb, rr, xx, put, mul, capped);
     F[0][IC] = xx[0];
     return done;
 }
@@ -1242,7 +1671,9 @@ __device__ __forceinline__ int rhs_eval(const Sys<U, G>& S, const DeviceProblem&
                                         double (&F)[U][UD], double (&up)[U][NUPa], double (&ua)[U][NUAa],
                                         int (&iua)[U][NIUAa], const double (&ra)[U], const double (&cb)[U],
                                         const double (&grow)[32], bool& capped) {
-    if constexpr (RHS == 0) {
+    if constexpr (RHS == 0 && U == 1) {
+        return coupled_rhs_quad<G, REC>(S, P, T, Xs, F, ua, iua, capped);
+    } else if constexpr (RHS == 0) {
         return coupled_rhs<U, G, REC>(S, P, T, Xs, F, up, ua, iua, capped);
     } else if constexpr (RHS == 3 || RHS == 4) {
         return coupled_rhs_sharedc<U, G, RHS == 4, REC>(S, P, T, Xs, F, up, ua, iua, ra, cb, capped);
@@ -1267,7 +1698,7 @@ struct Lane {
     int iua[U][NIUAa];
     double ev_a[U][NEa], ev_n[U][NEa];
     double ra[U], cb[U];   /* coupling factors a_i, b_i of the shared-matrix kernels */
-    double grow[32];       /* row of the shared symmetric matrix (RHS 5, 6) */
+    double grow[32];       /* this lane's share of the shared symmetric matrix (RHS 5, 6) */
 };
 
 struct Counters {
@@ -1285,6 +1716,32 @@ __device__ __forceinline__ double* upar_of(const Sys<U, G>& S, Lane<U>& L, int m
     else return L.up[m];
 }
 
+/* The stage derivatives K_j of this lane's units: with one unit per lane in
+ * shared memory (each is written once and read a few times a step, while the
+ * BiCG needs the registers), else in registers. */
+template <int U, int G, int J>
+struct Stages {
+    double k[U == 1 ? 1 : J][U][UD];
+    __device__ __forceinline__ void set(const Sys<U, G>& S, int st, const double (&F)[U][UD]) {
+        if constexpr (U == 1) {
+#pragma unroll
+            for (int c = 0; c < UD; c++) S.ks[(st * UD + c) * 32 * G + S.unit(0)] = F[0][c];
+        } else {
+#pragma unroll
+            for (int j = 0; j < J; j++)
+#pragma unroll
+                for (int m = 0; m < U; m++)
+#pragma unroll
+                    for (int c = 0; c < UD; c++)
+                        if (j == st) k[j][m][c] = F[m][c];
+        }
+    }
+    __device__ __forceinline__ double get(const Sys<U, G>& S, int j, int m, int c) const {
+        if constexpr (U == 1) return S.ks[(j * UD + c) * 32 * G + S.unit(0)];
+        else return k[j][m][c];
+    }
+};
+
 /* Cash-Karp tableau (Steppers.cuh:197-370): stage nodes and coefficients,
  * each entry the double nearest to the reference's literal fraction. */
 __constant__ double kCK_A[6][5] = {
@@ -1299,7 +1756,7 @@ __constant__ double kCK_C[6] = {0.0, 1.0 / 5.0, 3.0 / 10.0, 3.0 / 5.0, 1.0, 7.0 
 __constant__ double kRK4_A[4] = {0.0, 0.5, 0.5, 1.0};
 
 /* ---------------------------------------------------------------------------
- * RKCK45 step (Steppers.cuh:94-425); returns finiteness of y5 and the error.
+ * RKCK45 step (Steppers.cuh:94-425); returns whether y5 and the error of this lane's units are finite.
  * The six stages run as one loop so the coupled right-hand side is inlined
  * once; stage s evaluates at X + dt * (sum_j<s a_sj K_j) with the terms
  * accumulated in the reference's order (first a product, then fmas). */
@@ -1307,13 +1764,15 @@ template <int U, int RHS, int G, int REC>
 __device__ __forceinline__ bool step_rkck45(const Sys<U, G>& S, const DeviceProblem& P, Lane<U>& L,
                                             double T, double dt, double (&Yn)[U][UD], double (&E)[U][UD],
                                             Counters& cnt, bool& capped) {
-    double K[6][U][UD];
+    Stages<U, G, 6> K;
+    if constexpr (U > 1) {
 #pragma unroll
-    for (int j = 0; j < 6; j++)
+        for (int j = 0; j < 6; j++)
 #pragma unroll
-        for (int m = 0; m < U; m++)
+            for (int m = 0; m < U; m++)
 #pragma unroll
-            for (int c = 0; c < UD; c++) K[j][m][c] = 0.0;
+                for (int c = 0; c < UD; c++) K.k[j][m][c] = 0.0;
+    }
 #pragma unroll 1
     for (int st = 0; st < 6; st++) {
         double Xs[U][UD], F[U][UD];
@@ -1330,21 +1789,15 @@ __device__ __forceinline__ bool step_rkck45(const Sys<U, G>& S, const DeviceProb
             for (int m = 0; m < U; m++)
 #pragma unroll
                 for (int c = 0; c < UD; c++) {
-                    double acc = K[0][m][c] * kCK_A[st][0];
+                    double acc = K.get(S, 0, m, c) * kCK_A[st][0];
 #pragma unroll
                     for (int j = 1; j < 5; j++)
-                        if (j < st) acc = fma(K[j][m][c], kCK_A[st][j], acc);
+                        if (j < st) acc = fma(K.get(S, j, m, c), kCK_A[st][j], acc);
                     Xs[m][c] = fma(acc, dt, L.X[m][c]);
                 }
         }
         cnt.bicg += rhs_eval<U, RHS, G, REC>(S, P, Ts, Xs, F, L.up, L.ua, L.iua, L.ra, L.cb, L.grow, capped);
-#pragma unroll
-        for (int j = 0; j < 6; j++)
-#pragma unroll
-            for (int m = 0; m < U; m++)
-#pragma unroll
-                for (int c = 0; c < UD; c++)
-                    if (j == st) K[j][m][c] = F[m][c];
+        K.set(S, st, F);
     }
     cnt.rhs += 6;
     bool finite = true;
@@ -1352,34 +1805,36 @@ __device__ __forceinline__ bool step_rkck45(const Sys<U, G>& S, const DeviceProb
     for (int m = 0; m < U; m++)
 #pragma unroll
         for (int c = 0; c < UD; c++) {
-            double s = K[0][m][c] * (37.0 / 378.0);
-            s = fma(K[2][m][c], 250.0 / 621.0, s);
-            s = fma(K[3][m][c], 125.0 / 594.0, s);
-            s = fma(K[5][m][c], 512.0 / 1771.0, s);
+            double s = K.get(S, 0, m, c) * (37.0 / 378.0);
+            s = fma(K.get(S, 2, m, c), 250.0 / 621.0, s);
+            s = fma(K.get(S, 3, m, c), 125.0 / 594.0, s);
+            s = fma(K.get(S, 5, m, c), 512.0 / 1771.0, s);
             Yn[m][c] = fma(s, dt, L.X[m][c]);
-            double e = K[0][m][c] * (37.0 / 378.0 - 2825.0 / 27648.0);
-            e = fma(K[2][m][c], 250.0 / 621.0 - 18575.0 / 48384.0, e);
-            e = fma(K[3][m][c], 125.0 / 594.0 - 13525.0 / 55296.0, e);
-            e = fma(K[4][m][c], 0.0 - 277.0 / 14336.0, e);
-            e = fma(K[5][m][c], 512.0 / 1771.0 - 1.0 / 4.0, e);
+            double e = K.get(S, 0, m, c) * (37.0 / 378.0 - 2825.0 / 27648.0);
+            e = fma(K.get(S, 2, m, c), 250.0 / 621.0 - 18575.0 / 48384.0, e);
+            e = fma(K.get(S, 3, m, c), 125.0 / 594.0 - 13525.0 / 55296.0, e);
+            e = fma(K.get(S, 4, m, c), 0.0 - 277.0 / 14336.0, e);
+            e = fma(K.get(S, 5, m, c), 512.0 / 1771.0 - 1.0 / 4.0, e);
             E[m][c] = fma(dt, fabs(e), 1e-18);
             if (valid_unit(S, m) && (!isfinite(Yn[m][c]) || !isfinite(E[m][c]))) finite = false;
         }
-    return grp_all<U, G>(S, finite);
+    return finite;
 }
 
 /* classical RK4 step (the reference has only its fixed-step controller,
- * ErrorControllers.cuh:424-450) */
+ * ErrorControllers.cuh:424-450); returns whether this lane's new states are finite */
 template <int U, int RHS, int G, int REC>
 __device__ __forceinline__ bool step_rk4(const Sys<U, G>& S, const DeviceProblem& P, Lane<U>& L,
                                          double T, double dt, double (&Yn)[U][UD], Counters& cnt, bool& capped) {
-    double K[4][U][UD];
+    Stages<U, G, 4> K;
+    if constexpr (U > 1) {
 #pragma unroll
-    for (int j = 0; j < 4; j++)
+        for (int j = 0; j < 4; j++)
 #pragma unroll
-        for (int m = 0; m < U; m++)
+            for (int m = 0; m < U; m++)
 #pragma unroll
-            for (int c = 0; c < UD; c++) K[j][m][c] = 0.0;
+                for (int c = 0; c < UD; c++) K.k[j][m][c] = 0.0;
+    }
 #pragma unroll 1
     for (int st = 0; st < 4; st++) {
         double Xs[U][UD], F[U][UD];
@@ -1399,19 +1854,13 @@ __device__ __forceinline__ bool step_rk4(const Sys<U, G>& S, const DeviceProblem
                     double kprev = 0.0;
 #pragma unroll
                     for (int j = 0; j < 3; j++)
-                        if (j == st - 1) kprev = K[j][m][c];
+                        if (j == st - 1) kprev = K.get(S, j, m, c);
                     /* stage 3 uses K3 itself (a = 1): fma(K3, dt, X); stages 1, 2 use K*0.5 */
                     Xs[m][c] = st == 3 ? fma(kprev, dt, L.X[m][c]) : fma(kprev * kRK4_A[st], dt, L.X[m][c]);
                 }
         }
         cnt.bicg += rhs_eval<U, RHS, G, REC>(S, P, Ts, Xs, F, L.up, L.ua, L.iua, L.ra, L.cb, L.grow, capped);
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-#pragma unroll
-            for (int m = 0; m < U; m++)
-#pragma unroll
-                for (int c = 0; c < UD; c++)
-                    if (j == st) K[j][m][c] = F[m][c];
+        K.set(S, st, F);
     }
     cnt.rhs += 4;
     bool finite = true;
@@ -1419,14 +1868,14 @@ __device__ __forceinline__ bool step_rk4(const Sys<U, G>& S, const DeviceProblem
     for (int m = 0; m < U; m++)
 #pragma unroll
         for (int c = 0; c < UD; c++) {
-            double s = K[0][m][c] * (1.0 / 6.0);
-            s = fma(K[1][m][c], 1.0 / 3.0, s);
-            s = fma(K[2][m][c], 1.0 / 3.0, s);
-            s = fma(K[3][m][c], 1.0 / 6.0, s);
+            double s = K.get(S, 0, m, c) * (1.0 / 6.0);
+            s = fma(K.get(S, 1, m, c), 1.0 / 3.0, s);
+            s = fma(K.get(S, 2, m, c), 1.0 / 3.0, s);
+            s = fma(K.get(S, 3, m, c), 1.0 / 6.0, s);
             Yn[m][c] = fma(s, dt, L.X[m][c]);
             if (valid_unit(S, m) && !isfinite(Yn[m][c])) finite = false;
         }
-    return grp_all<U, G>(S, finite);
+    return finite;
 }
 
 /* dense-output store (DenseOutput.cuh:312-361), bounds-checked at the slot */
@@ -1526,22 +1975,33 @@ __device__ void run_period(const Sys<U, G>& S, const DeviceProblem& P, Lane<U>& 
             finite = step_rkck45<U, RHS, G, REC>(S, P, L, T, dt, Yn, E, cnt, capped);
             /* ErrorController_RKCK45 (ErrorControllers.cuh:454-542) */
             double rr = 1e30;
-            int ru = 1;
+            bool within = true;
 #pragma unroll
             for (int m = 0; m < U; m++) {
                 if (valid_unit(S, m)) {
+                    double et[UD], ratio[UD];
+                    bool ok = true;
 #pragma unroll
                     for (int c = 0; c < UD; c++) {
-                        double et = fmax(rtol[c] * fmax(fabs(Yn[m][c]), fabs(L.X[m][c])), atol[c]);
-                        ru = ru & (E[m][c] < et);
-                        rr = fmin(rr, et / E[m][c]);
+                        et[c] = fmax(rtol[c] * fmax(fabs(Yn[m][c]), fabs(L.X[m][c])), atol[c]);
+                        within = within && E[m][c] < et[c];
+                        ratio[c] = math::div_try(et[c], E[m][c], ok);
                     }
+                    if (!ok) {
+#pragma unroll
+                        for (int c = 0; c < UD; c++) ratio[c] = math::div_ieee(et[c], E[m][c]);
+                    }
+#pragma unroll
+                    for (int c = 0; c < UD; c++) rr = fmin(rr, ratio[c]);
                 }
             }
-            update = grp_all<U, G>(S, ru) ? 1 : 0;
-            double relerr = grp_min<U, G>(S, rr);
-            double mult = update == 1 ? 0.8 * bes::math::pow(relerr, 1.0 / 5.0)
-                                      : 0.8 * bes::math::pow(relerr, 1.0 / 4.0);
+            grp_step_votes<U, G>(S, finite, within, capped, rr);
+            update = within ? 1 : 0;
+            const double expo = within ? 1.0 / 5.0 : 1.0 / 4.0;
+            bool ok = true;
+            double mult = math::pow_try(rr, expo, ok);
+            if (!__all_sync(FULL, ok)) mult = math::pow_general(rr, expo);
+            mult = 0.8 * mult;
             if (!isfinite(mult)) finite = false;
             if (!finite) {
                 mult = P.shrink;
@@ -1558,10 +2018,13 @@ __device__ void run_period(const Sys<U, G>& S, const DeviceProblem& P, Lane<U>& 
             newdt = fmax(newdt, P.dtmin);
         } else {
             finite = step_rk4<U, RHS, G, REC>(S, P, L, T, dt, Yn, cnt, capped);
+            bool unused = true;
+            double none = 0.0;
+            grp_step_votes<U, G>(S, finite, unused, capped, none);
             if (!finite) { cnt.status |= BES_STATUS_NONFINITE; terminate = true; update = 0; }
             newdt = P.dt0;
         }
-        if (grp_any<U, G>(S, capped)) cnt.status |= BES_STATUS_BICG_CAP;
+        if (capped) cnt.status |= BES_STATUS_BICG_CAP;
 
         if (!terminate && NE > 0) {
             /* next event values at the trial state (Solver.cuh:393-414) */
@@ -1628,9 +2091,11 @@ __device__ void run_period(const Sys<U, G>& S, const DeviceProblem& P, Lane<U>& 
                         if (Uu != udt) anyU = 1;
                     }
                 }
-                T = grp_resolve<U, G>(S, T, TnewL, firstT);
-                dt = grp_resolve<U, G>(S, dt, dTnewL, firstD);
-                if (grp_any<U, G>(S, anyU)) udt = 1;
+                if (grp_any<U, G>(S, firstT >= 0 || firstD >= 0 || anyU != 0)) {
+                    T = grp_resolve<U, G>(S, T, TnewL, firstT);
+                    dt = grp_resolve<U, G>(S, dt, dTnewL, firstD);
+                    if (grp_any<U, G>(S, anyU)) udt = 1;
+                }
             }
             if (NE > 0) {
                 /* ActionAfterEventDetection when an event lands within tolerance (Solver.cuh:465-495) */
@@ -1658,9 +2123,11 @@ __device__ void run_period(const Sys<U, G>& S, const DeviceProblem& P, Lane<U>& 
                         }
                     }
                 }
-                T = grp_resolve<U, G>(S, T, TnewL, firstT);
-                dt = grp_resolve<U, G>(S, dt, dTnewL, firstD);
-                if (grp_any<U, G>(S, anyU)) udt = 1;
+                if (grp_any<U, G>(S, firstT >= 0 || firstD >= 0 || anyU != 0)) {
+                    T = grp_resolve<U, G>(S, T, TnewL, firstT);
+                    dt = grp_resolve<U, G>(S, dt, dTnewL, firstD);
+                    if (grp_any<U, G>(S, anyU)) udt = 1;
+                }
                 /* refresh event values at the accepted state (Solver.cuh:497-525) */
 #pragma unroll
                 for (int m = 0; m < U; m++)
@@ -1822,7 +2289,7 @@ __global__ void __launch_bounds__(RHS == 3 || RHS == 4 || RHS == 7 || G > 1 ? 25
         S.vrd = S.vxu + NM;
         S.xch = S.vrd + NM;
         S.flag = S.xch + 2 * XCH_BUF;
-        S.sPAR = S.xch + SM::XCH_DOUBLES;
+        S.sPAR = S.xch + SM::XCH_DOUBLES + SM::RED_DOUBLES;
         S.upsh = S.sPAR + NSPa + NSAa + NISAa;
     } else {
         using SM = WarpSmem<U, G>;
@@ -1835,10 +2302,13 @@ __global__ void __launch_bounds__(RHS == 3 || RHS == 4 || RHS == 7 || G > 1 ? 25
         S.vxu = S.vx1 + SM::NMAX;
         S.vrd = S.vxu + SM::NMAX;
         S.xch = S.vrd + SM::NMAX;
+        S.tpar = S.xch + 2 * RED_BUF;   /* U = G = 1 */
+        S.rdpar = S.tpar + 2 * RED_RUN;
         S.flag = S.xch + 2 * XCH_BUF;
-        S.sPAR = S.xch + SM::XCH_DOUBLES;
+        S.sPAR = S.xch + SM::XCH_DOUBLES + SM::RED_DOUBLES;
         S.upsh = S.sPAR + SM::SYS_DOUBLES;
     }
+    S.ks = S.upsh + 32 * U * G * NUPa;
     S.sACC = S.sPAR + NSPa;
     S.isACC = reinterpret_cast<int*>(S.sACC + NSAa);
     S.gPAR = P.gpar;
@@ -1894,11 +2364,17 @@ __global__ void __launch_bounds__(RHS == 3 || RHS == 4 || RHS == 7 || G > 1 ? 25
             for (int c = lane; c < NSA; c += 32) S.sACC[c] = P.sacc[(int64_t)c * P.n_systems + sid];
             for (int c = lane; c < NISA; c += 32) S.isACC[c] = P.isacc[(int64_t)c * P.n_systems + sid];
         }
+        if constexpr (RHS == 0 && U == 1) {
+            /* the rows and columns beyond N read as zeros (a right-hand side writes only the others) */
+            for (int idx = 32 * S.wis + lane; idx < WarpSmem<U, G>::W_DOUBLES; idx += 32 * G) S.W[idx] = 0.0;
+        }
         if constexpr (RHS == 5 || RHS == 6) {
-            /* row `lane` of the shared symmetric matrix, zero-padded to 32 */
+            /* rows 2r, 2r + 1 of the shared symmetric matrix at the columns 4t + 2h + e of lane 2r + h, zero-padded */
 #pragma unroll
-            for (int j = 0; j < 32; j++)
-                L.grow[j] = (lane < S.N && j < S.N) ? __ldg(S.C + lane + (int64_t)j * S.N) : 0.0;
+            for (int k = 0; k < 32; k++) {
+                const int row = (lane & ~1) + (k >> 4), j = 4 * ((k & 15) >> 1) + 2 * (lane & 1) + (k & 1);
+                L.grow[k] = (row < S.N && j < S.N) ? __ldg(S.C + row + (int64_t)j * S.N) : 0.0;
+            }
         }
         if constexpr (RHS == 7) {
             /* stage the system's band: Cb[d][i] = C[i][(i + d - bw) mod N] */

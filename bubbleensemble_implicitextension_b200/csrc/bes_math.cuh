@@ -66,7 +66,7 @@ __device__ __forceinline__ double pow2_scale(double x, int k) {
  * very close to a rounding boundary.
  * ok reports the proof that it is: the exact remainder r1 = a - b q1 (one
  * fma) satisfies |r1| < ulp(q1)/2 |b|, with q1 not a power of two (so the ulp
- * is the same on both sides of q1) and a, b within [2^-400, 2^400] (no
+ * is the same on both sides of q1) and a, b within [2^-400, 2^400) (no
  * overflow, underflow or subnormal along the way).  The test is sound for any
  * y: rounding is monotonic and ulp(q1)/2 |b| is exact, so a rounded remainder
  * below the bound means the exact one is.  A caller may go on with q1 before
@@ -88,11 +88,14 @@ __device__ __forceinline__ double div_markstein(double a, double b, double y, bo
     const double r0 = fma(-q0, b, a);
     const double q1 = fma(r0, y, q0);
     const double r1 = fma(-q1, b, a);
-    const long long qb = __double_as_longlong(q1);
-    const double half_ulp_b = __longlong_as_double(qb & 0x7ff0000000000000LL) * 0x1p-53 * fabs(b);
-    const double aa = fabs(a), ab = fabs(b);
-    ok = aa >= 0x1p-400 && aa <= 0x1p400 && ab >= 0x1p-400 && ab <= 0x1p400 &&
-         (qb & 0x000fffffffffffffLL) != 0 && fabs(r1) < half_ulp_b;
+    /* the conditions on exponent fields: integer arithmetic beside the remainder, one
+     * comparison in double.  With a and b in range, b's field plus q1's less
+     * 1076 is that of ulp(q1)/2 |b|, near a's less 53. */
+    const unsigned ah = (unsigned)__double2hiint(a) & 0x7fffffffu, bh = (unsigned)__double2hiint(b) & 0x7fffffffu;
+    const unsigned qh = (unsigned)__double2hiint(q1), ql = (unsigned)__double2loint(q1);
+    const double half_ulp_b = __hiloint2double((int)(bh + (qh & 0x7ff00000u) - (1076u << 20)), __double2loint(b));
+    ok = (ah >> 20) - 623u < 800u && (bh >> 20) - 623u < 800u && ((qh & 0x000fffffu) | ql) != 0u &&
+         fabs(r1) < half_ulp_b;
     return q1;
 }
 
@@ -108,12 +111,8 @@ __device__ __forceinline__ double div_known(double a, double b, double y) {
 #define BES_INV_LN2 1.4426950408889634
 #define BES_SQRT2 1.4142135623730951
 
-/* exp(a + b) with b a small correction */
-__device__ __forceinline__ double exp_ab(double a, double b) {
-    if (a != a) return a;
-    if (a > 709.8) return __longlong_as_double(0x7ff0000000000000LL);
-    if (a < -745.2) return 0.0;
-    double kd = round_nearest(a * BES_INV_LN2);
+/* exp(a + b - kd ln 2), kd = a / ln 2 rounded to an integer, b a small correction */
+__device__ __forceinline__ double exp_poly(double a, double b, double kd) {
     double r = fma(-kd, BES_LN2_HI, a);
     r = fma(-kd, BES_LN2_LO, r);
     r = r + b;
@@ -131,19 +130,29 @@ __device__ __forceinline__ double exp_ab(double a, double b) {
     p = fma(p, r, 0.5);
     p = fma(p, r, 1.0);
     p = fma(p, r, 1.0);
-    return pow2_scale(p, (int)kd);
+    return p;
 }
 
-/* log(x) as head + tail, x finite and > 0 */
-__device__ __forceinline__ void log_hl(double x, double& hi, double& lo) {
-    int e = 0;
-    if (x < 2.2250738585072014e-308) { x = x * 18014398509481984.0; e = -54; }
-    unsigned long long u = (unsigned long long)__double_as_longlong(x);
-    e += (int)((u >> 52) & 0x7ffULL) - 1023;
+/* exp(a + b) with b a small correction */
+__device__ __forceinline__ double exp_ab(double a, double b) {
+    if (a != a) return a;
+    if (a > 709.8) return __longlong_as_double(0x7ff0000000000000LL);
+    if (a < -745.2) return 0.0;
+    double kd = round_nearest(a * BES_INV_LN2);
+    return pow2_scale(exp_poly(a, b, kd), (int)kd);
+}
+
+/* x = 2^e m with m in (sqrt2/2, sqrt2], x normal: f = m - 1 */
+__device__ __forceinline__ double log_reduce(double x, int& e) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+    e = (int)((u >> 52) & 0x7ffULL) - 1023;
     double m = __longlong_as_double((long long)((u & 0x000fffffffffffffULL) | 0x3ff0000000000000ULL));
     if (m > BES_SQRT2) { m = m * 0.5; e += 1; }
-    double f = m - 1.0;
-    double s = f / (2.0 + f);
+    return m - 1.0;
+}
+
+/* log(2^e (1 + f)) as head + tail, s = f / (2 + f) */
+__device__ __forceinline__ void log_series(int e, double f, double s, double& hi, double& lo) {
     double z = s * s;
     double t = 0.07407407407407407;
     t = fma(t, z, 0.08);
@@ -172,6 +181,14 @@ __device__ __forceinline__ void log_hl(double x, double& hi, double& lo) {
     double h = sh + sl;
     hi = h;
     lo = sl - (h - sh);
+}
+
+/* log(x) as head + tail, x finite and > 0 */
+__device__ __forceinline__ void log_hl(double x, double& hi, double& lo) {
+    int e0 = 0, e;
+    if (x < 2.2250738585072014e-308) { x = x * 18014398509481984.0; e0 = -54; }
+    const double f = log_reduce(x, e);
+    log_series(e + e0, f, f / (2.0 + f), hi, lo);
 }
 
 __device__ __forceinline__ bool is_int(double y) {
@@ -210,6 +227,8 @@ __device__ __forceinline__ double pow(double x, double y) {
     return sign * exp_ab(ph, pl);
 }
 
+static __device__ __noinline__ double pow_general(double x, double y) { return pow(x, y); }
+
 /* (1/x)^y as exp(-y log x): no reciprocal on the dependency chain and no
  * rounding of 1/x; positive finite x and finite nonzero y, anything else
  * goes through pow(1/x, y) */
@@ -224,10 +243,8 @@ __device__ __forceinline__ double pow_recip(double x, double y) {
     return exp_ab(ph, pl);
 }
 
-/* sin(pi x), cos(pi x) */
-__device__ __forceinline__ void sincospi(double x, double& s, double& c) {
-    if (!isfinite(x)) { s = __longlong_as_double(0x7ff8000000000000LL); c = s; return; }
-    double n = round_nearest(x + x);
+/* sin(pi x), cos(pi x) from n = 2 x rounded to an integer, q = n mod 4 */
+__device__ __forceinline__ void sincospi_reduced(double x, double n, int q, double& s, double& c) {
     double r = fma(-0.5, n, x);
     double z = r * r;
     double ps = 7.952054001475513e-07;
@@ -250,11 +267,16 @@ __device__ __forceinline__ void sincospi(double x, double& s, double& c) {
     pc = fma(pc, z, 4.0587121264167685);
     pc = fma(pc, z, -4.934802200544679);
     pc = fma(pc, z, 1.0);
-    int q = (int)((long long)n & 3);
-    if (q == 0) { s = ps; c = pc; }
-    else if (q == 1) { s = pc; c = -ps; }
-    else if (q == 2) { s = -ps; c = -pc; }
-    else { s = -pc; c = ps; }
+    const double a = q & 1 ? pc : ps, b = q & 1 ? ps : pc;
+    s = q & 2 ? -a : a;
+    c = (q + 1) & 2 ? -b : b;
+}
+
+/* sin(pi x), cos(pi x) */
+__device__ __forceinline__ void sincospi(double x, double& s, double& c) {
+    if (!isfinite(x)) { s = __longlong_as_double(0x7ff8000000000000LL); c = s; return; }
+    const double n = round_nearest(x + x);
+    sincospi_reduced(x, n, (int)((long long)n & 3), s, c);
 }
 
 #define BES_PIO2_1 1.5707963267341256
@@ -297,6 +319,54 @@ __device__ __forceinline__ void sincos(double x, double& s, double& c) {
     else if (q == 1) { s = pc; c = -ps; }
     else if (q == 2) { s = -ps; c = -pc; }
     else { s = -pc; c = ps; }
+}
+
+/* ---------------------------------------------------------------------------
+ * The same functions over their ordinary range, without branches.  Each of
+ * them gives the bits of the function above where it leaves ok true, and clears
+ * ok anywhere else (a division whose quotient is not proven, an operand out of
+ * range); the caller collects ok over a whole expression and takes the general
+ * functions once for the rest.  One warp integrates a system, so its time is
+ * the length of its dependency chains: with the special cases branched off in
+ * each function the independent chains of a right-hand side (two divisions, the
+ * power, sine and cosine) ran one after the other. */
+
+/* a / b */
+__device__ __forceinline__ double div_try(double a, double b, bool& ok) {
+    bool proven;
+    const double q = div_markstein(a, b, recip_estimate(b), proven);
+    ok = ok && proven;
+    return q;
+}
+
+/* x to the nearest integer, and that integer; |x| < 2^30 */
+__device__ __forceinline__ double round_small(double x, int& i) {
+    const double t = x + 6755399441055744.0; /* 1.5 * 2^52: the integer stands in the low word */
+    i = __double2loint(t);
+    return t - 6755399441055744.0;
+}
+
+/* x^y of x in (1e-300, 1e300) and |y| < 1e300 */
+__device__ __forceinline__ double pow_try(double x, double y, bool& ok) {
+    int e, k;
+    const double f = log_reduce(x, e);
+    const double s = div_try(f, 2.0 + f, ok);
+    double lh, ll;
+    log_series(e, f, s, lh, ll);
+    const double ph = y * lh;
+    double pl = fma(y, lh, -ph);
+    pl = fma(y, ll, pl);
+    ok = ok && x > 1.0e-300 && x < 1.0e300 && fabs(y) < 1.0e300 && fabs(ph) < 700.0;
+    const double kd = round_small(ph * BES_INV_LN2, k);
+    return exp_poly(ph, pl, kd) * __longlong_as_double((long long)(k + 1023) << 52);
+}
+
+/* sin(pi x), cos(pi x) of |x| < 2^28 */
+__device__ __forceinline__ void sincospi_try(double x, double& s, double& c, bool& ok) {
+    int i;
+    const double n = round_small(x + x, i);
+    ok = ok && fabs(x) < 268435456.0;
+    sincospi_reduced(x, n, i & 3, s, c);
 }
 
 }  // namespace math

@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 
 from bubbleensemble_implicitextension_b200 import workloads as W
-from tests.helpers import assert_bitwise, run_gpu
+from tests.helpers import assert_bitwise, ragged_ensemble, run_gpu
 
 pytestmark = pytest.mark.gpu
 
@@ -18,4 +18,40 @@ def test_banded_operator_around_its_register_diagonals(n, bw, rec, gpu, oracle_l
     ens.max_steps_per_period = 300
     got = run_gpu(ens, n_periods=1, reset_at=-1, bicg_recurrence=rec)
     want = oracle_lib.run(ens, n_periods=1, reset_at=-1, bicg_variant=rec)
+    assert_bitwise(got, want, KEYS)
+
+
+def _bounded(ens, budget=250):
+    ens.max_steps_per_period = budget
+    return ens
+
+
+@pytest.mark.parametrize("rec", [0, 1])
+def test_own_matrices_at_the_edges_of_the_work_splits(rec, gpu, oracle_lib):
+    """Pairs of rows and column groups of one warp (N <= 32, in runs of 8, 16 and 32 columns), quads of rows with
+    every remainder of N mod 4 on two and on four warps."""
+    ens = _bounded(ragged_ensemble([1, 2, 3, 8, 9, 15, 16, 17, 31, 32, 33, 35, 63, 64, 65, 66, 67, 126, 128], seed=5))
+    got = run_gpu(ens, n_periods=1, reset_at=-1, bicg_recurrence=rec)
+    want = oracle_lib.run(ens, n_periods=1, reset_at=-1, bicg_variant=rec)
+    assert_bitwise(got, want, KEYS)
+
+
+@pytest.mark.parametrize("rec", [0, 1])
+@pytest.mark.parametrize("factored", [False, True])
+@pytest.mark.parametrize("n", [7, 16, 17, 31, 34, 63, 65, 99, 127])
+def test_shared_matrices_at_the_edges_of_the_work_splits(n, factored, rec, gpu, oracle_lib):
+    """One matrix for the launch, symmetric with unit factors or not, at odd sizes of every class."""
+    ens = _bounded(W.c3_ensemble(n_systems=3, n_units=n, n_periods=1, cube_um=400.0 * (n / 32) ** (1 / 3),
+                                 factored=factored), 120)
+    got = run_gpu(ens, n_periods=1, reset_at=-1, bicg_recurrence=rec, shared_matrices=True)
+    want = oracle_lib.run(ens, n_periods=1, reset_at=-1, bicg_variant=rec, shared_assoc=factored or n > 32)
+    assert_bitwise(got, want, KEYS)
+
+
+@pytest.mark.parametrize("rec", [0, 1])
+def test_step_budget_inside_an_event_and_two_frequencies(rec, gpu, oracle_lib):
+    """The dual-frequency drive of the uneven clouds (both elementary-function paths) with a small step budget."""
+    ens = _bounded(W.c2_ensemble(n_systems=24, seed=8, n_periods=2, reset_at=1), 200)
+    got = run_gpu(ens, bicg_recurrence=rec)
+    want = oracle_lib.run(ens, n_periods=2, reset_at=1, bicg_variant=rec)
     assert_bitwise(got, want, KEYS)
