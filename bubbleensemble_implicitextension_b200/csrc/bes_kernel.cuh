@@ -21,14 +21,14 @@
  * atomics become warp butterflies (the butterfly computes the reference's
  * halving-tree sum exactly, because IEEE addition is commutative); the
  * transposed product A^T p~, which the reference forms with N block-wide
- * reductions per BiCG iteration, becomes one column tree per lane over the
- * operator W_ij = (rD_i C_ij) X0_j^2 that is formed once per right-hand side
- * in shared memory (leading dimension 32UG+1: conflict-free row and column
- * reads).  When the launch shares one matrix, it is staged once per CTA
+ * reductions per BiCG iteration, becomes column trees over the operator
+ * W_ij = (rD_i C_ij) X0_j^2 that is formed once per right-hand side: in
+ * registers and shared memory for one warp, in tensor memory for a group.  When
+ * the launch shares one matrix, it is staged once per CTA
  * instead; when that matrix is symmetric (a geometry 1/d with the radii as
  * unit factors), both products become row sums of the same entries -- read
- * once from shared memory, or for N <= 32 held as a register row for the
- * whole system.  Every scalar of the step control is uniform over the group
+ * once from tensor memory, or for N <= 32 held in registers for the whole
+ * system.  Every scalar of the step control is uniform over the group
  * and held in registers; a single-warp system needs no block barrier at all,
  * a multi-warp system one named barrier per reduction.
  *
@@ -44,6 +44,7 @@
 #include "bes_device.h"
 #include "bes_math.cuh"
 #include "bes_status.h"
+#include "bes_tmem.cuh"
 
 #ifndef BES_SYSTEM_DEFINITION
 #include "km_model.cuh"
@@ -78,9 +79,9 @@ constexpr int XCH_BUF = 2 * 128 + 8;
  * runs a load reads at once start in different banks */
 constexpr int RED_RUN = 18, RED_BUF = 4 * RED_RUN;
 /* Shared-memory doubles per system (G warps, U units per lane, NMAX = 32 U G
- * units): one NMAX x (NMAX+1) matrix region (the operator W; with the
- * register-resident operator, U = G = 1, the system's coupling matrix C and
- * the part of W that A^T v reads), six broadcast vectors, the group's exchange buffers
+ * units): one matrix region (more than one unit per lane: the operator W, leading
+ * dimension NMAX+1; one: the system's coupling matrix C, for one warp with the
+ * part of W that A^T v reads), six broadcast vectors, the group's exchange buffers
  * (G > 1) or the warp's reduction buffers, the system-scope arrays, and the unit
  * parameters when each lane owns one unit (U = 1: in registers they crowd out
  * the BiCG state). */
@@ -89,7 +90,7 @@ struct WarpSmem {
     static constexpr int NMAX = 32 * U * G;
     static constexpr bool ONE = U == 1 && G == 1;   /* one warp, one unit per lane */
     static constexpr int LDW = NMAX + 1;
-    static constexpr int W_DOUBLES = NMAX * LDW;
+    static constexpr int W_DOUBLES = U == 1 && G > 1 ? NMAX * NMAX : NMAX * LDW;
     static constexpr int VEC_DOUBLES = 6 * NMAX;
     static constexpr int XCH_DOUBLES = G > 1 ? 2 * XCH_BUF + 8 : 0; /* two buffers of two values per unit, vote words */
     static constexpr int SYS_DOUBLES = NSPa + NSAa + NISAa;  /* ints stored in double slots */
@@ -106,17 +107,20 @@ struct WarpSmem {
                   "broadcast vectors must start on 16-byte boundaries");
 };
 
-/* Shared-memory layout of the shared-matrix variant (RHS = 3): one padded
- * copy of the launch's coupling matrix per CTA (one unit per lane: leading
- * dimension NMAX+1 for the quads; more: NMAX+2, rows are read lane-consecutive,
- * each lane's column is 16-byte aligned and its double2 reads are
- * conflict-free), then per system five broadcast
- * vectors, the group's exchange buffers and the system-scope arrays. */
-template <int U, int G = 1>
+/* Shared-memory layout of the shared-matrix variants: with RHS = 3, or more than
+ * one unit per lane, one padded copy of the launch's coupling matrix per CTA
+ * (one unit per lane: leading dimension NMAX+1 for the quads; more: NMAX+2, rows
+ * are read lane-consecutive, each lane's column is 16-byte aligned and its
+ * double2 reads are conflict-free); the symmetric matrix of one-unit-per-lane
+ * systems (RHS = 4) is in tensor memory.  Then per system five broadcast
+ * vectors, the group's exchange buffers, the system-scope arrays, the unit
+ * parameters and the stage derivatives. */
+template <int U, int G, bool SYM>
 struct SharedCSmem {
     static constexpr int NMAX = 32 * U * G;
+    static constexpr bool TMEM = SYM && U == 1;
     static constexpr int LDC = U == 1 ? NMAX + 1 : NMAX + 2;   /* odd for the quads' 64-bit reads */
-    static constexpr int C_DOUBLES = NMAX * LDC;
+    static constexpr int C_DOUBLES = TMEM ? 0 : NMAX * LDC;
     static constexpr int XCH_DOUBLES = G > 1 ? 2 * XCH_BUF + 8 : 0;
     static constexpr int UP_DOUBLES = U == 1 ? NMAX * NUPa : 0; /* unit parameters (one unit per lane) */
     static constexpr int K_DOUBLES = U == 1 ? 6 * UD * NMAX : 0;    /* stage derivatives (one unit per lane) */
@@ -126,6 +130,15 @@ struct SharedCSmem {
     static constexpr int WARP_BYTES = WARP_DOUBLES * 8;
     static_assert(C_DOUBLES % 2 == 0 && WARP_DOUBLES % 2 == 0, "16-byte alignment");
 };
+
+/* TMEM columns of a CTA of `warps` warps: RHS 4 keeps each lane's share of the
+ * shared matrix once for all systems of the CTA (NMAX doubles a lane); RHS 0
+ * keeps each system's row and column shares of W (2 NMAX doubles a lane), four
+ * warps side by side in the four quarters.  0: the variant uses none. */
+template <int U, int RHS, int G>
+__host__ __device__ constexpr int tmem_columns(int warps) {
+    return U != 1 || G == 1 ? 0 : RHS == 4 ? 2 * 32 * G : RHS == 0 ? 4 * 32 * G * ((warps + 3) / 4) : 0;
+}
 
 /* Shared-memory layout of the banded variant (RHS = 7, one unit per lane, G
  * warps, NMAX = 32 G units): per system the staged band of its coupling
@@ -209,6 +222,7 @@ struct Sys {
     double* upsh;      /* unit parameters of the register-operator variant: unit i at upsh[i * NUP] */
     double* xch;       /* the group's exchange buffers (G > 1), or warp_sum32's (U = G = 1) */
     double *tpar, *rdpar;   /* vectors split by parity (register-operator variants): entry i at par_slot(i) */
+    uint32_t tm;       /* this warp's lanes of the system's (RHS 0) or the CTA's (RHS 4) columns in tensor memory */
     double* flag;      /* the group's exit-vote words, one per warp (G > 1) */
     mutable int xsel;  /* which of the two exchange (or warp_sum32) buffers is next */
     double* ks;        /* stage derivatives (U = 1): entry j, component c of unit i at ks[(j * UD + c) * 32 U G + i] */
@@ -817,21 +831,24 @@ __device__ __forceinline__ int bicg_iterate(const Sys<U, G>& S, const DeviceProb
  * on a B200: own matrix, N = 101: 7710 -> 3610, N = 48: 4130 -> 1780; shared
  * symmetric matrix, N = 128: 3840 -> 2900, N = 51: 1950 -> 1740. */
 
-/* s[i]: this lane's chain of row i.  Returns (s0 + s1) + (s2 + s3) of its own row. */
+/* s[i]: this lane's chain of row i.  Returns (s0 + s1) + (s2 + s3) of its own row.
+ * M0, M1: the lane bits that hold c's two bits. */
+template <int M0, int M1>
 __device__ __forceinline__ double quad_chains(int c, const double (&s)[4]) {
     const bool odd = c & 1, high = c & 2;
     const double k0 = odd ? s[1] : s[0], k2 = odd ? s[3] : s[2], g0 = odd ? s[0] : s[1], g2 = odd ? s[2] : s[3];
-    const double a0 = k0 + __shfl_xor_sync(FULL, g0, 1), a2 = k2 + __shfl_xor_sync(FULL, g2, 1);
-    return (high ? a2 : a0) + __shfl_xor_sync(FULL, high ? a0 : a2, 2);
+    const double a0 = k0 + __shfl_xor_sync(FULL, g0, M0), a2 = k2 + __shfl_xor_sync(FULL, g2, M0);
+    return (high ? a2 : a0) + __shfl_xor_sync(FULL, high ? a0 : a2, M1);
 }
 
 /* s[i]: the halving subtree over the rows k = c (mod 4) of column i.  Returns the
  * whole tree (s0 + s2) + (s1 + s3) of this lane's own column. */
+template <int M0, int M1>
 __device__ __forceinline__ double quad_subtrees(int c, const double (&s)[4]) {
     const bool odd = c & 1, high = c & 2;
     const double k0 = high ? s[2] : s[0], k1 = high ? s[3] : s[1], g0 = high ? s[0] : s[2], g1 = high ? s[1] : s[3];
-    const double a0 = k0 + __shfl_xor_sync(FULL, g0, 2), a1 = k1 + __shfl_xor_sync(FULL, g1, 2);
-    return (odd ? a1 : a0) + __shfl_xor_sync(FULL, odd ? a0 : a1, 1);
+    const double a0 = k0 + __shfl_xor_sync(FULL, g0, M1), a1 = k1 + __shfl_xor_sync(FULL, g1, M1);
+    return (odd ? a1 : a0) + __shfl_xor_sync(FULL, odd ? a0 : a1, M0);
 }
 
 /* sums of this lane's row of M against K posted vectors (columns j < N) */
@@ -860,7 +877,7 @@ __device__ __forceinline__ void quad_row_sums(const double* M, int row0, int c, 
     for (int t = 0; t < full; t++) group(t);
     if (c < (N & 3)) group(full);
 #pragma unroll
-    for (int k = 0; k < K; k++) out[k] = quad_chains(c, s[k]);
+    for (int k = 0; k < K; k++) out[k] = quad_chains<1, 2>(c, s[k]);
 }
 
 /* sum of this lane's column of M against a posted vector, halving tree over the NMAX rows (zero-padded) */
@@ -876,24 +893,116 @@ __device__ __forceinline__ double quad_column_tree(const double* M, int col0, in
         auto leaf = [&](int t) -> double { return m[i * LD + 4 * t] * x[t]; };
         s[i] = TreeSum<1, NMAX / 4>::run(0, leaf);
     }
-    return quad_subtrees(c, s);
+    return quad_subtrees<1, 2>(c, s);
 }
 
 /* ---------------------------------------------------------------------------
- * Coupled right-hand side with the operator W in shared memory and one unit
- * per lane on G warps (Steppers.cuh:432-562): W_ij = (rD_i C_ij) X1sq_j formed
- * once per right-hand side from the system's matrix in HBM (L2), products as
- * quads. */
+ * The same split with the matrix in tensor memory.  Lane l = 8c + r takes the
+ * rows r, r + 8, r + 16, r + 24 of its warp's 32 and the columns of chain c (the
+ * eight lanes of a chain read one word of a posted vector, which shared memory
+ * serves in one cycle a load), and keeps row l = r + 8c.  Its NMAX entries are
+ * its own, so they sit in its TMEM lane, sixteen doubles a chunk: chunk k of the
+ * row share holds the column groups t = 4k .. 4k + 3, four rows each; of the
+ * column share the leaves 4k .. 4k + 3 of the halving tree, in bit-reversed
+ * order of t, four columns each.  A chunk is loaded while the one before is
+ * used; its latency is some 130 cycles, so chunks of eight doubles (40 cycles of
+ * work) were slower than shared memory, and the loop is unrolled over all of
+ * NMAX (guards on the chunks spilled registers).  The FP64 pipe is the bound now; shared memory's 128 bytes a clock were
+ * (N = 128: 1540 of the 2070 cycles of a product).  Cycles per BiCG iteration of
+ * a lone system on a B200: own matrix, N = 101: 3610 -> 2040, N = 48: 1780 ->
+ * 1410; shared symmetric matrix, N = 128: 2900 -> 1960 (two on an SM: 4290 ->
+ * 2660), N = 51: 1740 -> 1430. *
+
+/* sums of this lane's row share against K posted vectors, entry j of vector k at v[K j + k];
+ * the entries from N to the next multiple of 8 are zeros */
+template <int K, int NMAX>
+__device__ __forceinline__ void tmem_row_sums(uint32_t addr, int c, const double* v, double (&out)[K]) {
+    double s[K][4];
+#pragma unroll
+    for (int k = 0; k < K; k++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) s[k][i] = 0.0;
+    const double* vc = v + K * c;
+    tmem::Chunk m[2];
+    m[0].load(addr);
+#pragma unroll
+    for (int ch = 0; ch < NMAX / 16; ch++) {
+        m[ch & 1].wait();
+        if (ch + 1 < NMAX / 16) m[(ch + 1) & 1].load(addr + 32 * (ch + 1));
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            double x[K];
+            if constexpr (K == 2) {
+                const double2 p = *reinterpret_cast<const double2*>(vc + 8 * (4 * ch + e));
+                x[0] = p.x;
+                x[1] = p.y;
+            } else {
+                x[0] = vc[4 * (4 * ch + e)];
+            }
+#pragma unroll
+            for (int k = 0; k < K; k++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) s[k][i] = fma(m[ch & 1].get(4 * e + i), x[k], s[k][i]);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < K; k++) out[k] = quad_chains<8, 16>(c, s[k]);
+}
+
+/* t of leaf m of the halving tree over T = 2^B column groups: m's bits reversed */
+__host__ __device__ constexpr int tree_leaf(int m, int T) {
+    int t = 0;
+    for (int b = 1; b < T; b *= 2) t = 2 * t + (m / b) % 2;
+    return t;
+}
+
+/* halving tree of this lane's column share against a posted vector, over the NMAX (zero-padded) rows */
+template <int NMAX>
+__device__ __forceinline__ double tmem_column_tree(uint32_t addr, int c, const double* v) {
+    constexpr int T = NMAX / 4, CH = T / 4;
+    double part[CH][4];
+    tmem::Chunk m[2];
+    m[0].load(addr);
+#pragma unroll
+    for (int ch = 0; ch < CH; ch++) {
+        m[ch & 1].wait();
+        if (ch + 1 < CH) m[(ch + 1) & 1].load(addr + 32 * (ch + 1));
+        double x[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) x[e] = v[4 * tree_leaf(4 * ch + e, T) + c];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            part[ch][i] = (m[ch & 1].get(i) * x[0] + m[ch & 1].get(4 + i) * x[1]) +
+                          (m[ch & 1].get(8 + i) * x[2] + m[ch & 1].get(12 + i) * x[3]);
+            /* join the subtrees that this chunk completes */
+#pragma unroll
+            for (int w = 1; w < CH; w *= 2)
+                if ((ch + 1) % (2 * w) == 0) part[ch + 1 - 2 * w][i] = part[ch + 1 - 2 * w][i] + part[ch + 1 - w][i];
+        }
+    }
+    return quad_subtrees<8, 16>(c, part[0]);
+}
+
+/* ---------------------------------------------------------------------------
+ * Coupled right-hand side with the operator W in tensor memory and one unit
+ * per lane on G warps (Steppers.cuh:432-562): a lane forms its row share and its
+ * column share of W_ij = (rD_i C_ij) X1sq_j once per right-hand side from the
+ * system's matrix, which is staged in shared memory once per system (zero-padded,
+ * C[i][j] at (i ^ f(j)) + j NMAX with f(j) = j's low three bits reversed onto
+ * bits 3, 2, 1: neither reads along rows nor along columns meet bank conflicts).
+ * From L2 on every right-hand side the forming took 8080 cycles of a
+ * 101-bubble system, now 4560. */
+__device__ __forceinline__ int quad_swizzle(int j) { return ((j & 1) << 3) | ((j & 2) << 1) | ((j & 4) >> 1); }
+
 template <int G, int REC>
 __device__ __forceinline__ int coupled_rhs_quad(const Sys<1, G>& S, const DeviceProblem& P, double T,
                                                 double (&Xs)[1][UD], double (&F)[1][UD], double (&ua)[1][NUAa],
                                                 int (&iua)[1][NIUAa], bool& capped) {
     constexpr int NMAX = WarpSmem<1, G>::NMAX;
-    constexpr int LD = WarpSmem<1, G>::LDW;
     const int N = S.N;
     const int i = S.unit(0);
     const bool valid = i < N;
-    const int c = S.lane & 3, row0 = i & ~3;
+    const int c = S.lane >> 3, r0 = S.lane & 7, row0 = 32 * S.wis + r0;
     double xu = 0.0, rd = 0.0;
     grp_sync(S);
     if (valid) {
@@ -910,51 +1019,56 @@ __device__ __forceinline__ int coupled_rhs_quad(const Sys<1, G>& S, const Device
     } else {
 #pragma unroll
         for (int k = 0; k < UD; k++) F[0][k] = 0.0;
+        S.vcpt[i] = 0.0;
+        S.vx1[i] = 0.0;
+        S.vxu[i] = 0.0;
     }
     S.vrd[i] = rd;
     grp_sync(S);
-    /* b = rD (C CPT) + x_u, r = b - A x_u, and W */
-    double bs[4] = {0.0, 0.0, 0.0, 0.0}, as[4] = {0.0, 0.0, 0.0, 0.0}, rd4[4];
+    /* b = rD (C CPT) + x_u, r = b - A x_u, and W (C and the posted vectors are zeros beyond N) */
+    double bs[4] = {0.0, 0.0, 0.0, 0.0}, as[4] = {0.0, 0.0, 0.0, 0.0}, rd4[4], x14[4];
 #pragma unroll
-    for (int k = 0; k < 4; k++) rd4[k] = S.vrd[row0 + k];
-    const double* Cg = S.C + row0 + (int64_t)c * N;
-    double* Wq = S.W + row0 + c * LD;
-    const bool in[4] = {row0 < N, row0 + 1 < N, row0 + 2 < N, row0 + 3 < N};
-    auto load = [&](int t, double (&w)[4]) {
+    for (int k = 0; k < 4; k++) {
+        rd4[k] = S.vrd[row0 + 8 * k];
+        x14[k] = S.vx1[row0 + 8 * k];
+    }
+    const double* C = S.W;
+    const int flip = quad_swizzle(c);
+#pragma unroll 2
+    for (int ch = 0; ch < NMAX / 16; ch++) {
+        tmem::Chunk m;
 #pragma unroll
-        for (int k = 0; k < 4; k++) w[k] = in[k] ? __ldg(Cg + (int64_t)4 * t * N + k) : 0.0;
-    };
-    auto form = [&](int t, const double (&w)[4]) {
-        const int j = 4 * t + c;
-        const double x1 = S.vx1[j], cp = S.vcpt[j], xj = S.vxu[j];
+        for (int e = 0; e < 4; e++) {
+            const int j = 16 * ch + 4 * e + c;
+            const double x1 = S.vx1[j], cp = S.vcpt[j], xj = S.vxu[j];
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            bs[k] = fma(w[k], cp, bs[k]);
-            as[k] = fma(w[k] * x1, xj, as[k]);
-            Wq[4 * t * LD + k] = (rd4[k] * w[k]) * x1;
+            for (int k = 0; k < 4; k++) {
+                const double cij = C[((row0 + 8 * k) ^ (flip | ((e & 1) << 1))) + j * NMAX];
+                bs[k] = fma(cij, cp, bs[k]);
+                as[k] = fma(cij * x1, xj, as[k]);
+                m.set(4 * e + k, (rd4[k] * cij) * x1);
+            }
         }
-    };
-    const int full = N >> 2;
-    int t = 0;
-    for (; t + 3 < full; t += 4) {
-        /* sixteen loads from L2 in flight */
-        double w[4][4];
+        m.store(S.tm + 32 * ch);
+    }
+    const int cflip = quad_swizzle(r0);
+#pragma unroll 2
+    for (int ch = 0; ch < NMAX / 16; ch++) {
+        tmem::Chunk m;
 #pragma unroll
-        for (int e = 0; e < 4; e++) load(t + e, w[e]);
+        for (int e = 0; e < 4; e++) {
+            /* leaf 4 ch + e: its bits reversed are t (tree_leaf) */
+            const int t = (int)(__brev(4u * (unsigned)ch + (unsigned)e) >> (32 - (G == 2 ? 4 : 5)));
+            const int j = 4 * t + c;
+            const double rdj = S.vrd[j];
 #pragma unroll
-        for (int e = 0; e < 4; e++) form(t + e, w[e]);
+            for (int k = 0; k < 4; k++)
+                m.set(4 * e + k, (rdj * C[(j ^ cflip) + (row0 + 8 * k) * NMAX]) * x14[k]);
+        }
+        m.store(S.tm + 2 * NMAX + 32 * ch);
     }
-    for (; t < full; t++) {
-        double w[4];
-        load(t, w);
-        form(t, w);
-    }
-    if (c < (N & 3)) {
-        double w[4];
-        load(full, w);
-        form(full, w);
-    }
-    const double bsum = quad_chains(c, bs), asum = quad_chains(c, as);
+    const double bsum = quad_chains<8, 16>(c, bs), asum = quad_chains<8, 16>(c, as);
+    tmem::wait_stores();
     double r = 0.0, bval = 0.0;
     if (valid) {
         const double b = fma(rd, bsum, xu);
@@ -969,9 +1083,8 @@ __device__ __forceinline__ int coupled_rhs_quad(const Sys<1, G>& S, const Device
     /* q = A v (row sums of W), q~ = A^T vt (column tree of W) */
     auto mul = [&](const double (&v)[1], const double (&vt)[1], double (&q)[1], double (&qt)[1]) {
         double qs[1];
-        const double* const vec[1] = {S.vp};
-        quad_row_sums<LD, 1>(S.W, row0, c, N, vec, qs);
-        const double qts = quad_column_tree<NMAX, LD>(S.W, row0, c, S.vpt);
+        tmem_row_sums<1, NMAX>(S.tm, c, S.vp, qs);
+        const double qts = tmem_column_tree<NMAX>(S.tm + 2 * NMAX, c, S.vpt);
         q[0] = valid ? v[0] + qs[0] : 0.0;
         qt[0] = valid ? vt[0] + qts : 0.0;
     };
@@ -1271,9 +1384,11 @@ __device__ __forceinline__ int coupled_rhs_sharedc(const Sys<U, G>& S, const Dev
                                                    double (&up)[U][NUPa], double (&ua)[U][NUAa],
                                                    int (&iua)[U][NIUAa], const double (&ra)[U],
                                                    const double (&cb)[U], bool& capped) {
-    constexpr int NMAX = SharedCSmem<U, G>::NMAX;
-    constexpr int LDC = SharedCSmem<U, G>::LDC;
+    using SM = SharedCSmem<U, G, SYM>;
+    constexpr int NMAX = SM::NMAX;
+    constexpr int LDC = SM::LDC;
     constexpr int H = NMAX / 2;
+    static_assert(U > 1 || !SYM, "the symmetric matrix of one-unit-per-lane systems is in tensor memory");
     const int N = S.N;
     /* with C = diag(a) G diag(b): x1 holds u = b X1sq (applied before G), rd holds v = rD a (after G) */
     double xu[U], rd[U], x1[U], r[U], x[U], bv[U];
@@ -1340,7 +1455,7 @@ __device__ __forceinline__ int coupled_rhs_sharedc(const Sys<U, G>& S, const Dev
         if constexpr (U == 1) {
             const double* const vec[2] = {reinterpret_cast<const double*>(v2), reinterpret_cast<const double*>(w2)};
             double o[2];
-            quad_row_sums<LDC, 2>(S.W, row0, c, N, vec, o);
+            quad_row_sums<LDC, 2>(S.W, row0, c, N, vec, o);   /* the right-hand side's sums only */
             outv[0] = o[0];
             outw[0] = o[1];
             return;
@@ -1454,6 +1569,65 @@ __device__ __forceinline__ int coupled_rhs_sharedc(const Sys<U, G>& S, const Dev
     const int done = bicg_iterate<U, G, REC>(S, P, bv, r, x, put, mul, capped);
 #pragma unroll
     for (int m = 0; m < U; m++) F[m][IC] = x[m];
+    return done;
+}
+
+/* ---------------------------------------------------------------------------
+ * Coupled right-hand side with the launch's shared symmetric matrix and one unit
+ * per lane on G warps (RHS = 4): the scaled products of coupled_rhs_sharedc, both
+ * as row sums of the lane's share of G in tensor memory (stored once per CTA)
+ * against two vectors posted side by side. */
+template <int G, int REC>
+__device__ __forceinline__ int coupled_rhs_symquad(const Sys<1, G>& S, const DeviceProblem& P, double T,
+                                                   double (&Xs)[1][UD], double (&F)[1][UD], double (&ua)[1][NUAa],
+                                                   int (&iua)[1][NIUAa], const double (&ra)[1], const double (&cb)[1],
+                                                   bool& capped) {
+    const int N = S.N;
+    const int i = S.unit(0);
+    const bool valid = i < N;
+    const int c = S.lane >> 3;
+    double2* post = reinterpret_cast<double2*>(S.vp) + i;   /* vp and vpt: the pairs of all NMAX units */
+    double xu = 0.0, rd = 0.0, x1 = 0.0;
+    grp_sync(S);
+    if (valid) {
+        double Fl[UD], cpt, cpf;
+        CoupledSystems_PerBlock_OdeFunction<double>(S.sid, i, Fl, Xs[0], T, S.upsh + i * NUPa, S.sPAR, S.gPAR,
+                                                    S.igPAR, ua[0], iua[0], S.sACC, S.isACC, &cpt, &cpf);
+#pragma unroll
+        for (int k = 0; k < UD; k++) F[0][k] = Fl[k];
+        xu = Fl[IC];
+        rd = cpf * ra[0];                       /* v = rD a  */
+        x1 = cb[0] * (Xs[0][0] * Xs[0][0]);     /* u = b X1sq */
+        *post = make_double2(cb[0] * cpt, x1 * xu);
+    } else {
+#pragma unroll
+        for (int k = 0; k < UD; k++) F[0][k] = 0.0;
+        *post = make_double2(0.0, 0.0);
+    }
+    grp_sync(S);
+    double sums[2];
+    tmem_row_sums<2, 32 * G>(S.tm, c, S.vp, sums);
+    double r = 0.0, bval = 0.0;
+    if (valid) {
+        const double b = fma(rd, sums[0], xu);
+        const double ax = fma(rd, sums[1], xu);
+        r = b - ax;
+        bval = b;
+    }
+    /* q = A v = v + v_f (G (u v)), q~ = A^T vt = vt + u (G (v_f vt)) with u = b X1sq, v_f = rD a */
+    auto put = [&](const double (&v)[1], const double (&vt)[1]) {
+        *post = valid ? make_double2(x1 * v[0], rd * vt[0]) : make_double2(0.0, 0.0);
+    };
+    auto mul = [&](const double (&v)[1], const double (&vt)[1], double (&q)[1], double (&qt)[1]) {
+        double qs[2];
+        tmem_row_sums<2, 32 * G>(S.tm, c, S.vp, qs);
+        q[0] = valid ? fma(rd, qs[0], v[0]) : 0.0;
+        qt[0] = valid ? fma(x1, qs[1], vt[0]) : 0.0;
+    };
+    double rr[1] = {r}, xx[1] = {xu};
+    const double bb[1] = {bval};
+    const int done = bicg_iterate<1, G, REC>(S, P, bb, rr, xx, put, mul, capped);
+    F[0][IC] = xx[0];
     return done;
 }
 
@@ -1675,6 +1849,8 @@ __device__ __forceinline__ int rhs_eval(const Sys<U, G>& S, const DeviceProblem&
         return coupled_rhs_quad<G, REC>(S, P, T, Xs, F, ua, iua, capped);
     } else if constexpr (RHS == 0) {
         return coupled_rhs<U, G, REC>(S, P, T, Xs, F, up, ua, iua, capped);
+    } else if constexpr (RHS == 4 && U == 1) {
+        return coupled_rhs_symquad<G, REC>(S, P, T, Xs, F, ua, iua, ra, cb, capped);
     } else if constexpr (RHS == 3 || RHS == 4) {
         return coupled_rhs_sharedc<U, G, RHS == 4, REC>(S, P, T, Xs, F, up, ua, iua, ra, cb, capped);
     } else if constexpr (RHS == 5 || RHS == 6) {
@@ -2250,9 +2426,46 @@ __global__ void __launch_bounds__(RHS == 3 || RHS == 4 || RHS == 7 || G > 1 ? 25
     S.bar = 1u + (unsigned)slot;
     S.xsel = 0;
     S.tot = P.total_units;
+    constexpr bool TMEM = tmem_columns<U, RHS, G>(G) > 0;
+    __shared__ uint32_t tmem_base;
+    const uint32_t tmem_cols = tmem_columns<U, RHS, G>((int)blockDim.x >> 5);
+    S.tm = 0;
+    if constexpr (TMEM) {
+        if (wib == 0) tmem::alloc(&tmem_base, tmem_cols);
+        tmem::fence_before_sync();
+        __syncthreads();
+        tmem::fence_after_sync();
+        /* the lanes of this warp's quarter; four warps lie side by side, with RHS 0 the next four behind them */
+        S.tm = tmem_base + ((uint32_t)(32 * (wib & 3)) << 16) + (RHS == 0 ? (uint32_t)(4 * 32 * G * (wib >> 2)) : 0u);
+    }
+    if constexpr (RHS == 4 && U == 1) {
+        /* this lane's share of the launch's shared matrix, zero-padded: stored by the CTA's first four warps */
+        const int s0 = P.order[0];
+        const int n0 = P.units[s0];
+        const double* Cg = P.coupling + P.coupling_offset[s0];
+        const int c = lane >> 3, row0 = 32 * S.wis + (lane & 7);
+        if (wib < 4) {
+            for (int ch = 0; ch < 32 * G / 16; ch++) {
+                tmem::Chunk m;
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int j = 16 * ch + 4 * e + c;
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        m.set(4 * e + k,
+                              row0 + 8 * k < n0 && j < n0 ? __ldg(Cg + row0 + 8 * k + (int64_t)j * n0) : 0.0);
+                }
+                m.store(S.tm + 32 * ch);
+            }
+            tmem::wait_stores();
+        }
+        tmem::fence_before_sync();
+        __syncthreads();
+        tmem::fence_after_sync();
+    }
     if constexpr (RHS == 3 || RHS == 4) {
-        /* one copy of the launch's shared coupling matrix per CTA, zero-padded */
-        using SM = SharedCSmem<U, G>;
+        /* one copy of the launch's shared coupling matrix per CTA, zero-padded (none in shared memory with TMEM) */
+        using SM = SharedCSmem<U, G, RHS == 4>;
         constexpr int LDC = SM::LDC;
         const int s0 = P.order[0];
         const int n0 = P.units[s0];
@@ -2365,8 +2578,12 @@ __global__ void __launch_bounds__(RHS == 3 || RHS == 4 || RHS == 7 || G > 1 ? 25
             for (int c = lane; c < NISA; c += 32) S.isACC[c] = P.isacc[(int64_t)c * P.n_systems + sid];
         }
         if constexpr (RHS == 0 && U == 1) {
-            /* the rows and columns beyond N read as zeros (a right-hand side writes only the others) */
-            for (int idx = 32 * S.wis + lane; idx < WarpSmem<U, G>::W_DOUBLES; idx += 32 * G) S.W[idx] = 0.0;
+            /* stage the system's coupling matrix, zero-padded and swizzled (see coupled_rhs_quad) */
+            constexpr int NM = 32 * G;
+            const int r = 32 * S.wis + lane;
+#pragma unroll 8
+            for (int c = 0; c < NM; c++)
+                S.W[(r ^ quad_swizzle(c)) + c * NM] = (r < S.N && c < S.N) ? __ldg(S.C + r + (int64_t)c * S.N) : 0.0;
         }
         if constexpr (RHS == 5 || RHS == 6) {
             /* rows 2r, 2r + 1 of the shared symmetric matrix at the columns 4t + 2h + e of lane 2r + h, zero-padded */
@@ -2444,6 +2661,15 @@ __global__ void __launch_bounds__(RHS == 3 || RHS == 4 || RHS == 7 || G > 1 ? 25
             }
         }
         grp_sync(S);
+    }
+    if constexpr (TMEM) {
+        /* every warp's loads have been waited for */
+        tmem::fence_before_sync();
+        __syncthreads();
+        if (wib == 0) {
+            tmem::fence_after_sync();
+            tmem::dealloc(tmem_base, tmem_cols);
+        }
     }
 }
 

@@ -33,12 +33,25 @@
         return cudaGetLastError();                                                                            \
     }
 
+/* at least the share of an SM's shared memory (228 KB, 1 KB reserved and a few words static per
+ * CTA) that the CTA takes of its 512 columns of tensor memory: whatever launches share an SM, the
+ * columns of the CTAs that fit are there, and an allocation never waits for another CTA */
+inline size_t tmem_fit(size_t smem, int columns) {
+    if (columns == 0) return smem;
+    size_t least = (size_t)228 * 1024 * columns / 512 - 1024 - 256;
+    if (least > 226 * 1024) least = 226 * 1024;
+    return smem > least ? smem : least;
+}
+
 /* per-system shared memory (operator or staged matrix per system) */
-#define BES_SMEM_WARP(U_, G_) (size_t)(warps / (G_)) * WarpSmem<U_, G_>::BYTES
+#define BES_SMEM_WARP(U_, G_) \
+    tmem_fit((size_t)(warps / (G_)) * WarpSmem<U_, G_>::BYTES, tmem_columns<U_, ((U_) == 1 && (G_) > 1 ? 0 : 1), G_>(warps))
 /* per-system band of the coupling matrix, sized by the run-time band width */
 #define BES_SMEM_BAND(G_) (size_t)(warps / (G_)) * (size_t)BandSmem<G_>::doubles(band) * 8
 /* one staged matrix per CTA plus per-system vectors */
-#define BES_SMEM_SHARED(U_, G_) \
-    (size_t)SharedCSmem<U_, G_>::C_BYTES + (size_t)(warps / (G_)) * SharedCSmem<U_, G_>::WARP_BYTES
+#define BES_SMEM_SHARED(U_, G_, SYM_)                                    \
+    tmem_fit((size_t)SharedCSmem<U_, G_, SYM_>::C_BYTES +                \
+                 (size_t)(warps / (G_)) * SharedCSmem<U_, G_, SYM_>::WARP_BYTES, \
+             tmem_columns<U_, (SYM_) ? 4 : 3, G_>(warps))
 
 #endif

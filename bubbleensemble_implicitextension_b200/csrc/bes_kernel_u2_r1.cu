@@ -4,6 +4,6 @@
 
 namespace bes {
 BES_KERNEL_VARIANT(2, 0, 1, 1, BES_SMEM_WARP(2, 1))
-BES_KERNEL_VARIANT(2, 3, 1, 1, BES_SMEM_SHARED(2, 1))
-BES_KERNEL_VARIANT(2, 4, 1, 1, BES_SMEM_SHARED(2, 1))
+BES_KERNEL_VARIANT(2, 3, 1, 1, BES_SMEM_SHARED(2, 1, false))
+BES_KERNEL_VARIANT(2, 4, 1, 1, BES_SMEM_SHARED(2, 1, true))
 }  // namespace bes

@@ -4,6 +4,6 @@
 
 namespace bes {
 BES_KERNEL_VARIANT(4, 0, 1, 1, BES_SMEM_WARP(4, 1))
-BES_KERNEL_VARIANT(4, 3, 1, 1, BES_SMEM_SHARED(4, 1))
-BES_KERNEL_VARIANT(4, 4, 1, 1, BES_SMEM_SHARED(4, 1))
+BES_KERNEL_VARIANT(4, 3, 1, 1, BES_SMEM_SHARED(4, 1, false))
+BES_KERNEL_VARIANT(4, 4, 1, 1, BES_SMEM_SHARED(4, 1, true))
 }  // namespace bes
