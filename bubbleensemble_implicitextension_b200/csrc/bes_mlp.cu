@@ -8,7 +8,14 @@
  *   - master weights and biases in FP32, Adam moments in FP32;
  *   - weights used by the kernels rounded to BF16 after every update;
  *   - layer inputs (activations) stored in BF16, pre-activations in FP32;
- *   - every product accumulated in FP32 (tiled GEMM, 64 x 64 tiles).
+ *   - every product accumulated in FP32, each output one fma chain over the
+ *     inner index from zero, whatever kernel forms it.
+ * Networks of up to 256 units a layer run fused: mlp_rows takes a tile of rows
+ * through every layer (and, for training, back through every input gradient)
+ * with the activations in shared memory, mlp_weight_grads forms every layer's
+ * weight and bias gradients and the loss in one launch.  A minibatch of 512 is
+ * bound by launches and by filling the chip, not by its 0.6 GFLOP.  Wider
+ * networks run layer by layer (gemm_kernel, 64 x 64 tiles).
  * GELU is the tanh form 0.5 x (1 + tanh(sqrt(2/pi) (x + 0.044715 x^3))).
  * Parameter vector layout (get/set): for each layer, W [fan_out][fan_in]
  * row-major, then b [fan_out].
@@ -189,6 +196,351 @@ __global__ void refresh_bf16(const float* __restrict__ w, int64_t count, const u
     if (i < count && is_weight[i]) wb[wb_index[i]] = __float2bfloat16_rn(w[i]);
 }
 
+/* ---- fused kernels (every layer at most FUSED wide) ---------------------------------------- */
+
+constexpr int FUSED = 256;      /* widest layer; also the threads of a CTA */
+constexpr int MAX_LAYERS = 16;
+constexpr int SLAB = 32;        /* inner indices of a weight slab in shared memory */
+constexpr int MAX_OUT = 16;     /* widest last layer */
+constexpr int GT = 32;          /* weight-gradient tile */
+
+/* what the fused kernels see of a network */
+struct NetView {
+    int n_layers, n_in, n_out;
+    int fin[MAX_LAYERS], fout[MAX_LAYERS];
+    const __nv_bfloat16* w[MAX_LAYERS];   /* [fan_out][fan_in] */
+    const float* bias[MAX_LAYERS];
+    __nv_bfloat16* act[MAX_LAYERS];       /* layer inputs [batch][fan_in] (training) */
+    float* pre[MAX_LAYERS];               /* pre-activations [batch][fan_out], then their gradients (training) */
+    float* dw[MAX_LAYERS];
+    float* db[MAX_LAYERS];
+    const float *in_mean, *in_std, *out_mean, *out_std;
+};
+
+/* two fmas at once: (d.x, d.y) += (a.x b.x, a.y b.y), each rounded as fmaf rounds it */
+__device__ __forceinline__ void fma2(float2& d, float2 a, float2 b) {
+    unsigned long long x = *reinterpret_cast<unsigned long long*>(&d);
+    asm("fma.rn.f32x2 %0, %1, %2, %0;"
+        : "+l"(x)
+        : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
+    d = *reinterpret_cast<float2*>(&x);
+}
+
+template <int N>
+struct alignas(4 * N) Vec {
+    float v[N];
+};
+
+/* acc[i][j] = sum_k A[k][row + i] B(k, col + j) for this thread's RT rows and CT columns, k in order.
+ * A is in shared memory ([k][ROWS]); B comes in slabs of SLAB inner indices through Bs.
+ * TRANSPOSED: B(k, n) = w[n ldw + k] (forward), else w[k ldw + n] (input gradient); n < N, zeros beyond. */
+template <int RT, int CT, bool TRANSPOSED>
+__device__ __forceinline__ void tile_product(const float* As, float (*Bs)[SLAB][FUSED], const __nv_bfloat16* __restrict__ w,
+                                             int ldw, int K, int N, int row, int col, float2 (&acc)[RT / 2][CT]) {
+    constexpr int ROWS = RT * CT;
+    const int tid = threadIdx.x;
+#pragma unroll
+    for (int i = 0; i < RT / 2; i++)
+#pragma unroll
+        for (int j = 0; j < CT; j++) acc[i][j] = make_float2(0.f, 0.f);
+    /* the next slab travels in registers while this one is used: eight weights a load where the rows
+     * of w allow it (forward: four lanes a row of w, 64 rows a pass; input gradient: eight columns of
+     * every eighth row).  Column n of inner index k stands at n ^ slot(k), so that the forward's
+     * transposing stores (eight n and four octets of k a warp) meet no bank conflicts and a reader's
+     * neighbouring columns stay neighbours. */
+    auto slot = [](int k) { return 8 * ((k >> 3) & 3); };
+    const bool aligned = (ldw & 7) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
+    alignas(16) __nv_bfloat16 next[SLAB];
+    const int n8 = 8 * (tid & 31), k8 = tid >> 5;      /* input gradient */
+    const int n64 = tid >> 2, k4 = 8 * (tid & 3);      /* forward */
+    auto fetch = [&](int k0) {
+        if (aligned && k0 + SLAB <= K) {
+#pragma unroll
+            for (int q = 0; q < SLAB / 8; q++) {
+                uint4 v = make_uint4(0u, 0u, 0u, 0u);
+                if (TRANSPOSED ? n64 + 64 * q < N : n8 < N)
+                    v = __ldg(reinterpret_cast<const uint4*>(TRANSPOSED ? w + (int64_t)(n64 + 64 * q) * ldw + k0 + k4
+                                                                        : w + (int64_t)(k0 + k8 + 8 * q) * ldw + n8));
+                *reinterpret_cast<uint4*>(next + 8 * q) = v;
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < SLAB; q++) {
+                const int k = k0 + q;
+                next[q] = __float2bfloat16_rn(0.f);
+                if (tid < N && k < K) next[q] = TRANSPOSED ? w[(int64_t)tid * ldw + k] : w[(int64_t)k * ldw + tid];
+            }
+        }
+    };
+    fetch(0);
+    int buf = 0;
+    for (int k0 = 0; k0 < K; k0 += SLAB, buf ^= 1) {
+        if (aligned && k0 + SLAB <= K) {
+#pragma unroll
+            for (int q = 0; q < SLAB / 8; q++) {
+                if (TRANSPOSED) {
+#pragma unroll
+                    for (int e = 0; e < 8; e++) Bs[buf][k4 + e][(n64 + 64 * q) ^ k4] = __bfloat162float(next[8 * q + e]);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 8; e += 4) {
+                        const __nv_bfloat16* f = next + 8 * q + e;
+                        *reinterpret_cast<float4*>(&Bs[buf][k8 + 8 * q][(n8 + e) ^ slot(k8 + 8 * q)]) = make_float4(
+                            __bfloat162float(f[0]), __bfloat162float(f[1]), __bfloat162float(f[2]), __bfloat162float(f[3]));
+                    }
+                }
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < SLAB; q++) Bs[buf][q][tid ^ slot(q)] = __bfloat162float(next[q]);
+        }
+        if (k0 + SLAB < K) fetch(k0 + SLAB);
+        __syncthreads();
+        auto one = [&](int q) {
+            Vec<RT> a = *reinterpret_cast<const Vec<RT>*>(As + (k0 + q) * ROWS + row);
+            Vec<CT> b = *reinterpret_cast<const Vec<CT>*>(&Bs[buf][q][col ^ slot(q)]);
+#pragma unroll
+            for (int j = 0; j < CT; j++)
+#pragma unroll
+                for (int i = 0; i < RT / 2; i++)
+                    fma2(acc[i][j], make_float2(a.v[2 * i], a.v[2 * i + 1]), make_float2(b.v[j], b.v[j]));
+        };
+        if (k0 + SLAB <= K) {
+#pragma unroll
+            for (int q = 0; q < SLAB; q++) one(q);
+        } else {
+            for (int q = 0; q < K - k0; q++) one(q);
+        }
+    }
+    __syncthreads();   /* As and Bs are free */
+}
+
+/* A tile of RT CT rows through the network: 256 threads as CT groups of RT rows, each thread CT
+ * columns.  A thread's fmas per inner index need RT + CT words of shared memory, so large batches
+ * take 8 x 4 (32 rows a CTA); small ones fewer rows a CTA, to fill the chip.
+ * TRAIN: stores the layer inputs, then goes back: the gradients of every layer's pre-activations
+ * (in place of the pre-activations) and the squared errors.
+ * B200, width 256, depth 4: 16384 points 1000 -> 221 us, a training step of 512 rows with its
+ * gradients read back 740 -> 189 us (the layers as separate GEMM and elementwise launches before). */
+template <int RT, int CT, bool TRAIN>
+__global__ void __launch_bounds__(FUSED, 2) mlp_rows(NetView net, const float* __restrict__ x, int batch,
+                                                      float* __restrict__ y, const float* __restrict__ target,
+                                                      float* __restrict__ err) {
+    constexpr int ROWS = RT * CT;
+    extern __shared__ __align__(16) float smem[];
+    float* As = smem;                                                          /* [FUSED][ROWS] */
+    float(*Bs)[SLAB][FUSED] = reinterpret_cast<float(*)[SLAB][FUSED]>(smem + FUSED * ROWS);   /* [2][SLAB][FUSED] */
+    const int tid = threadIdx.x;
+    const int row = (tid / (FUSED / CT)) * RT, col = (tid % (FUSED / CT)) * CT;
+    const int64_t b0 = (int64_t)blockIdx.x * ROWS;
+    const int rows = (int)min((int64_t)ROWS, batch - b0);
+    for (int e = tid; e < ROWS * net.n_in; e += FUSED) {
+        const int r = e / net.n_in, f = e % net.n_in;
+        __nv_bfloat16 v = __float2bfloat16_rn(0.f);
+        if (r < rows) {
+            v = __float2bfloat16_rn((x[b0 * net.n_in + e] - net.in_mean[f]) / net.in_std[f]);
+            if (TRAIN) net.act[0][b0 * net.n_in + e] = v;
+        }
+        As[f * ROWS + r] = __bfloat162float(v);
+    }
+    __syncthreads();
+    const int last = net.n_layers - 1;
+    for (int l = 0; l < last; l++) {
+        const int O = net.fout[l];
+        float2 acc[RT / 2][CT];
+        tile_product<RT, CT, true>(As, Bs, net.w[l], net.fin[l], net.fin[l], O, row, col, acc);
+#pragma unroll
+        for (int j = 0; j < CT; j++) {
+            const int n = col + j;
+            if (n >= O) continue;
+            const float bias = net.bias[l][n];
+            Vec<RT> out;
+#pragma unroll
+            for (int i = 0; i < RT; i++) {
+                const float z = (i & 1 ? acc[i / 2][j].y : acc[i / 2][j].x) + bias;
+                const __nv_bfloat16 a = __float2bfloat16_rn(gelu_t(z));
+                out.v[i] = __bfloat162float(a);
+                if (TRAIN && row + i < rows) {
+                    net.pre[l][(b0 + row + i) * O + n] = z;
+                    net.act[l + 1][(b0 + row + i) * O + n] = a;
+                }
+            }
+            *reinterpret_cast<Vec<RT>*>(As + n * ROWS + row) = out;
+        }
+        __syncthreads();
+    }
+    /* the last layer has few columns: one thread an output */
+    const int K = net.fin[last], O = net.n_out;
+    float* dz = &Bs[0][0][0];   /* [n_out][ROWS] while As is still read */
+    for (int e = tid; e < ROWS * O; e += FUSED) {
+        const int r = e % ROWS, n = e / ROWS;
+        const __nv_bfloat16* wn = net.w[last] + (int64_t)n * K;
+        float s = 0.f;
+#pragma unroll 8
+        for (int k = 0; k < K; k++) s = fmaf(As[k * ROWS + r], __bfloat162float(wn[k]), s);
+        const float z = s + net.bias[last][n];
+        const int64_t at = (b0 + r) * O + n;
+        float g = 0.f;
+        if (r < rows) {
+            if (y) y[at] = z * net.out_std[n] + net.out_mean[n];
+            if (TRAIN) {
+                const float d = z - (target[at] - net.out_mean[n]) / net.out_std[n];
+                g = 2.f * d / (float)((int64_t)batch * O);
+                err[at] = d * d;
+                net.pre[last][at] = g;
+            }
+        }
+        if (TRAIN) dz[e] = g;
+    }
+    if constexpr (TRAIN) {
+        __syncthreads();
+        for (int e = tid; e < ROWS * O; e += FUSED) As[e] = dz[e];
+        __syncthreads();
+        for (int l = last; l > 0; l--) {
+            const int I = net.fin[l];
+            float2 acc[RT / 2][CT];
+            tile_product<RT, CT, false>(As, Bs, net.w[l], I, net.fout[l], I, row, col, acc);
+#pragma unroll
+            for (int j = 0; j < CT; j++) {
+                const int n = col + j;
+                if (n >= I) continue;
+                Vec<RT> out;
+#pragma unroll
+                for (int i = 0; i < RT; i++) {
+                    out.v[i] = 0.f;
+                    if (row + i < rows) {
+                        float* pre = net.pre[l - 1] + (b0 + row + i) * I + n;   /* this thread wrote it */
+                        out.v[i] = (i & 1 ? acc[i / 2][j].y : acc[i / 2][j].x) * gelu_dt(*pre);
+                        *pre = out.v[i];
+                    }
+                }
+                *reinterpret_cast<Vec<RT>*>(As + n * ROWS + row) = out;
+            }
+            __syncthreads();
+        }
+    }
+}
+
+/* Every layer's dW = dZ^T X and db = column sums of dZ, and the loss, as blocks of one launch: the
+ * tiles of all dW (GT x GT, a thread one row and four columns, the batch in slabs of GT rows), then the bias
+ * gradients (GT columns a block, a warp a column: lane-strided sums and a butterfly), then the loss. */
+struct GradPlan {
+    int first[MAX_LAYERS + 1];        /* first tile of each layer */
+    int first_bias[MAX_LAYERS + 1];   /* first bias block of each layer, after the tiles */
+};
+
+__global__ void __launch_bounds__(256) mlp_weight_grads(NetView net, GradPlan plan, int batch, const float* __restrict__ err,
+                                                        float* __restrict__ loss) {
+    __shared__ __align__(16) float As[2][GT][GT], Bs[2][GT][GT];
+    __shared__ float part[256];
+    const int tid = threadIdx.x, L = net.n_layers;
+    int blk = blockIdx.x;
+    if (blk < plan.first[L]) {
+        int l = 0;
+        while (blk >= plan.first[l + 1]) l++;
+        blk -= plan.first[l];
+        const int O = net.fout[l], I = net.fin[l], nt = (I + GT - 1) / GT;
+        const int o0 = (blk / nt) * GT, i0 = (blk % nt) * GT;
+        const float* __restrict__ dz = net.pre[l];
+        const __nv_bfloat16* __restrict__ act = net.act[l];
+        const int c = tid & 31, r = tid >> 5;   /* loads: column c of rows r, r + 8, .. */
+        const bool ina = o0 + c < O, inb = i0 + c < I;
+        const float* pa = dz + (int64_t)r * O + o0 + c;
+        const __nv_bfloat16* pb = act + (int64_t)r * I + i0 + c;
+        float fa[GT / 8], fb[GT / 8];
+        auto fetch = [&](int k0) {
+#pragma unroll
+            for (int q = 0; q < GT / 8; q++) {
+                const bool in = k0 + r + 8 * q < batch;
+                fa[q] = in && ina ? pa[(int64_t)(k0 + 8 * q) * O] : 0.f;
+                fb[q] = in && inb ? __bfloat162float(pb[(int64_t)(k0 + 8 * q) * I]) : 0.f;
+            }
+        };
+        /* this thread: row o0 + ty, columns i0 + 4 tx .. + 3 */
+        const int tx = tid & 7, ty = tid >> 3;
+        float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        fetch(0);
+        int buf = 0;
+        for (int k0 = 0; k0 < batch; k0 += GT, buf ^= 1) {
+#pragma unroll
+            for (int q = 0; q < GT / 8; q++) {
+                As[buf][r + 8 * q][c] = fa[q];
+                Bs[buf][r + 8 * q][c] = fb[q];
+            }
+            if (k0 + GT < batch) fetch(k0 + GT);
+            __syncthreads();
+            auto one = [&](int q) {
+                const float a = As[buf][q][ty];
+                const float4 b = *reinterpret_cast<const float4*>(&Bs[buf][q][4 * tx]);
+                fma2(acc[0], make_float2(a, a), make_float2(b.x, b.y));
+                fma2(acc[1], make_float2(a, a), make_float2(b.z, b.w));
+            };
+            if (k0 + GT <= batch) {
+#pragma unroll
+                for (int q = 0; q < GT; q++) one(q);
+            } else {
+                for (int q = 0; q < batch - k0; q++) one(q);
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+            const int o = o0 + ty, i = i0 + 4 * tx + b;
+            if (o < O && i < I) net.dw[l][(int64_t)o * I + i] = b & 1 ? acc[b / 2].y : acc[b / 2].x;
+        }
+        return;
+    }
+    blk -= plan.first[L];
+    if (blk < plan.first_bias[L]) {
+        int l = 0;
+        while (blk >= plan.first_bias[l + 1]) l++;
+        const int O = net.fout[l], o0 = (blk - plan.first_bias[l]) * GT;
+        const int lane = tid & 31, warp = tid >> 5;
+        const float* __restrict__ dz = net.pre[l];
+        float s[GT / 8];   /* columns o0 + warp + 8 q, rows lane, lane + 32, .. */
+#pragma unroll
+        for (int q = 0; q < GT / 8; q++) s[q] = 0.f;
+        float(*rows)[GT + 1] = reinterpret_cast<float(*)[GT + 1]>(&As[0][0][0]);   /* GT (GT + 1) <= 2 GT GT */
+        float next[GT / 8];
+        auto fetch = [&](int b) {
+#pragma unroll
+            for (int q = 0; q < GT / 8; q++) {
+                const int k = b + warp + 8 * q;
+                next[q] = k < batch && o0 + lane < O ? dz[(int64_t)k * O + o0 + lane] : 0.f;
+            }
+        };
+        fetch(0);
+        for (int b = 0; b < batch; b += GT) {
+            __syncthreads();
+#pragma unroll
+            for (int q = 0; q < GT / 8; q++) rows[warp + 8 * q][lane] = next[q];
+            if (b + GT < batch) fetch(b + GT);
+            __syncthreads();
+            if (b + lane < batch) {
+#pragma unroll
+                for (int q = 0; q < GT / 8; q++) s[q] += rows[lane][warp + 8 * q];
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < GT / 8; q++) {
+#pragma unroll
+            for (int off = 16; off >= 1; off >>= 1) s[q] += __shfl_xor_sync(0xffffffffu, s[q], off);
+            if (lane == 0 && o0 + warp + 8 * q < O) net.db[l][o0 + warp + 8 * q] = s[q];
+        }
+        return;
+    }
+    /* the loss, in the order of sum_errors' 256 partial sums */
+    const int64_t count = (int64_t)batch * net.n_out;
+    float s = 0.f;
+    for (int64_t i = tid; i < count; i += 256) s += err[i];
+    part[tid] = s;
+    __syncthreads();
+    for (int h = 128; h >= 1; h >>= 1) {
+        if (tid < h) part[tid] += part[tid + h];
+        __syncthreads();
+    }
+    if (tid == 0) loss[0] = part[0] / (float)count;
+}
+
 inline int blocks_for(int64_t n, int t) { return (int)((n + t - 1) / t); }
 
 }  // namespace
@@ -243,6 +595,59 @@ cudaError_t gemm(int M, int N, int K, const TA* A, int lda, const TB* B, int ldb
     dim3 grid((N + TILE - 1) / TILE, (M + TILE - 1) / TILE);
     gemm_kernel<TA, TB, A_T, B_T><<<grid, 256, 0, s>>>(M, N, K, A, lda, B, ldb, C, ldc);
     return cudaGetLastError();
+}
+
+/* may the network run in the fused kernels */
+bool fused(const bes_mlp* h) {
+    return h->width <= FUSED && h->n_in <= FUSED && h->n_out <= MAX_OUT && h->n_layers <= MAX_LAYERS;
+}
+
+NetView view(const bes_mlp* h) {
+    NetView v;
+    std::memset(&v, 0, sizeof v);
+    v.n_layers = h->n_layers;
+    v.n_in = h->n_in;
+    v.n_out = h->n_out;
+    for (int l = 0; l < h->n_layers; l++) {
+        v.fin[l] = h->fin[l];
+        v.fout[l] = h->fout[l];
+        v.w[l] = h->wb + h->wb_off[l];
+        v.bias[l] = h->master + h->b_off[l];
+        v.act[l] = h->act[l];
+        v.pre[l] = h->pre[l];
+        v.dw[l] = h->grad + h->w_off[l];
+        v.db[l] = h->grad + h->b_off[l];
+    }
+    v.in_mean = h->in_mean;
+    v.in_std = h->in_std;
+    v.out_mean = h->out_mean;
+    v.out_std = h->out_std;
+    return v;
+}
+
+template <int RT, int CT, bool TRAIN>
+cudaError_t launch_rows(const NetView& v, const float* x, int batch, float* y, const float* target, float* err,
+                        cudaStream_t s) {
+    constexpr int ROWS = RT * CT;
+    constexpr size_t smem = sizeof(float) * (FUSED * ROWS + 2 * SLAB * FUSED);
+    if (smem > 48 * 1024) {
+        cudaError_t e =
+            cudaFuncSetAttribute(mlp_rows<RT, CT, TRAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    mlp_rows<RT, CT, TRAIN><<<(batch + ROWS - 1) / ROWS, FUSED, smem, s>>>(v, x, batch, y, target, err);
+    return cudaGetLastError();
+}
+
+/* rows a CTA: as many as still give every SM a tile (see mlp_rows) */
+template <bool TRAIN>
+cudaError_t rows_of(const NetView& v, const float* x, int batch, float* y, const float* target, float* err,
+                    cudaStream_t s) {
+    const int sms = 148;   /* of a B200 */
+    if (batch <= 4 * sms) return launch_rows<4, 1, TRAIN>(v, x, batch, y, target, err, s);
+    if (batch <= 8 * sms) return launch_rows<4, 2, TRAIN>(v, x, batch, y, target, err, s);
+    if (batch <= 16 * sms) return launch_rows<4, 4, TRAIN>(v, x, batch, y, target, err, s);
+    return launch_rows<8, 4, TRAIN>(v, x, batch, y, target, err, s);
 }
 
 /* forward through every layer; y (device, may be null) gets the de-standardised outputs */
@@ -415,6 +820,10 @@ bes_status bes_mlp_get_gradients(bes_mlp* h, float* host, int64_t count) {
 bes_status bes_mlp_forward(bes_mlp* h, const float* x, int32_t batch, float* y, void* stream) {
     if (!h || !x || !y || batch < 1 || batch > h->max_batch) return BES_ERR_ARGUMENT;
     MLP_TRY(h, cudaSetDevice(h->device));
+    if (fused(h)) {
+        MLP_TRY(h, (rows_of<false>(view(h), x, batch, y, nullptr, nullptr, (cudaStream_t)stream)));
+        return BES_OK;
+    }
     return forward(h, x, batch, y, (cudaStream_t)stream);
 }
 
@@ -423,6 +832,25 @@ bes_status bes_mlp_backward(bes_mlp* h, const float* x, const float* target, int
     if (!h || !x || !target || batch < 1 || batch > h->max_batch) return BES_ERR_ARGUMENT;
     MLP_TRY(h, cudaSetDevice(h->device));
     cudaStream_t s = (cudaStream_t)stream;
+    if (fused(h)) {
+        const NetView v = view(h);
+        MLP_TRY(h, (rows_of<true>(v, x, batch, nullptr, target, h->err, s)));
+        GradPlan plan;
+        std::memset(&plan, 0, sizeof plan);
+        for (int l = 0; l < h->n_layers; l++) {
+            const int to = (h->fout[l] + GT - 1) / GT, ti = (h->fin[l] + GT - 1) / GT;
+            plan.first[l + 1] = plan.first[l] + to * ti;
+            plan.first_bias[l + 1] = plan.first_bias[l] + to;
+        }
+        const int blocks = plan.first[h->n_layers] + plan.first_bias[h->n_layers] + (loss_host ? 1 : 0);
+        mlp_weight_grads<<<blocks, 256, 0, s>>>(v, plan, batch, h->err, h->loss);
+        MLP_TRY(h, cudaGetLastError());
+        if (loss_host) {
+            MLP_TRY(h, cudaMemcpyAsync(loss_host, h->loss, 4, cudaMemcpyDeviceToHost, s));
+            MLP_TRY(h, cudaStreamSynchronize(s));
+        }
+        return BES_OK;
+    }
     bes_status st = forward(h, x, batch, nullptr, s);
     if (st) return st;
     const int L = h->n_layers;
