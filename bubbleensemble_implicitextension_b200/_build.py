@@ -19,7 +19,7 @@ INCLUDE = PKG.parent / "include"
 BUILD = PKG / "_build"
 LIB = PKG / "libbes.so"
 
-KERNEL_UNITS = [f"bes_kernel_{c}{r}.cu" for c in ("u1", "u2", "u4", "g2", "g4") for r in ("", "_r1")]
+KERNEL_UNITS = [f"bes_kernel_{c}{r}.cu" for c in ("u1", "t4", "u2", "u4", "g2", "g4", "d2", "d4") for r in ("", "_r1")]
 SOURCES = ["bes_api.cu", "bes_launch.cu", "bes_peak.cu", "bes_noalloc.cu", "bes_mlp.cu", *KERNEL_UNITS]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

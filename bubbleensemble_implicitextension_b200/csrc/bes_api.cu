@@ -381,10 +381,18 @@ struct ClassLaunch {
     int grid, wpb;
 };
 
+/* do the systems of up to 32 units run on teams */
+bool team_pays(const bes_solver* h) {
+    return bes::team_pays(std::min(h->active, h->n_systems),
+                          h->shared_coupling && h->class_shared[0] && h->class_symmetric[0], h->sm_count);
+}
+
 /* launch shape of one class (no stream work: safe before a capture) */
 bes_status plan_shape(bes_solver* h, int cls, int warps_per_system, int requested_wpb, ClassLaunch* L) {
     const bes::Variant v = bes::class_variant(cls, h->class0_all32, h->shared_coupling && h->class_shared[cls],
-                                         warps_per_system, h->class_symmetric[cls], h->bicg_recurrence, h->cbw);
+                                         warps_per_system, h->class_symmetric[cls], h->bicg_recurrence, h->cbw,
+                                         team_pays(h),
+                                         bes::dense_pays(cls, h->class_count[cls], h->sm_count));
     const int count = h->class_count[cls];
     if (bes::max_warps_per_block(v) < v.G)
         return fail(h, BES_ERR_CUDA, "solver kernel variant (U=%d, G=%d) does not fit in shared memory", v.U, v.G);
@@ -398,7 +406,8 @@ bes_status plan_shape(bes_solver* h, int cls, int warps_per_system, int requeste
     const int needed = (count + systems_per_cta - 1) / systems_per_cta;
     L->v = v;
     L->wpb = wpb;
-    L->grid = std::max(1, std::min(needed, per_sm * h->sm_count));
+    /* at least a CTA per SM while there are systems for it: slots that find none left end at once */
+    L->grid = std::max(1, std::min(std::max(needed, std::min(count, h->sm_count)), per_sm * h->sm_count));
     return BES_OK;
 }
 
@@ -1422,10 +1431,12 @@ bes_status bes_autotune(bes_solver* h, int32_t n_periods, int64_t step_cap, bes_
         if (h->class_count[cls] == 0) continue;
         float best = -1.0f;
         int best_wps = 0, best_wpb = 0;
-        for (int wps = 0; wps <= (cls == 0 ? 0 : 1) && !st; wps++) {
+        const bool team = team_pays(h);
+        for (int wps = 0; wps <= (cls == 0 && !team ? 0 : 1) && !st; wps++) {
             const bes::Variant v = bes::class_variant(cls, h->class0_all32,
                                                       h->shared_coupling && h->class_shared[cls], wps,
-                                                      h->class_symmetric[cls], h->bicg_recurrence, h->cbw);
+                                                      h->class_symmetric[cls], h->bicg_recurrence, h->cbw, team,
+                                                      bes::dense_pays(cls, h->class_count[cls], h->sm_count));
             const int cap = bes::max_warps_per_block(v);
             for (int wpb = v.G; wpb <= cap && !st; wpb *= 2) {
                 ClassLaunch L;

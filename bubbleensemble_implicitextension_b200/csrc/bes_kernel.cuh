@@ -78,14 +78,16 @@ constexpr int XCH_BUF = 2 * 128 + 8;
  * values of one or two vectors, each run padded by one double2 so that the
  * runs a load reads at once start in different banks */
 constexpr int RED_RUN = 18, RED_BUF = 4 * RED_RUN;
+/* warps of a team: one system of up to 32 units on TEAM warps (RHS > 10: the variant RHS - 10) */
+constexpr int TEAM = 4;
 /* Shared-memory doubles per system (G warps, U units per lane, NMAX = 32 U G
  * units): one matrix region (more than one unit per lane: the operator W, leading
  * dimension NMAX+1; one: the system's coupling matrix C, for one warp with the
  * part of W that A^T v reads), six broadcast vectors, the group's exchange buffers
  * (G > 1) or the warp's reduction buffers, the system-scope arrays, and the unit
  * parameters when each lane owns one unit (U = 1: in registers they crowd out
- * the BiCG state). */
-template <int U, int G = 1>
+ * the BiCG state).  T: the warps of a team, each with such a region. */
+template <int U, int G = 1, int T = 1>
 struct WarpSmem {
     static constexpr int NMAX = 32 * U * G;
     static constexpr bool ONE = U == 1 && G == 1;   /* one warp, one unit per lane */
@@ -96,12 +98,14 @@ struct WarpSmem {
     static constexpr int SYS_DOUBLES = NSPa + NSAa + NISAa;  /* ints stored in double slots */
     static constexpr int RED_DOUBLES = ONE ? 3 * RED_BUF : 0;   /* warp_sum32's buffers, two vectors by parity */
     static constexpr int UP_DOUBLES = U == 1 ? NMAX * NUPa : 0; /* unit parameters (one unit per lane) */
-    static constexpr int WT_DOUBLES = ONE ? NMAX * NMAX : 0;  /* each lane's column share of W */
+    static constexpr int WT_DOUBLES = ONE && T == 1 ? NMAX * NMAX : 0;  /* each lane's column share of W */
+    static constexpr int XT_DOUBLES = T > 1 ? 2 * T * 32 : 0;   /* a team's two exchange buffers (its first warp's are used) */
     /* per-system stride rounded up to 256 bytes: every system's vectors stay
      * 16-byte aligned for the double2 broadcast loads */
     static constexpr int K_DOUBLES = U == 1 ? 6 * UD * NMAX : 0;   /* stage derivatives (one unit per lane) */
     static constexpr int DOUBLES =
-        (W_DOUBLES + WT_DOUBLES + VEC_DOUBLES + XCH_DOUBLES + RED_DOUBLES + SYS_DOUBLES + UP_DOUBLES + K_DOUBLES + 31) / 32 * 32;
+        (W_DOUBLES + WT_DOUBLES + VEC_DOUBLES + XCH_DOUBLES + RED_DOUBLES + SYS_DOUBLES + UP_DOUBLES + K_DOUBLES + XT_DOUBLES +
+         31) / 32 * 32;
     static constexpr int BYTES = DOUBLES * 8;
     static_assert(DOUBLES % 2 == 0 && W_DOUBLES % 2 == 0 && NMAX % 2 == 0,
                   "broadcast vectors must start on 16-byte boundaries");
@@ -222,6 +226,10 @@ struct Sys {
     double* upsh;      /* unit parameters of the register-operator variant: unit i at upsh[i * NUP] */
     double* xch;       /* the group's exchange buffers (G > 1), or warp_sum32's (U = G = 1) */
     double *tpar, *rdpar;   /* vectors split by parity (register-operator variants): entry i at par_slot(i) */
+    int tw;            /* this warp's place in its team (T > 1), else 0 */
+    bool lead;         /* the warp that writes the system's results: a team's first, else every warp */
+    double* xt;        /* the team's exchange buffers */
+    mutable int tsel;  /* which of them is next */
     uint32_t tm;       /* this warp's lanes of the system's (RHS 0) or the CTA's (RHS 4) columns in tensor memory */
     double* flag;      /* the group's exit-vote words, one per warp (G > 1) */
     mutable int xsel;  /* which of the two exchange (or warp_sum32) buffers is next */
@@ -1718,6 +1726,177 @@ __device__ __forceinline__ int coupled_rhs_regsym(const Sys<1>& S, const DeviceP
 }
 
 /* ---------------------------------------------------------------------------
+ * Systems of up to 32 units on a team of four warps, for launches of so few
+ * systems that warps are to spare (RHS 11, 12: own matrix; 15, 16: shared symmetric
+ * matrix with unit factors; the even ones without N guards).  Every warp of the
+ * team integrates the whole system, in private registers and shared memory, from
+ * the same values to the same bits -- every decision included -- and only the
+ * products, half of a BiCG iteration on one warp, are divided: warps 0 and 1 form
+ * q, warps 2 and 3 q~, each over two of its four chains (of the column tree: one
+ * parity of the rows), lane l for unit l.  Each posts its partial sums in the
+ * team's exchange buffer, one named barrier, and all read them.  The two buffers
+ * alternate, so one is rewritten only after a later exchange's barrier.  The
+ * host's rule (team_pays) says for how many systems. */
+__device__ __forceinline__ double* team_buffer(const Sys<1>& S) {
+    double* b = S.xt + (S.tsel & 1) * (TEAM * 32);
+    S.tsel++;
+    return b;
+}
+__device__ __forceinline__ void team_sync(const Sys<1>& S) {
+    asm volatile("bar.sync %0, %1;" ::"r"(S.bar), "r"(32 * TEAM) : "memory");
+}
+/* warp 0's value to the whole team */
+__device__ __forceinline__ int team_share(const Sys<1>& S, int v) {
+    double* x = team_buffer(S);
+    if (S.tw == 0 && S.lane == 0) x[0] = (double)v;
+    team_sync(S);
+    return (int)x[0];
+}
+/* the partial sums of the four warps: first = (warp 0's + warp 1's), second = (warp 2's + warp 3's) */
+__device__ __forceinline__ void team_exchange(const Sys<1>& S, double partial, double& first, double& second) {
+    double* x = team_buffer(S);
+    x[32 * S.tw + S.lane] = partial;
+    team_sync(S);
+    first = x[S.lane] + x[32 + S.lane];
+    second = x[64 + S.lane] + x[96 + S.lane];
+}
+
+template <bool SYM, int NFIX, int REC>
+__device__ __forceinline__ int coupled_rhs_team(const Sys<1>& S, const DeviceProblem& P, double T, double (&Xs)[1][UD],
+                                                double (&F)[1][UD], double (&ua)[1][NUAa], int (&iua)[1][NIUAa],
+                                                const double (&ra)[1], const double (&cb)[1], const double (&g)[32],
+                                                bool& capped) {
+    constexpr int LDC = WarpSmem<1>::LDW;
+    const int N = NFIX ? NFIX : S.N;
+    const int i = S.lane;
+    const int h = S.tw & 1;           /* chains 2h, 2h + 1, or the rows of parity h */
+    const bool second = S.tw >= 2;    /* forms q~ */
+    const bool valid = i < N;
+    double xu = 0.0, rd = 0.0, x1 = 0.0, cp = 0.0;
+    __syncwarp();
+    if (valid) {
+        double Fl[UD], cpt, cpf;
+        CoupledSystems_PerBlock_OdeFunction<double>(S.sid, i, Fl, Xs[0], T, S.upsh + i * NUPa, S.sPAR, S.gPAR,
+                                                    S.igPAR, ua[0], iua[0], S.sACC, S.isACC, &cpt, &cpf);
+#pragma unroll
+        for (int k = 0; k < UD; k++) F[0][k] = Fl[k];
+        xu = Fl[IC];
+        rd = SYM ? cpf * ra[0] : cpf;                                          /* v = rD a  */
+        x1 = SYM ? cb[0] * (Xs[0][0] * Xs[0][0]) : Xs[0][0] * Xs[0][0];        /* u = b X1sq */
+        cp = SYM ? cb[0] * cpt : cpt;
+    } else {
+#pragma unroll
+        for (int k = 0; k < UD; k++) F[0][k] = 0.0;
+    }
+    const double2* vp2 = reinterpret_cast<const double2*>(S.vp) + h;
+    const double2* tp2 = reinterpret_cast<const double2*>(S.tpar + h * RED_RUN);
+    const int tslot = par_slot(i);
+    double w[16];   /* this lane's 16 entries of G or of W */
+    /* this warp's chains of row i of w against the vector posted at vp */
+    auto row_part = [&]() -> double {
+        double s[2] = {0.0, 0.0};
+        column_groups<NFIX>(N, [&](int t) {
+            const double2 a = vp2[2 * t];
+            s[0] = fma(w[2 * t], a.x, s[0]);
+            s[1] = fma(w[2 * t + 1], a.y, s[1]);
+        });
+        return s[0] + s[1];
+    };
+    double bsum, asum;
+    if constexpr (SYM) {
+#pragma unroll
+        for (int k = 0; k < 16; k++) w[k] = g[k];
+        S.vp[i] = second ? x1 * xu : cp;
+        __syncwarp();
+        team_exchange(S, row_part(), bsum, asum);
+    } else {
+        S.vx1[i] = x1;
+        S.vxu[i] = xu;
+        S.vcpt[i] = cp;
+        S.rdpar[tslot] = rd;
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 16; k++) w[k] = 0.0;
+        const double* C = S.W;   /* C[i][j] at i + j * LDC, zero-padded */
+        double bs[2] = {0.0, 0.0}, as[2] = {0.0, 0.0};
+        if (!second) {
+            const double2* vx1_2 = reinterpret_cast<const double2*>(S.vx1) + h;
+            const double2* vcpt2 = reinterpret_cast<const double2*>(S.vcpt) + h;
+            const double2* vxu2 = reinterpret_cast<const double2*>(S.vxu) + h;
+            column_groups<NFIX>(N, [&](int t) {
+                const double2 x1p = vx1_2[2 * t], cpp = vcpt2[2 * t], xup = vxu2[2 * t];
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const double c = C[i + (4 * t + 2 * h + e) * LDC];
+                    const double x1j = e ? x1p.y : x1p.x;
+                    bs[e] = fma(c, e ? cpp.y : cpp.x, bs[e]);
+                    as[e] = fma(c * x1j, e ? xup.y : xup.x, as[e]);
+                    w[2 * t + e] = (rd * c) * x1j;
+                }
+            });
+        } else {
+            const double2* rdp2 = reinterpret_cast<const double2*>(S.rdpar + h * RED_RUN);
+            column_groups<NFIX>(N, [&](int t) {
+                const double2 rdk = rdp2[t];
+#pragma unroll
+                for (int e = 0; e < 2; e++)
+                    w[2 * t + e] = ((e ? rdk.y : rdk.x) * C[4 * t + 2 * e + h + i * LDC]) * x1;
+            });
+        }
+        double* x = team_buffer(S);
+        if (!second) {
+            x[32 * h + i] = bs[0] + bs[1];
+            x[64 + 32 * h + i] = as[0] + as[1];
+        }
+        team_sync(S);
+        bsum = x[i] + x[32 + i];
+        asum = x[64 + i] + x[96 + i];
+    }
+    double r = 0.0, bval = 0.0;
+    if (valid) {
+        const double b = fma(rd, bsum, xu);
+        const double ax = fma(rd, asum, xu);
+        r = b - ax;
+        bval = b;
+    }
+    auto put = [&](const double (&v)[1], const double (&vt)[1]) {
+        if constexpr (SYM) S.vp[i] = valid ? (second ? rd * vt[0] : x1 * v[0]) : 0.0;
+        else if (!second) S.vp[i] = v[0];
+        else S.tpar[tslot] = vt[0];
+    };
+    auto mul = [&](const double (&v)[1], const double (&vt)[1], double (&qo)[1], double (&qto)[1]) {
+        double part, qs, qts;
+        if (SYM || !second) {
+            part = row_part();
+        } else {
+            double u[16];
+#pragma unroll
+            for (int k = 0; k < 16; k++) u[k] = 0.0;
+            column_groups<NFIX>(N, [&](int t) {
+                const double2 c = tp2[t];
+                u[2 * t] = w[2 * t] * c.x;
+                u[2 * t + 1] = w[2 * t + 1] * c.y;
+            });
+            auto leaf = [&](int k) -> double { return u[k]; };
+            part = TreeSum<1, 16>::run(0, leaf);
+        }
+        team_exchange(S, part, qs, qts);
+        if constexpr (SYM) {
+            qo[0] = valid ? fma(rd, qs, v[0]) : 0.0;
+            qto[0] = valid ? fma(x1, qts, vt[0]) : 0.0;
+        } else {
+            qo[0] = valid ? v[0] + qs : 0.0;
+            qto[0] = valid ? vt[0] + qts : 0.0;
+        }
+    };
+    double rr[1] = {r}, xx[1] = {xu};
+    const double bb[1] = {bval};
+    const int done = bicg_iterate<1, 1, REC>(S, P, bb, rr, xx, put, mul, capped);
+    F[0][IC] = xx[0];
+    return done;
+}
+
+/* ---------------------------------------------------------------------------
  * Coupled right-hand side for banded coupling storage (RHS = 7; the
  * reference's CBW modes, Steppers.cuh:586-641, whose implicit products read
  * full storage, :660,692): only the wrapping band of nd = min(2 bw + 1, N)
@@ -1853,6 +2032,8 @@ __device__ __forceinline__ int rhs_eval(const Sys<U, G>& S, const DeviceProblem&
         return coupled_rhs_symquad<G, REC>(S, P, T, Xs, F, ua, iua, ra, cb, capped);
     } else if constexpr (RHS == 3 || RHS == 4) {
         return coupled_rhs_sharedc<U, G, RHS == 4, REC>(S, P, T, Xs, F, up, ua, iua, ra, cb, capped);
+    } else if constexpr (RHS > 10) {
+        return coupled_rhs_team<(RHS > 14), RHS % 2 == 0 ? 32 : 0, REC>(S, P, T, Xs, F, ua, iua, ra, cb, grow, capped);
     } else if constexpr (RHS == 5 || RHS == 6) {
         static_assert(U == 1 && G == 1, "the register-resident operator needs one unit per lane");
         return coupled_rhs_regsym<RHS == 6 ? 32 : 0, REC>(S, P, T, Xs, F, ua, iua, ra, cb, grow, capped);
@@ -2059,7 +2240,7 @@ template <int U, int G>
 __device__ __forceinline__ void store_dense(const Sys<U, G>& S, const DeviceProblem& P, const Lane<U>& L,
                                             int& idx, int update_do, int update, int& skipped,
                                             double& do_time, double T, double TD1) {
-    if (update_do == 1 && idx < P.ndo) {
+    if (update_do == 1 && idx < P.ndo && S.lead) {
 #pragma unroll
         for (int m = 0; m < U; m++) {
             const int i = S.unit(m);
@@ -2082,7 +2263,7 @@ __device__ __forceinline__ void store_dense(const Sys<U, G>& S, const DeviceProb
 /* ---------------------------------------------------------------------------
  * One reference Solve() of one system (Solver.cuh:82-648). */
 template <int U, int RHS, int G, int REC>
-__device__ void run_period(const Sys<U, G>& S, const DeviceProblem& P, Lane<U>& L, Counters& cnt,
+__device__ __forceinline__ void run_period(const Sys<U, G>& S, const DeviceProblem& P, Lane<U>& L, Counters& cnt,
                            double (&TD)[2], double& T, int& do_idx) {
     const double TD1 = TD[1];
     double dt = P.dt0, newdt = P.dt0;
@@ -2363,6 +2544,7 @@ __device__ void run_period(const Sys<U, G>& S, const DeviceProblem& P, Lane<U>& 
  * periods, so nothing stays in registers across a period. */
 template <int U, int G>
 __device__ __forceinline__ void analysis_start(const Sys<U, G>& S, const DeviceProblem& P, const Lane<U>& L) {
+    if (!S.lead) return;
 #pragma unroll
     for (int m = 0; m < U; m++) {
         const int i = S.unit(m);
@@ -2381,6 +2563,7 @@ __device__ __forceinline__ void analysis_start(const Sys<U, G>& S, const DeviceP
 template <int U, int G>
 __device__ __forceinline__ void analysis_period_end(const Sys<U, G>& S, const DeviceProblem& P, const Lane<U>& L,
                                                     int per) {
+    if (!S.lead) return;
 #pragma unroll
     for (int m = 0; m < U; m++) {
         const int i = S.unit(m);
@@ -2410,9 +2593,13 @@ __device__ __forceinline__ void analysis_period_end(const Sys<U, G>& S, const De
  * (both BiCG products as row sums from one read of each entry).  G > 1 runs
  * one unit per lane (U = 1) and
  * exchanges the group's values through shared memory and a named barrier per
- * system slot (barrier 0 is left to __syncthreads). */
-template <int U, int RHS, int G, int REC>
-__global__ void __launch_bounds__(RHS == 3 || RHS == 4 || RHS == 7 || G > 1 ? 256 : 128, 1) bes_ensemble_kernel(DeviceProblem P) {
+ * system slot (barrier 0 is left to __syncthreads).  V > 20 is RHS V - 20 compiled
+ * for sixteen warps an SM (128 registers a thread), V = RHS otherwise.  RHS > 10 runs the variant
+ * RHS - 10 of a system of up to 32 units on a team of warps (coupled_rhs_team). */
+template <int U, int V, int G, int REC>
+__global__ void __launch_bounds__(V > 20 ? 512 : V == 3 || V == 4 || V == 7 || V > 10 || G > 1 ? 256 : 128, 1)
+    bes_ensemble_kernel(DeviceProblem P) {
+    constexpr int RHS = V > 20 ? V - 20 : V;
     static_assert(G == 1 || U == 1, "multi-warp systems run one unit per lane");
     static_assert(G == 1 || (RHS != 1 && RHS != 2 && RHS != 5 && RHS != 6),
                   "the register-resident operators are single-warp");
@@ -2423,7 +2610,11 @@ __global__ void __launch_bounds__(RHS == 3 || RHS == 4 || RHS == 7 || G > 1 ? 25
     Sys<U, G> S;
     S.lane = lane;
     S.wis = wib % G;
-    S.bar = 1u + (unsigned)slot;
+    S.tw = RHS > 10 ? wib % TEAM : 0;
+    S.lead = S.tw == 0;
+    S.xt = nullptr;
+    S.tsel = 0;
+    S.bar = 1u + (unsigned)(RHS > 10 ? wib / TEAM : slot);
     S.xsel = 0;
     S.tot = P.total_units;
     constexpr bool TMEM = tmem_columns<U, RHS, G>(G) > 0;
@@ -2505,8 +2696,9 @@ __global__ void __launch_bounds__(RHS == 3 || RHS == 4 || RHS == 7 || G > 1 ? 25
         S.sPAR = S.xch + SM::XCH_DOUBLES + SM::RED_DOUBLES;
         S.upsh = S.sPAR + NSPa + NSAa + NISAa;
     } else {
-        using SM = WarpSmem<U, G>;
+        using SM = WarpSmem<U, G, (RHS > 10 ? TEAM : 1)>;
         double* base = smem + (size_t)slot * SM::DOUBLES;
+        if constexpr (RHS > 10) S.xt = base - (size_t)S.tw * SM::DOUBLES + SM::DOUBLES - SM::XT_DOUBLES;
         S.W = base;
         S.vp = base + SM::W_DOUBLES + SM::WT_DOUBLES;
         S.vpt = S.vp + SM::NMAX;
@@ -2532,8 +2724,9 @@ __global__ void __launch_bounds__(RHS == 3 || RHS == 4 || RHS == 7 || G > 1 ? 25
     Lane<U> L;
     for (;;) {
         int k = 0;
-        if (lane == 0 && leader) k = atomicAdd(P.work_counter, 1);
+        if (lane == 0 && leader && S.lead) k = atomicAdd(P.work_counter, 1);
         k = __shfl_sync(FULL, k, 0);
+        if constexpr (RHS > 10) k = team_share(S, k);
         if constexpr (G > 1) {
             double kk[G];
             grp_share(S, (double)k, kk);
@@ -2560,7 +2753,7 @@ __global__ void __launch_bounds__(RHS == 3 || RHS == 4 || RHS == 7 || G > 1 ? 25
 #pragma unroll
                 for (int c = 0; c < NUP; c++) L.up[m][c] = v ? __ldg(P.upar + (int64_t)c * S.tot + g) : 0.0;
             }
-            if constexpr (RHS >= 3) {
+            if constexpr ((RHS >= 3 && RHS < 10) || RHS > 14) {
                 L.ra[m] = v ? (P.coupling_row_scale ? __ldg(P.coupling_row_scale + g) : 1.0) : 0.0;
                 L.cb[m] = v ? (P.coupling_col_scale ? __ldg(P.coupling_col_scale + g) : 1.0) : 0.0;
             } else {
@@ -2585,6 +2778,14 @@ __global__ void __launch_bounds__(RHS == 3 || RHS == 4 || RHS == 7 || G > 1 ? 25
             for (int c = 0; c < NM; c++)
                 S.W[(r ^ quad_swizzle(c)) + c * NM] = (r < S.N && c < S.N) ? __ldg(S.C + r + (int64_t)c * S.N) : 0.0;
         }
+        if constexpr (RHS > 14) {
+            /* row `lane` of the shared symmetric matrix at the columns of this warp's two chains, zero-padded */
+#pragma unroll
+            for (int k = 0; k < 16; k++) {
+                const int j = 4 * (k >> 1) + 2 * (S.tw & 1) + (k & 1);
+                L.grow[k] = (lane < S.N && j < S.N) ? __ldg(S.C + lane + (int64_t)j * S.N) : 0.0;
+            }
+        }
         if constexpr (RHS == 5 || RHS == 6) {
             /* rows 2r, 2r + 1 of the shared symmetric matrix at the columns 4t + 2h + e of lane 2r + h, zero-padded */
 #pragma unroll
@@ -2604,7 +2805,7 @@ __global__ void __launch_bounds__(RHS == 3 || RHS == 4 || RHS == 7 || G > 1 ? 25
                 S.W[idx] = r < S.N ? __ldg(S.C + r + (int64_t)c * S.N) : 0.0;
             }
         }
-        if constexpr (RHS == 1 || RHS == 2) {
+        if constexpr (RHS == 1 || RHS == 2 || RHS == 11 || RHS == 12) {
             /* stage the system's coupling matrix, zero-padded to 32 x 33 */
             constexpr int LDC = WarpSmem<1>::LDW;
             for (int idx = lane; idx < 32 * LDC; idx += 32) {
@@ -2636,7 +2837,7 @@ __global__ void __launch_bounds__(RHS == 3 || RHS == 4 || RHS == 7 || G > 1 ? 25
 #pragma unroll
         for (int m = 0; m < U; m++) {
             const int i = S.unit(m);
-            if (i < S.N) {
+            if (i < S.N && S.lead) {
                 const int64_t g = S.off + i;
 #pragma unroll
                 for (int c = 0; c < UD; c++) P.state[(int64_t)c * S.tot + g] = L.X[m][c];
@@ -2645,7 +2846,7 @@ __global__ void __launch_bounds__(RHS == 3 || RHS == 4 || RHS == 7 || G > 1 ? 25
                 for (int c = 0; c < NIUA; c++) P.iuacc[(int64_t)c * S.tot + g] = L.iua[m][c];
             }
         }
-        if (leader) {
+        if (leader && S.lead) {
             for (int c = lane; c < NSA; c += 32) P.sacc[(int64_t)c * P.n_systems + sid] = S.sACC[c];
             for (int c = lane; c < NISA; c += 32) P.isacc[(int64_t)c * P.n_systems + sid] = S.isACC[c];
             if (lane == 0) {

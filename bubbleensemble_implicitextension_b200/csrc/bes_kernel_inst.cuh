@@ -46,6 +46,8 @@ inline size_t tmem_fit(size_t smem, int columns) {
 /* per-system shared memory (operator or staged matrix per system) */
 #define BES_SMEM_WARP(U_, G_) \
     tmem_fit((size_t)(warps / (G_)) * WarpSmem<U_, G_>::BYTES, tmem_columns<U_, ((U_) == 1 && (G_) > 1 ? 0 : 1), G_>(warps))
+/* a team's warps, each with its own region */
+#define BES_SMEM_TEAM (size_t)warps * WarpSmem<1, 1, TEAM>::BYTES
 /* per-system band of the coupling matrix, sized by the run-time band width */
 #define BES_SMEM_BAND(G_) (size_t)(warps / (G_)) * (size_t)BandSmem<G_>::doubles(band) * 8
 /* one staged matrix per CTA plus per-system vectors */

@@ -15,27 +15,37 @@ struct Tag {
 
 template <int REC, class F>
 bool dispatch_rec(Variant v, F&& f) {
-    const int key = v.U * 100 + v.rhs * 10 + v.G;
+    const int key = v.U * 1000 + v.rhs * 10 + v.G;
     switch (key) {
-        case 111: f(Tag<1, 1, 1, REC>{}); return true;
-        case 121: f(Tag<1, 2, 1, REC>{}); return true;
-        case 151: f(Tag<1, 5, 1, REC>{}); return true;
-        case 161: f(Tag<1, 6, 1, REC>{}); return true;
-        case 201: f(Tag<2, 0, 1, REC>{}); return true;
-        case 231: f(Tag<2, 3, 1, REC>{}); return true;
-        case 401: f(Tag<4, 0, 1, REC>{}); return true;
-        case 431: f(Tag<4, 3, 1, REC>{}); return true;
-        case 241: f(Tag<2, 4, 1, REC>{}); return true;
-        case 441: f(Tag<4, 4, 1, REC>{}); return true;
-        case 142: f(Tag<1, 4, 2, REC>{}); return true;
-        case 144: f(Tag<1, 4, 4, REC>{}); return true;
-        case 102: f(Tag<1, 0, 2, REC>{}); return true;
-        case 132: f(Tag<1, 3, 2, REC>{}); return true;
-        case 104: f(Tag<1, 0, 4, REC>{}); return true;
-        case 134: f(Tag<1, 3, 4, REC>{}); return true;
-        case 171: f(Tag<1, 7, 1, REC>{}); return true;
-        case 172: f(Tag<1, 7, 2, REC>{}); return true;
-        case 174: f(Tag<1, 7, 4, REC>{}); return true;
+        case 1011: f(Tag<1, 1, 1, REC>{}); return true;
+        case 1021: f(Tag<1, 2, 1, REC>{}); return true;
+        case 1051: f(Tag<1, 5, 1, REC>{}); return true;
+        case 1061: f(Tag<1, 6, 1, REC>{}); return true;
+        case 2001: f(Tag<2, 0, 1, REC>{}); return true;
+        case 2031: f(Tag<2, 3, 1, REC>{}); return true;
+        case 4001: f(Tag<4, 0, 1, REC>{}); return true;
+        case 4031: f(Tag<4, 3, 1, REC>{}); return true;
+        case 2041: f(Tag<2, 4, 1, REC>{}); return true;
+        case 4041: f(Tag<4, 4, 1, REC>{}); return true;
+        case 1042: f(Tag<1, 4, 2, REC>{}); return true;
+        case 1044: f(Tag<1, 4, 4, REC>{}); return true;
+        case 1002: f(Tag<1, 0, 2, REC>{}); return true;
+        case 1032: f(Tag<1, 3, 2, REC>{}); return true;
+        case 1004: f(Tag<1, 0, 4, REC>{}); return true;
+        case 1034: f(Tag<1, 3, 4, REC>{}); return true;
+        case 1071: f(Tag<1, 7, 1, REC>{}); return true;
+        case 1072: f(Tag<1, 7, 2, REC>{}); return true;
+        case 1074: f(Tag<1, 7, 4, REC>{}); return true;
+        /* teams: four warps a system */
+        case 1114: f(Tag<1, 11, 1, REC>{}); return true;
+        case 1124: f(Tag<1, 12, 1, REC>{}); return true;
+        case 1154: f(Tag<1, 15, 1, REC>{}); return true;
+        case 1164: f(Tag<1, 16, 1, REC>{}); return true;
+        /* sixteen warps an SM */
+        case 1242: f(Tag<1, 24, 2, REC>{}); return true;
+        case 1244: f(Tag<1, 24, 4, REC>{}); return true;
+        case 1272: f(Tag<1, 27, 2, REC>{}); return true;
+        case 1274: f(Tag<1, 27, 4, REC>{}); return true;
         default: return false;
     }
 }
@@ -62,7 +72,7 @@ size_t cta_smem_bytes(Variant v, int warps) {
 
 int max_warps_per_block(Variant v) {
     /* the kernels' launch bounds: 256 threads with RHS 3 or G > 1, else 128 */
-    const int cap = (v.rhs == 3 || v.rhs == 4 || v.rhs == 7 || v.G > 1) ? 8 : 4;
+    const int cap = v.rhs > 20 ? 16 : (v.rhs == 3 || v.rhs == 4 || v.rhs == 7 || v.G > 1) ? 8 : 4;
     int w = 0;
     while (w + v.G <= cap && cta_smem_bytes(v, w + v.G) <= 227 * 1024) w += v.G;
     return w;
@@ -84,22 +94,41 @@ cudaError_t launch(Variant v, const DeviceProblem& P, int grid, int warps, cudaS
  * (rhs 2: every system has exactly 32 units); larger N runs one unit per lane
  * on 2 or 4 warps (or 2 or 4 units per lane on one warp) with W in shared
  * memory, or one staged copy of a matrix shared by the whole class when the
- * caller asked for shared coupling matrices (SharedCouplingMatrices).  With
+ * caller asked for shared coupling matrices (SharedCouplingMatrices); team asks
+ * for four warps a system of up to 32 units where the model's callbacks can run
+ * on each of them (no global parameters they could write).  With
  * banded coupling storage (band > 0) every class whose matrix is not staged
  * as a shared symmetric (N <= 32) or shared (N > 32) matrix runs the banded
  * operator, one unit per lane on 1, 2 or 4 warps. */
-Variant class_variant(int cls, bool all32, bool shared, int warps_per_system, bool symmetric, int rec, int band) {
+Variant class_variant(int cls, bool all32, bool shared, int warps_per_system, bool symmetric, int rec, int band,
+                      bool team, bool dense) {
     if (cls == 0) {
-        if (shared && symmetric) return Variant{1, all32 ? 6 : 5, 1, rec};   /* row of G in registers */
-        if (band > 0) return Variant{1, 7, 1, rec, band};
-        return Variant{1, all32 ? 2 : 1, 1, rec};
+        const bool sym = shared && symmetric;   /* a share of G in registers */
+        if (!sym && band > 0) return Variant{1, 7, 1, rec, band};
+        const int rhs = sym ? (all32 ? 6 : 5) : (all32 ? 2 : 1);
+        if (team && warps_per_system != 1 && BES_MODEL_NGP == 0 && BES_MODEL_NIGP == 0)
+            return Variant{1, rhs + 10, TEAM, rec};
+        return Variant{1, rhs, 1, rec};
     }
     const int width = cls == 1 ? 2 : 4;
-    if (!shared && band > 0) return Variant{1, 7, width, rec, band};   /* banded storage: one unit per lane */
+    if (!shared && band > 0) return Variant{1, dense ? 27 : 7, width, rec, band};   /* banded storage: one unit per lane */
     const int rhs = shared ? (symmetric ? 4 : 3) : 0;
     if (warps_per_system == 1) return Variant{width, rhs, 1, rec};
-    return Variant{1, rhs, width, rec};
+    return Variant{1, rhs == 4 && dense ? 24 : rhs, width, rec};
 }
+
+/* Does a launch of `total` systems run those of up to 32 units on teams of four warps?  Eight warps of
+ * 255 registers are what an SM holds, and a team's warps repeat everything but the products, so a
+ * system to an SM always gains (8 bubbles alone 33.0 -> 31.6 ms, 64 x 16 bubbles with RK4 17.4 -> 16.2),
+ * two only with the shared symmetric matrix (256 x 32: 331 -> 324 and 325 -> 289 ms of two draws; own
+ * matrix 322 -> 326), and beside multi-warp systems none (384 uneven clouds: 92 -> 112 ms). */
+bool team_pays(int total, bool symmetric, int sm_count) { return total <= (symmetric ? 2 : 1) * sm_count; }
+
+/* Do `count` systems of class cls (1: two warps each, 2: four) run the kernels compiled for sixteen
+ * warps an SM?  As soon as there are more than the eight warps of 255 registers hold at once: the
+ * 128-register kernels spill a little, but run twice the systems side by side (512 shared-geometry
+ * systems of 128 bubbles 331 -> 291 ms, 512 rings of 128 307 -> 252 ms per pass). */
+bool dense_pays(int cls, int count, int sm_count) { return count > (cls == 1 ? 4 : 2) * sm_count; }
 
 /* CTA shape of a launch of `count` systems: spread small ensembles over every
  * SM, fill SMs otherwise; `requested` > 0 asks for that many warps per CTA */

@@ -10,7 +10,9 @@
  * (both BiCG products as row sums from one shared-memory read); RHS 5 / 6
  * (U = G = 1, N <= 32) keep a row of a shared symmetric matrix in registers
  * (6: every system has 32 units); RHS 7 (U = 1) keeps only the wrapping
- * band of banded coupling storage (CBW > 0).  Every variant exists with both BiCG
+ * band of banded coupling storage (CBW > 0); RHS 11, 12, 15, 16 with G = 4 are
+ * RHS 1, 2, 5, 6 on a team of four warps a system; RHS 24 and 27 are RHS 4 and 7
+ * compiled for sixteen warps an SM.  Every variant exists with both BiCG
  * recurrences (REC 0: the reference's; 1: the single-reduction form). */
 #ifndef BES_LAUNCH_H
 #define BES_LAUNCH_H
@@ -46,7 +48,12 @@ cudaError_t launch(Variant v, const DeviceProblem& P, int grid, int warps, cudaS
  * coupling matrix; warps_per_system 1 keeps every system on one warp; rec:
  * the BiCG recurrence */
 Variant class_variant(int cls, bool all32, bool shared, int warps_per_system, bool symmetric = false, int rec = 0,
-                      int band = 0);
+                      int band = 0, bool team = false, bool dense = false);
+/* whether `count` systems of class cls > 0 run at sixteen warps an SM */
+bool dense_pays(int cls, int count, int sm_count);
+/* whether a launch of `total` systems runs those of up to 32 units on teams of four warps
+ * (symmetric: they share one symmetric matrix) */
+bool team_pays(int total, bool symmetric, int sm_count);
 /* warps per CTA for `count` systems of variant v (requested > 0: that many,
  * clamped to what the variant allows and rounded down to a multiple of G) */
 int class_warps_per_block(Variant v, int count, int sm_count, int requested);

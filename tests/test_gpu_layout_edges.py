@@ -55,3 +55,31 @@ def test_step_budget_inside_an_event_and_two_frequencies(rec, gpu, oracle_lib):
     got = run_gpu(ens, bicg_recurrence=rec)
     want = oracle_lib.run(ens, n_periods=2, reset_at=1, bicg_variant=rec)
     assert_bitwise(got, want, KEYS)
+
+
+@pytest.mark.parametrize("rec", [0, 1])
+def test_one_warp_systems(rec, gpu, oracle_lib):
+    """Systems of up to 32 units on one warp each (few systems run on teams of four by default), own matrices and
+    one shared symmetric matrix."""
+    ens = _bounded(ragged_ensemble([1, 2, 7, 8, 9, 15, 16, 17, 24, 31, 32], seed=6))
+    got = run_gpu(ens, n_periods=1, reset_at=-1, bicg_recurrence=rec, warps_per_system=1)
+    want = oracle_lib.run(ens, n_periods=1, reset_at=-1, bicg_variant=rec)
+    assert_bitwise(got, want, KEYS)
+    for n in (9, 32):
+        ens = _bounded(W.c1_ensemble(n_pa=2, n_f=2, n_units=n, factored=True))
+        got = run_gpu(ens, n_periods=1, reset_at=-1, bicg_recurrence=rec, warps_per_system=1)
+        want = oracle_lib.run(ens, n_periods=1, reset_at=-1, bicg_variant=rec, shared_assoc=True)
+        assert_bitwise(got, want, KEYS)
+
+
+@pytest.mark.parametrize("rec", [0, 1])
+@pytest.mark.parametrize("banded", [False, True])
+@pytest.mark.parametrize("n,systems", [(66, 301), (35, 597)])
+def test_more_systems_than_eight_warps_an_sm_hold(n, systems, banded, rec, gpu, oracle_lib):
+    """The kernels compiled for sixteen warps an SM: shared symmetric matrix and banded storage, two and four warps."""
+    ens = (W.ring_ensemble(n_systems=systems, n_units=n, band_width=2) if banded
+           else W.c3_ensemble(n_systems=systems, n_units=n, n_periods=1))
+    ens = _bounded(ens, 12)
+    got = run_gpu(ens, n_periods=1, reset_at=-1, bicg_recurrence=rec)
+    want = oracle_lib.run(ens, n_periods=1, reset_at=-1, bicg_variant=rec)
+    assert_bitwise(got, want, KEYS)
