@@ -387,12 +387,16 @@ bool team_pays(const bes_solver* h) {
                           h->shared_coupling && h->class_shared[0] && h->class_symmetric[0], h->sm_count);
 }
 
+bool sparse_pays(const bes_solver* h) {
+    return bes::sparse_pays(h->class_count[0], std::min(h->active, h->n_systems), h->sm_count);
+}
+
 /* launch shape of one class (no stream work: safe before a capture) */
 bes_status plan_shape(bes_solver* h, int cls, int warps_per_system, int requested_wpb, ClassLaunch* L) {
     const bes::Variant v = bes::class_variant(cls, h->class0_all32, h->shared_coupling && h->class_shared[cls],
                                          warps_per_system, h->class_symmetric[cls], h->bicg_recurrence, h->cbw,
                                          team_pays(h),
-                                         bes::dense_pays(cls, h->class_count[cls], h->sm_count));
+                                         bes::dense_pays(cls, h->class_count[cls], h->sm_count), sparse_pays(h));
     const int count = h->class_count[cls];
     if (bes::max_warps_per_block(v) < v.G)
         return fail(h, BES_ERR_CUDA, "solver kernel variant (U=%d, G=%d) does not fit in shared memory", v.U, v.G);
@@ -1103,7 +1107,7 @@ bes_status bes_solve_periods(bes_solver* h, int32_t n_periods, int32_t reset_at)
         if (h->class_count[cls] > 0 && (st = plan_class(h, cls, &L[cls]))) return st;
     if (h->scaled_coupling[0] || h->scaled_coupling[1])
         for (int cls = 0; cls < 3; cls++)
-            if (h->class_count[cls] > 0 && L[cls].v.rhs < 3)
+            if (h->class_count[cls] > 0 && bes::own_matrix(L[cls].v))
                 return fail(h, BES_ERR_ARGUMENT,
                             "bes_solve_periods: CouplingRowScale / CouplingColumnScale hold values other than 1, "
                             "which only the shared-matrix kernels apply: turn SharedCouplingMatrices on and give "
@@ -1436,7 +1440,8 @@ bes_status bes_autotune(bes_solver* h, int32_t n_periods, int64_t step_cap, bes_
             const bes::Variant v = bes::class_variant(cls, h->class0_all32,
                                                       h->shared_coupling && h->class_shared[cls], wps,
                                                       h->class_symmetric[cls], h->bicg_recurrence, h->cbw, team,
-                                                      bes::dense_pays(cls, h->class_count[cls], h->sm_count));
+                                                      bes::dense_pays(cls, h->class_count[cls], h->sm_count),
+                                                      sparse_pays(h));
             const int cap = bes::max_warps_per_block(v);
             for (int wpb = v.G; wpb <= cap && !st; wpb *= 2) {
                 ClassLaunch L;

@@ -86,7 +86,8 @@ constexpr int TEAM = 4;
  * part of W that A^T v reads), six broadcast vectors, the group's exchange buffers
  * (G > 1) or the warp's reduction buffers, the system-scope arrays, and the unit
  * parameters when each lane owns one unit (U = 1: in registers they crowd out
- * the BiCG state).  T: the warps of a team, each with such a region. */
+ * the BiCG state).  T: the warps of a team, each with such a region; 0: one warp,
+ * its part of W in tensor memory. */
 template <int U, int G = 1, int T = 1>
 struct WarpSmem {
     static constexpr int NMAX = 32 * U * G;
@@ -138,10 +139,11 @@ struct SharedCSmem {
 /* TMEM columns of a CTA of `warps` warps: RHS 4 keeps each lane's share of the
  * shared matrix once for all systems of the CTA (NMAX doubles a lane); RHS 0
  * keeps each system's row and column shares of W (2 NMAX doubles a lane), four
- * warps side by side in the four quarters.  0: the variant uses none. */
+ * warps side by side in the four quarters; RHS 8 and 9 (at most four warps) each
+ * warp's column share (32 doubles a lane).  0: the variant uses none. */
 template <int U, int RHS, int G>
 __host__ __device__ constexpr int tmem_columns(int warps) {
-    return U != 1 || G == 1 ? 0 : RHS == 4 ? 2 * 32 * G : RHS == 0 ? 4 * 32 * G * ((warps + 3) / 4) : 0;
+    return U == 1 && G == 1 && (RHS == 8 || RHS == 9) ? 64 : U != 1 || G == 1 ? 0 : RHS == 4 ? 2 * 32 * G : RHS == 0 ? 4 * 32 * G * ((warps + 3) / 4) : 0;
 }
 
 /* Shared-memory layout of the banded variant (RHS = 7, one unit per lane, G
@@ -1255,13 +1257,15 @@ __device__ __forceinline__ void column_groups(int N, Fn&& f) {
  * rows, two chains: 32 doubles in registers) and those its share of A^T vt
  * reads: for the two columns 2r and 2r + 1 the rows of parity h, because the
  * halving tree over the rows splits into its even and its odd subtree until its
- * last addition (32 doubles of its own in shared memory, lane-consecutive
- * double2; in registers as well they spill).  The system's coupling matrix is
+ * last addition: 32 doubles of its own, in shared memory (lane-consecutive
+ * double2) or with TMEM in tensor memory; in registers as well they spill.  With
+ * a warp to itself on each sub-partition tensor memory is the faster place (256
+ * systems of 32: 322 -> 292 ms), with two the slower (1024: 287 -> 331 ms).  The system's coupling matrix is
  * staged once per system, zero-padded (leading dimension 33); the vector of the
  * transposed product is posted split by parity.
  * NFIX = 32 drops the N guards for full warps.  Same arithmetic, in the same
  * order, as the shared-memory variant. */
-template <int NFIX, int REC>
+template <int NFIX, int REC, bool TMEM>
 __device__ __forceinline__ int coupled_rhs_regw(const Sys<1>& S, const DeviceProblem& P, double T,
                                                 double (&Xs)[1][UD], double (&F)[1][UD],
                                                 double (&up)[1][NUPa], double (&ua)[1][NUAa],
@@ -1294,7 +1298,9 @@ __device__ __forceinline__ int coupled_rhs_regw(const Sys<1>& S, const DevicePro
     S.rdpar[par_slot(i)] = rd;
     __syncwarp();
     double wr[2][16];
-    double2* wc = reinterpret_cast<double2*>(S.W + 32 * LDC) + i;   /* entry k of columns r0, r0 + 1 at wc[32 k] */
+    /* the column share, entry k of columns r0, r0 + 1: at wc[32 k], or 2k and 2k + 1 of the chunks */
+    double2* wc = reinterpret_cast<double2*>(S.W + 32 * LDC) + i;
+    tmem::Chunk tc[2];
     double bs[2][2] = {{0.0, 0.0}, {0.0, 0.0}}, as[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
     const double* C = S.W;   /* C[i][j] at i + j * LDC */
     const double2* vx1_2 = reinterpret_cast<const double2*>(S.vx1);
@@ -1303,7 +1309,11 @@ __device__ __forceinline__ int coupled_rhs_regw(const Sys<1>& S, const DevicePro
     const double2* rdp2 = reinterpret_cast<const double2*>(S.rdpar + h * RED_RUN);
     const double2 rd2 = reinterpret_cast<const double2*>(S.vrd)[i >> 1], x12 = vx1_2[i >> 1];
 #pragma unroll
-    for (int t = 0; t < 16; t++) wr[0][t] = wr[1][t] = 0.0;
+    for (int t = 0; t < 16; t++) {
+        wr[0][t] = wr[1][t] = 0.0;
+        tc[t >> 3].set(2 * (t & 7), 0.0);
+        tc[t >> 3].set(2 * (t & 7) + 1, 0.0);
+    }
     column_groups<NFIX>(N, [&](int t) {
         const double2 x1p = vx1_2[2 * t + h], cpp = vcpt2[2 * t + h], xup = vxu2[2 * t + h];
         const double2 rdk = rdp2[t];   /* rows k = 4t + h and 4t + 2 + h */
@@ -1321,9 +1331,20 @@ __device__ __forceinline__ int coupled_rhs_regw(const Sys<1>& S, const DevicePro
             wr[1][2 * t + e] = (rd2.y * c1) * x1j;
             const int k = 4 * t + 2 * e + h;   /* the row with index 2t + e among those of parity h */
             const double rk = e ? rdk.y : rdk.x;
-            wc[32 * (2 * t + e)] = make_double2((rk * C[k + r0 * LDC]) * x12.x, (rk * C[k + (r0 + 1) * LDC]) * x12.y);
+            const double wk0 = (rk * C[k + r0 * LDC]) * x12.x, wk1 = (rk * C[k + (r0 + 1) * LDC]) * x12.y;
+            if constexpr (TMEM) {
+                tc[t >> 2].set(2 * (2 * (t & 3) + e), wk0);
+                tc[t >> 2].set(2 * (2 * (t & 3) + e) + 1, wk1);
+            } else {
+                wc[32 * (2 * t + e)] = make_double2(wk0, wk1);
+            }
         }
     });
+    if constexpr (TMEM) {
+        tc[0].store(S.tm);
+        tc[1].store(S.tm + 32);
+        tmem::wait_stores();
+    }
     double r = 0.0, bval = 0.0;
     {
         const double bsum = pair_exchange(h, bs[0][0] + bs[0][1], bs[1][0] + bs[1][1]);
@@ -1348,18 +1369,42 @@ __device__ __forceinline__ int coupled_rhs_regw(const Sys<1>& S, const DevicePro
         double u[2][16];
 #pragma unroll
         for (int k = 0; k < 16; k++) u[0][k] = u[1][k] = 0.0;
+        /* from tensor memory the column share arrives in two chunks, the first beside the row sums */
+        tmem::Chunk m;
+        if constexpr (TMEM) m.load(S.tm);
         column_groups<NFIX>(N, [&](int t) {
-            const double2 a = vp2[2 * t + h], c = tp2[t];
+            const double2 a = vp2[2 * t + h];
             qs[0][0] = fma(wr[0][2 * t], a.x, qs[0][0]);
             qs[1][0] = fma(wr[1][2 * t], a.x, qs[1][0]);
             qs[0][1] = fma(wr[0][2 * t + 1], a.y, qs[0][1]);
             qs[1][1] = fma(wr[1][2 * t + 1], a.y, qs[1][1]);
-            const double2 w0 = wc[32 * (2 * t)], w1 = wc[32 * (2 * t + 1)];
-            u[0][2 * t] = w0.x * c.x;
-            u[1][2 * t] = w0.y * c.x;
-            u[0][2 * t + 1] = w1.x * c.y;
-            u[1][2 * t + 1] = w1.y * c.y;
+            if constexpr (!TMEM) {
+                const double2 c = tp2[t], w0 = wc[32 * (2 * t)], w1 = wc[32 * (2 * t + 1)];
+                u[0][2 * t] = w0.x * c.x;
+                u[1][2 * t] = w0.y * c.x;
+                u[0][2 * t + 1] = w1.x * c.y;
+                u[1][2 * t + 1] = w1.y * c.y;
+            }
         });
+        if constexpr (TMEM) {
+            auto products = [&](int ch) {
+#pragma unroll
+                for (int t = 4 * ch; t < 4 * ch + 4; t++) {
+                    const double2 c = tp2[t];
+                    u[0][2 * t] = m.get(4 * (t & 3)) * c.x;
+                    u[1][2 * t] = m.get(4 * (t & 3) + 1) * c.x;
+                    u[0][2 * t + 1] = m.get(4 * (t & 3) + 2) * c.y;
+                    u[1][2 * t + 1] = m.get(4 * (t & 3) + 3) * c.y;
+                }
+            };
+            m.wait();
+            products(0);
+            if (NFIX != 0 || N > 16) {
+                m.load(S.tm + 32);
+                m.wait();
+                products(1);
+            }
+        }
         const double q = v[0] + pair_exchange(h, qs[0][0] + qs[0][1], qs[1][0] + qs[1][1]);
         auto leaf0 = [&](int k) -> double { return u[0][k]; };
         auto leaf1 = [&](int k) -> double { return u[1][k]; };
@@ -2042,7 +2087,7 @@ __device__ __forceinline__ int rhs_eval(const Sys<U, G>& S, const DeviceProblem&
         return coupled_rhs_band<G, REC>(S, P, T, Xs, F, ua, iua, capped);
     } else {
         static_assert(U == 1, "the register-resident operator needs one unit per lane");
-        return coupled_rhs_regw<RHS == 2 ? 32 : 0, REC>(S, P, T, Xs, F, up, ua, iua, capped);
+        return coupled_rhs_regw<RHS == 2 || RHS == 9 ? 32 : 0, REC, (RHS > 7)>(S, P, T, Xs, F, up, ua, iua, capped);
     }
 }
 
@@ -2593,7 +2638,8 @@ __device__ __forceinline__ void analysis_period_end(const Sys<U, G>& S, const De
  * (both BiCG products as row sums from one read of each entry).  G > 1 runs
  * one unit per lane (U = 1) and
  * exchanges the group's values through shared memory and a named barrier per
- * system slot (barrier 0 is left to __syncthreads).  V > 20 is RHS V - 20 compiled
+ * system slot (barrier 0 is left to __syncthreads).  RHS 8 and 9 are RHS 1 and 2
+ * with the column share of W in tensor memory.  V > 20 is RHS V - 20 compiled
  * for sixteen warps an SM (128 registers a thread), V = RHS otherwise.  RHS > 10 runs the variant
  * RHS - 10 of a system of up to 32 units on a team of warps (coupled_rhs_team). */
 template <int U, int V, int G, int REC>
@@ -2696,7 +2742,7 @@ __global__ void __launch_bounds__(V > 20 ? 512 : V == 3 || V == 4 || V == 7 || V
         S.sPAR = S.xch + SM::XCH_DOUBLES + SM::RED_DOUBLES;
         S.upsh = S.sPAR + NSPa + NSAa + NISAa;
     } else {
-        using SM = WarpSmem<U, G, (RHS > 10 ? TEAM : 1)>;
+        using SM = WarpSmem<U, G, (RHS > 10 ? TEAM : RHS > 7 ? 0 : 1)>;
         double* base = smem + (size_t)slot * SM::DOUBLES;
         if constexpr (RHS > 10) S.xt = base - (size_t)S.tw * SM::DOUBLES + SM::DOUBLES - SM::XT_DOUBLES;
         S.W = base;
@@ -2753,7 +2799,7 @@ __global__ void __launch_bounds__(V > 20 ? 512 : V == 3 || V == 4 || V == 7 || V
 #pragma unroll
                 for (int c = 0; c < NUP; c++) L.up[m][c] = v ? __ldg(P.upar + (int64_t)c * S.tot + g) : 0.0;
             }
-            if constexpr ((RHS >= 3 && RHS < 10) || RHS > 14) {
+            if constexpr ((RHS >= 3 && RHS <= 7) || RHS > 14) {
                 L.ra[m] = v ? (P.coupling_row_scale ? __ldg(P.coupling_row_scale + g) : 1.0) : 0.0;
                 L.cb[m] = v ? (P.coupling_col_scale ? __ldg(P.coupling_col_scale + g) : 1.0) : 0.0;
             } else {
@@ -2805,7 +2851,7 @@ __global__ void __launch_bounds__(V > 20 ? 512 : V == 3 || V == 4 || V == 7 || V
                 S.W[idx] = r < S.N ? __ldg(S.C + r + (int64_t)c * S.N) : 0.0;
             }
         }
-        if constexpr (RHS == 1 || RHS == 2 || RHS == 11 || RHS == 12) {
+        if constexpr (RHS == 1 || RHS == 2 || RHS == 8 || RHS == 9 || RHS == 11 || RHS == 12) {
             /* stage the system's coupling matrix, zero-padded to 32 x 33 */
             constexpr int LDC = WarpSmem<1>::LDW;
             for (int idx = lane; idx < 32 * LDC; idx += 32) {

@@ -46,6 +46,9 @@ inline size_t tmem_fit(size_t smem, int columns) {
 /* per-system shared memory (operator or staged matrix per system) */
 #define BES_SMEM_WARP(U_, G_) \
     tmem_fit((size_t)(warps / (G_)) * WarpSmem<U_, G_>::BYTES, tmem_columns<U_, ((U_) == 1 && (G_) > 1 ? 0 : 1), G_>(warps))
+/* one warp a system, its column share of W in tensor memory */
+#define BES_SMEM_WARP_TMEM(RHS_) \
+    tmem_fit((size_t)warps * WarpSmem<1, 1, 0>::BYTES, tmem_columns<1, RHS_, 1>(warps))
 /* a team's warps, each with its own region */
 #define BES_SMEM_TEAM (size_t)warps * WarpSmem<1, 1, TEAM>::BYTES
 /* per-system band of the coupling matrix, sized by the run-time band width */

@@ -19,6 +19,8 @@ bool dispatch_rec(Variant v, F&& f) {
     switch (key) {
         case 1011: f(Tag<1, 1, 1, REC>{}); return true;
         case 1021: f(Tag<1, 2, 1, REC>{}); return true;
+        case 1081: f(Tag<1, 8, 1, REC>{}); return true;
+        case 1091: f(Tag<1, 9, 1, REC>{}); return true;
         case 1051: f(Tag<1, 5, 1, REC>{}); return true;
         case 1061: f(Tag<1, 6, 1, REC>{}); return true;
         case 2001: f(Tag<2, 0, 1, REC>{}); return true;
@@ -101,14 +103,14 @@ cudaError_t launch(Variant v, const DeviceProblem& P, int grid, int warps, cudaS
  * as a shared symmetric (N <= 32) or shared (N > 32) matrix runs the banded
  * operator, one unit per lane on 1, 2 or 4 warps. */
 Variant class_variant(int cls, bool all32, bool shared, int warps_per_system, bool symmetric, int rec, int band,
-                      bool team, bool dense) {
+                      bool team, bool dense, bool sparse) {
     if (cls == 0) {
         const bool sym = shared && symmetric;   /* a share of G in registers */
         if (!sym && band > 0) return Variant{1, 7, 1, rec, band};
         const int rhs = sym ? (all32 ? 6 : 5) : (all32 ? 2 : 1);
         if (team && warps_per_system != 1 && BES_MODEL_NGP == 0 && BES_MODEL_NIGP == 0)
             return Variant{1, rhs + 10, TEAM, rec};
-        return Variant{1, rhs, 1, rec};
+        return Variant{1, !sym && sparse ? rhs + 7 : rhs, 1, rec};
     }
     const int width = cls == 1 ? 2 : 4;
     if (!shared && band > 0) return Variant{1, dense ? 27 : 7, width, rec, band};   /* banded storage: one unit per lane */
@@ -123,6 +125,12 @@ Variant class_variant(int cls, bool all32, bool shared, int warps_per_system, bo
  * two only with the shared symmetric matrix (256 x 32: 331 -> 324 and 325 -> 289 ms of two draws; own
  * matrix 322 -> 326), and beside multi-warp systems none (384 uneven clouds: 92 -> 112 ms). */
 bool team_pays(int total, bool symmetric, int sm_count) { return total <= (symmetric ? 2 : 1) * sm_count; }
+
+/* Does a launch of `total` systems, all of up to 32 units, keep the column share of W in tensor
+ * memory?  While no sub-partition holds two of its warps (see coupled_rhs_regw for both sides);
+ * beside multi-warp systems, whose matrices stream from there, it slowed both (384 uneven clouds
+ * 92 -> 110 ms). */
+bool sparse_pays(int count, int total, int sm_count) { return count == total && total <= 4 * sm_count; }
 
 /* Do `count` systems of class cls (1: two warps each, 2: four) run the kernels compiled for sixteen
  * warps an SM?  As soon as there are more than the eight warps of 255 registers hold at once: the

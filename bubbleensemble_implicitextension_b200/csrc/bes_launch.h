@@ -12,7 +12,8 @@
  * (6: every system has 32 units); RHS 7 (U = 1) keeps only the wrapping
  * band of banded coupling storage (CBW > 0); RHS 11, 12, 15, 16 with G = 4 are
  * RHS 1, 2, 5, 6 on a team of four warps a system; RHS 24 and 27 are RHS 4 and 7
- * compiled for sixteen warps an SM.  Every variant exists with both BiCG
+ * compiled for sixteen warps an SM; RHS 8 and 9 are RHS 1 and 2 with a share of
+ * the operator in tensor memory.  Every variant exists with both BiCG
  * recurrences (REC 0: the reference's; 1: the single-reduction form). */
 #ifndef BES_LAUNCH_H
 #define BES_LAUNCH_H
@@ -32,6 +33,10 @@ struct Variant {
     int band = 0;   /* band width of the banded variant (RHS 7) */
 };
 
+/* does the variant read each system's own full matrix (no unit coupling factors applied) */
+inline bool own_matrix(const Variant& v) {
+    return v.rhs < 3 || v.rhs == 8 || v.rhs == 9 || v.rhs == 11 || v.rhs == 12;
+}
 /* is (U, RHS, G) one of the built variants */
 bool variant_exists(Variant v);
 /* dynamic shared memory of a CTA of `warps` warps (a multiple of G) */
@@ -48,7 +53,9 @@ cudaError_t launch(Variant v, const DeviceProblem& P, int grid, int warps, cudaS
  * coupling matrix; warps_per_system 1 keeps every system on one warp; rec:
  * the BiCG recurrence */
 Variant class_variant(int cls, bool all32, bool shared, int warps_per_system, bool symmetric = false, int rec = 0,
-                      int band = 0, bool team = false, bool dense = false);
+                      int band = 0, bool team = false, bool dense = false, bool sparse = false);
+/* whether `count` systems of up to 32 units among `total` keep a share of W in tensor memory (own matrices, one warp) */
+bool sparse_pays(int count, int total, int sm_count);
 /* whether `count` systems of class cls > 0 run at sixteen warps an SM */
 bool dense_pays(int cls, int count, int sm_count);
 /* whether a launch of `total` systems runs those of up to 32 units on teams of four warps

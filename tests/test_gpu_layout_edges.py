@@ -83,3 +83,19 @@ def test_more_systems_than_eight_warps_an_sm_hold(n, systems, banded, rec, gpu, 
     got = run_gpu(ens, n_periods=1, reset_at=-1, bicg_recurrence=rec)
     want = oracle_lib.run(ens, n_periods=1, reset_at=-1, bicg_variant=rec)
     assert_bitwise(got, want, KEYS)
+
+
+@pytest.mark.parametrize("systems", [4, 200, 700])
+def test_unit_factors_need_a_shared_matrix(systems, gpu):
+    """Coupling factors other than 1 with a matrix per system are refused whichever one-warp kernel or team the
+    number of systems selects."""
+    from bubbleensemble_implicitextension_b200 import solver as S
+    ens = W.c1_ensemble(n_pa=systems, n_f=1, n_units=8)
+    ps = ens.make_solver()
+    try:
+        ps.set_array(S.ListOfVariables.CouplingRowScale, np.full(ens.total_units, 2.0))
+        ps.SynchroniseFromHostToDevice(S.ListOfVariables.All)
+        with pytest.raises(S.BesError, match="CouplingRowScale"):
+            ps.solve_periods(1, -1)
+    finally:
+        ps.close()
