@@ -97,8 +97,7 @@ cudaError_t launch(Variant v, const DeviceProblem& P, int grid, int warps, cudaS
  * on 2 or 4 warps (or 2 or 4 units per lane on one warp) with W in shared
  * memory, or one staged copy of a matrix shared by the whole class when the
  * caller asked for shared coupling matrices (SharedCouplingMatrices); team asks
- * for four warps a system of up to 32 units where the model's callbacks can run
- * on each of them (no global parameters they could write).  With
+ * for four warps a system of up to 32 units (see team_pays).  With
  * banded coupling storage (band > 0) every class whose matrix is not staged
  * as a shared symmetric (N <= 32) or shared (N > 32) matrix runs the banded
  * operator, one unit per lane on 1, 2 or 4 warps. */
@@ -108,8 +107,7 @@ Variant class_variant(int cls, bool all32, bool shared, int warps_per_system, bo
         const bool sym = shared && symmetric;   /* a share of G in registers */
         if (!sym && band > 0) return Variant{1, 7, 1, rec, band};
         const int rhs = sym ? (all32 ? 6 : 5) : (all32 ? 2 : 1);
-        if (team && warps_per_system != 1 && BES_MODEL_NGP == 0 && BES_MODEL_NIGP == 0)
-            return Variant{1, rhs + 10, TEAM, rec};
+        if (team && warps_per_system != 1) return Variant{1, rhs + 10, TEAM, rec};
         return Variant{1, !sym && sparse ? rhs + 7 : rhs, 1, rec};
     }
     const int width = cls == 1 ? 2 : 4;
@@ -119,12 +117,23 @@ Variant class_variant(int cls, bool all32, bool shared, int warps_per_system, bo
     return Variant{1, rhs == 4 && dense ? 24 : rhs, width, rec};
 }
 
-/* Does a launch of `total` systems run those of up to 32 units on teams of four warps?  Eight warps of
+/* Can every warp of a team run the model's callbacks and come to the same bits?  Only while the callbacks
+ * write nothing but their own unit's values: a global parameter would be written four times, and each warp
+ * has its own copy of the system-scope values, on which the units of a system may race (plain stores, atomic
+ * sums).  Nothing orders those alike in two warps, so the copies could differ, the warps decide differently,
+ * and one wait at a team barrier for an exchange that the others never make. */
+constexpr bool TEAM_MODEL = BES_MODEL_NGP == 0 && BES_MODEL_NIGP == 0 && BES_MODEL_NSP == 0 && BES_MODEL_NSA == 0 &&
+                            BES_MODEL_NISA == 0;
+
+/* Does a launch of `total` systems run those of up to 32 units on teams of four warps (where TEAM_MODEL
+ * allows them)?  Eight warps of
  * 255 registers are what an SM holds, and a team's warps repeat everything but the products, so a
  * system to an SM always gains (8 bubbles alone 33.0 -> 31.6 ms, 64 x 16 bubbles with RK4 17.4 -> 16.2),
  * two only with the shared symmetric matrix (256 x 32: 331 -> 324 and 325 -> 289 ms of two draws; own
  * matrix 322 -> 326), and beside multi-warp systems none (384 uneven clouds: 92 -> 112 ms). */
-bool team_pays(int total, bool symmetric, int sm_count) { return total <= (symmetric ? 2 : 1) * sm_count; }
+bool team_pays(int total, bool symmetric, int sm_count) {
+    return TEAM_MODEL && total <= (symmetric ? 2 : 1) * sm_count;
+}
 
 /* Does a launch of `total` systems, all of up to 32 units, keep the column share of W in tensor
  * memory?  While no sub-partition holds two of its warps (see coupled_rhs_regw for both sides);
