@@ -146,7 +146,10 @@ __host__ __device__ constexpr int tmem_columns(int warps) {
     return U == 1 && G == 1 && (RHS == 8 || RHS == 9) ? 64 : U != 1 || G == 1 ? 0 : RHS == 4 ? 2 * 32 * G : RHS == 0 ? 4 * 32 * G * ((warps + 3) / 4) : 0;
 }
 
-/* Shared-memory layout of the banded variant (RHS = 7, one unit per lane, G
+/* diagonals of the banded operator in registers; RHS 7 has no others */
+constexpr int BAND_REGS = 8;
+
+/* Shared-memory layout of the banded variants (RHS = 7 and 10, one unit per lane, G
  * warps, NMAX = 32 G units): per system the staged band of its coupling
  * matrix Cb[d][i] = C[i][(i + d - bw) mod N] and the operator by diagonal
  * Wb[d][i], ND = min(2 bw + 1, NMAX) diagonals each, then the six broadcast
@@ -1958,10 +1961,14 @@ __device__ __forceinline__ int coupled_rhs_team(const Sys<1>& S, const DevicePro
  * operator's first BAND_REGS diagonals -- all of them up to bw = 3, the rings
  * and chains in use -- stay in registers for the whole right-hand side, in
  * both directions, so an iteration reads only the two vectors: 512 rings of
- * 128 bubbles with bw = 1, 4000 steps each, 445 -> 348 ms on a B200. */
-constexpr int BAND_REGS = 8;
+ * 128 bubbles with bw = 1, 4000 steps each, 445 -> 348 ms on a B200.
+ * WIDE (RHS 10): more diagonals than that.  The rest is read from shared memory,
+ * four diagonals a group without guards and two groups at once, so that sixteen
+ * entries are on their way together (a guard on each entry exposed every load's
+ * latency).  A kernel of its own: with the loop in the kernel of narrow bands,
+ * those lose 3 %. */
 
-template <int G, int REC>
+template <int G, bool WIDE, int REC>
 __device__ __forceinline__ int coupled_rhs_band(const Sys<1, G>& S, const DeviceProblem& P, double T,
                                                 double (&Xs)[1][UD], double (&F)[1][UD], double (&ua)[1][NUAa],
                                                 int (&iua)[1][NIUAa], bool& capped) {
@@ -2014,9 +2021,15 @@ __device__ __forceinline__ int coupled_rhs_band(const Sys<1, G>& S, const Device
         };
 #pragma unroll
         for (int d = 0; d < BAND_REGS; d++) wr[d] = d < nd ? form(d, bs[d & 3], as[d & 3]) : 0.0;
-        for (int d = BAND_REGS; d < nd; d += 4) {
+        if constexpr (WIDE) {
+            int d = BAND_REGS;
+#pragma unroll 2
+            for (; d + 3 < nd; d += 4) {
 #pragma unroll
-            for (int e = 0; e < 4; e++)
+                for (int e = 0; e < 4; e++) form(d + e, bs[e], as[e]);
+            }
+#pragma unroll
+            for (int e = 0; e < 3; e++)
                 if (d + e < nd) form(d + e, bs[e], as[e]);
         }
         const double b = fma(rd, (bs[0] + bs[1]) + (bs[2] + bs[3]), xu);
@@ -2041,14 +2054,21 @@ __device__ __forceinline__ int coupled_rhs_band(const Sys<1, G>& S, const Device
                     qs[d & 3] = fma(wr[d], S.vp[col(d)], qs[d & 3]);
                     ts[d & 3] = fma(wt[d], S.vpt[row(d)], ts[d & 3]);
                 }
-            for (int d = BAND_REGS; d < nd; d += 4) {
+            if constexpr (WIDE) {
+                auto entry = [&](int d, double& qk, double& tk) {
+                    const int kk = row(d);
+                    qk = fma(Wb[d * NMAX + i], S.vp[col(d)], qk);
+                    tk = fma(Wb[d * NMAX + kk], S.vpt[kk], tk);
+                };
+                int d = BAND_REGS;
+#pragma unroll 2
+                for (; d + 3 < nd; d += 4) {
 #pragma unroll
-                for (int e = 0; e < 4; e++)
-                    if (d + e < nd) {
-                        const int kk = row(d + e);
-                        qs[e] = fma(Wb[(d + e) * NMAX + i], S.vp[col(d + e)], qs[e]);
-                        ts[e] = fma(Wb[(d + e) * NMAX + kk], S.vpt[kk], ts[e]);
-                    }
+                    for (int e = 0; e < 4; e++) entry(d + e, qs[e], ts[e]);
+                }
+#pragma unroll
+                for (int e = 0; e < 3; e++)
+                    if (d + e < nd) entry(d + e, qs[e], ts[e]);
             }
             q = v[0] + ((qs[0] + qs[1]) + (qs[2] + qs[3]));
             qt = vt[0] + ((ts[0] + ts[1]) + (ts[2] + ts[3]));
@@ -2082,9 +2102,9 @@ __device__ __forceinline__ int rhs_eval(const Sys<U, G>& S, const DeviceProblem&
     } else if constexpr (RHS == 5 || RHS == 6) {
         static_assert(U == 1 && G == 1, "the register-resident operator needs one unit per lane");
         return coupled_rhs_regsym<RHS == 6 ? 32 : 0, REC>(S, P, T, Xs, F, ua, iua, ra, cb, grow, capped);
-    } else if constexpr (RHS == 7) {
+    } else if constexpr (RHS == 7 || RHS == 10) {
         static_assert(U == 1, "the banded operator runs one unit per lane");
-        return coupled_rhs_band<G, REC>(S, P, T, Xs, F, ua, iua, capped);
+        return coupled_rhs_band<G, RHS == 10, REC>(S, P, T, Xs, F, ua, iua, capped);
     } else {
         static_assert(U == 1, "the register-resident operator needs one unit per lane");
         return coupled_rhs_regw<RHS == 2 || RHS == 9 ? 32 : 0, REC, (RHS > 7)>(S, P, T, Xs, F, up, ua, iua, capped);
@@ -2638,14 +2658,16 @@ __device__ __forceinline__ void analysis_period_end(const Sys<U, G>& S, const De
  * (both BiCG products as row sums from one read of each entry).  G > 1 runs
  * one unit per lane (U = 1) and
  * exchanges the group's values through shared memory and a named barrier per
- * system slot (barrier 0 is left to __syncthreads).  RHS 8 and 9 are RHS 1 and 2
+ * system slot (barrier 0 is left to __syncthreads).  RHS 7 and 10 are the banded
+ * operator of narrow and of wide bands.  RHS 8 and 9 are RHS 1 and 2
  * with the column share of W in tensor memory.  V > 20 is RHS V - 20 compiled
  * for sixteen warps an SM (128 registers a thread), V = RHS otherwise.  RHS > 10 runs the variant
  * RHS - 10 of a system of up to 32 units on a team of warps (coupled_rhs_team). */
 template <int U, int V, int G, int REC>
-__global__ void __launch_bounds__(V > 20 ? 512 : V == 3 || V == 4 || V == 7 || V > 10 || G > 1 ? 256 : 128, 1)
+__global__ void __launch_bounds__(V > 20 ? 512 : V == 3 || V == 4 || V == 7 || V >= 10 || G > 1 ? 256 : 128, 1)
     bes_ensemble_kernel(DeviceProblem P) {
     constexpr int RHS = V > 20 ? V - 20 : V;
+    constexpr bool BAND = RHS == 7 || RHS == 10;
     static_assert(G == 1 || U == 1, "multi-warp systems run one unit per lane");
     static_assert(G == 1 || (RHS != 1 && RHS != 2 && RHS != 5 && RHS != 6),
                   "the register-resident operators are single-warp");
@@ -2725,7 +2747,7 @@ __global__ void __launch_bounds__(V > 20 ? 512 : V == 3 || V == 4 || V == 7 || V
         S.flag = S.xch + 2 * XCH_BUF;
         S.sPAR = S.xch + SM::XCH_DOUBLES;
         S.upsh = S.sPAR + NSPa + NSAa + NISAa;
-    } else if constexpr (RHS == 7) {
+    } else if constexpr (BAND) {
         using SM = BandSmem<G>;
         constexpr int NM = SM::NMAX;
         const int ND = SM::diagonals(P.band_width);
@@ -2840,7 +2862,7 @@ __global__ void __launch_bounds__(V > 20 ? 512 : V == 3 || V == 4 || V == 7 || V
                 L.grow[k] = (row < S.N && j < S.N) ? __ldg(S.C + row + (int64_t)j * S.N) : 0.0;
             }
         }
-        if constexpr (RHS == 7) {
+        if constexpr (BAND) {
             /* stage the system's band: Cb[d][i] = C[i][(i + d - bw) mod N] */
             constexpr int NM = BandSmem<G>::NMAX;
             const int ND = BandSmem<G>::diagonals(P.band_width);

@@ -38,6 +38,9 @@ bool dispatch_rec(Variant v, F&& f) {
         case 1071: f(Tag<1, 7, 1, REC>{}); return true;
         case 1072: f(Tag<1, 7, 2, REC>{}); return true;
         case 1074: f(Tag<1, 7, 4, REC>{}); return true;
+        case 1101: f(Tag<1, 10, 1, REC>{}); return true;
+        case 1102: f(Tag<1, 10, 2, REC>{}); return true;
+        case 1104: f(Tag<1, 10, 4, REC>{}); return true;
         /* teams: four warps a system */
         case 1114: f(Tag<1, 11, 1, REC>{}); return true;
         case 1124: f(Tag<1, 12, 1, REC>{}); return true;
@@ -74,7 +77,7 @@ size_t cta_smem_bytes(Variant v, int warps) {
 
 int max_warps_per_block(Variant v) {
     /* the kernels' launch bounds: 256 threads with RHS 3 or G > 1, else 128 */
-    const int cap = v.rhs > 20 ? 16 : (v.rhs == 3 || v.rhs == 4 || v.rhs == 7 || v.G > 1) ? 8 : 4;
+    const int cap = v.rhs > 20 ? 16 : (v.rhs == 3 || v.rhs == 4 || v.rhs == 7 || v.rhs == 10 || v.G > 1) ? 8 : 4;
     int w = 0;
     while (w + v.G <= cap && cta_smem_bytes(v, w + v.G) <= 227 * 1024) w += v.G;
     return w;
@@ -103,15 +106,16 @@ cudaError_t launch(Variant v, const DeviceProblem& P, int grid, int warps, cudaS
  * operator, one unit per lane on 1, 2 or 4 warps. */
 Variant class_variant(int cls, bool all32, bool shared, int warps_per_system, bool symmetric, int rec, int band,
                       bool team, bool dense, bool sparse) {
+    const bool wide = 2 * band + 1 > BAND_REGS;   /* more diagonals than the registers take */
     if (cls == 0) {
         const bool sym = shared && symmetric;   /* a share of G in registers */
-        if (!sym && band > 0) return Variant{1, 7, 1, rec, band};
+        if (!sym && band > 0) return Variant{1, wide ? 10 : 7, 1, rec, band};
         const int rhs = sym ? (all32 ? 6 : 5) : (all32 ? 2 : 1);
         if (team && warps_per_system != 1) return Variant{1, rhs + 10, TEAM, rec};
         return Variant{1, !sym && sparse ? rhs + 7 : rhs, 1, rec};
     }
     const int width = cls == 1 ? 2 : 4;
-    if (!shared && band > 0) return Variant{1, dense ? 27 : 7, width, rec, band};   /* banded storage: one unit per lane */
+    if (!shared && band > 0) return Variant{1, wide ? 10 : dense ? 27 : 7, width, rec, band};   /* banded storage: one unit per lane */
     const int rhs = shared ? (symmetric ? 4 : 3) : 0;
     if (warps_per_system == 1) return Variant{width, rhs, 1, rec};
     return Variant{1, rhs == 4 && dense ? 24 : rhs, width, rec};

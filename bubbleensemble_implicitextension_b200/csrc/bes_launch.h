@@ -10,7 +10,8 @@
  * (both BiCG products as row sums from one shared-memory read); RHS 5 / 6
  * (U = G = 1, N <= 32) keep a row of a shared symmetric matrix in registers
  * (6: every system has 32 units); RHS 7 (U = 1) keeps only the wrapping
- * band of banded coupling storage (CBW > 0); RHS 11, 12, 15, 16 with G = 4 are
+ * band of banded coupling storage (CBW > 0), RHS 10 one of more than eight
+ * diagonals; RHS 11, 12, 15, 16 with G = 4 are
  * RHS 1, 2, 5, 6 on a team of four warps a system; RHS 24 and 27 are RHS 4 and 7
  * compiled for sixteen warps an SM; RHS 8 and 9 are RHS 1 and 2 with a share of
  * the operator in tensor memory.  Every variant exists with both BiCG
@@ -30,7 +31,7 @@ namespace bes {
 struct Variant {
     int U, rhs, G;
     int rec = 0;
-    int band = 0;   /* band width of the banded variant (RHS 7) */
+    int band = 0;   /* band width of the banded variants (RHS 7, 10) */
 };
 
 /* does the variant read each system's own full matrix (no unit coupling factors applied) */

@@ -36,3 +36,16 @@ def test_banded_ragged_sizes_one_launch_per_class(gpu, oracle_lib):
     got = run_gpu(ens, n_periods=1, reset_at=-1)
     want = oracle_lib.run(ens, n_periods=1, reset_at=-1)
     assert_bitwise(got, want, KEYS)
+
+
+@pytest.mark.parametrize("rec", [0, 1])
+@pytest.mark.parametrize("n,bw", [(32, 12), (31, 15), (50, 9), (50, 30), (64, 20), (64, 40), (128, 4),
+                                  (128, 8), (101, 30), (128, 45)])
+def test_wide_bands_match_oracle(n, bw, rec, gpu, oracle_lib):
+    """More diagonals than the operator keeps in registers, every remainder of the rest mod 4 (2 bw + 1 or n of
+    them, eight in registers)."""
+    ens = W.ring_ensemble(n_systems=3, n_units=n, band_width=bw)
+    ens.max_steps_per_period = 200
+    got = run_gpu(ens, n_periods=1, reset_at=-1, bicg_recurrence=rec)
+    want = oracle_lib.run(ens, n_periods=1, reset_at=-1, bicg_variant=rec)
+    assert_bitwise(got, want, KEYS)
