@@ -154,16 +154,20 @@ constexpr int BAND_REGS = 8;
  * matrix Cb[d][i] = C[i][(i + d - bw) mod N] and the operator by diagonal
  * Wb[d][i], ND = min(2 bw + 1, NMAX) diagonals each, then the six broadcast
  * vectors, the group's exchange buffers, the system-scope arrays and the unit
- * parameters.  The band width is a run-time value, so is the layout. */
-template <int G>
+ * parameters.  The band width is a run-time value, so is the layout.  Narrow
+ * bands add the stage derivatives; wide ones (RHS = 10) need the room: with the
+ * derivatives' 12 KB a system of 128 units does not fit beyond bw = 45 (48
+ * without), and two share an SM up to bw = 17 (20 without). */
+template <int G, bool WIDE>
 struct BandSmem {
     static constexpr int NMAX = 32 * G;
     static constexpr int XCH_DOUBLES = G > 1 ? 2 * XCH_BUF + 8 : 0;
     static constexpr int RED_DOUBLES = G == 1 ? 2 * RED_BUF : 0;   /* warp_sum32's buffers */
+    static constexpr int K_DOUBLES = WIDE ? 0 : 6 * UD * NMAX;   /* stage derivatives */
     __host__ __device__ static constexpr int diagonals(int bw) { return 2 * bw + 1 < NMAX ? 2 * bw + 1 : NMAX; }
     __host__ __device__ static constexpr int doubles(int bw) {
-        return (2 * diagonals(bw) * NMAX + 6 * NMAX + XCH_DOUBLES + RED_DOUBLES + NSPa + NSAa + NISAa + NMAX * NUPa + 6 * UD * NMAX + 31) /
-               32 * 32;
+        return (2 * diagonals(bw) * NMAX + 6 * NMAX + XCH_DOUBLES + RED_DOUBLES + NSPa + NSAa + NISAa + NMAX * NUPa +
+                K_DOUBLES + 31) / 32 * 32;
     }
 };
 
@@ -1975,7 +1979,7 @@ __device__ __forceinline__ int coupled_rhs_band(const Sys<1, G>& S, const Device
     constexpr int NMAX = 32 * G;
     const int N = S.N;
     const int bw = P.band_width;
-    const int ND = BandSmem<G>::diagonals(bw);
+    const int ND = BandSmem<G, WIDE>::diagonals(bw);
     const int nd = ND < N ? ND : N;
     const int i = S.unit(0);
     const bool valid = i < N;
@@ -2138,14 +2142,18 @@ __device__ __forceinline__ double* upar_of(const Sys<U, G>& S, Lane<U>& L, int m
     else return L.up[m];
 }
 
-/* The stage derivatives K_j of this lane's units: with one unit per lane in
- * shared memory (each is written once and read a few times a step, while the
- * BiCG needs the registers), else in registers. */
-template <int U, int G, int J>
+/* are a variant's stage derivatives in shared memory */
+template <int U, int RHS>
+__device__ constexpr bool stages_shared() { return U == 1 && RHS != 10; }
+
+/* The stage derivatives K_j of this lane's units: SHARED in shared memory (each
+ * is written once and read a few times a step, while the BiCG needs the
+ * registers), else in registers. */
+template <int U, int G, int J, bool SHARED>
 struct Stages {
-    double k[U == 1 ? 1 : J][U][UD];
+    double k[SHARED ? 1 : J][U][UD];
     __device__ __forceinline__ void set(const Sys<U, G>& S, int st, const double (&F)[U][UD]) {
-        if constexpr (U == 1) {
+        if constexpr (SHARED) {
 #pragma unroll
             for (int c = 0; c < UD; c++) S.ks[(st * UD + c) * 32 * G + S.unit(0)] = F[0][c];
         } else {
@@ -2159,7 +2167,7 @@ struct Stages {
         }
     }
     __device__ __forceinline__ double get(const Sys<U, G>& S, int j, int m, int c) const {
-        if constexpr (U == 1) return S.ks[(j * UD + c) * 32 * G + S.unit(0)];
+        if constexpr (SHARED) return S.ks[(j * UD + c) * 32 * G + S.unit(0)];
         else return k[j][m][c];
     }
 };
@@ -2186,8 +2194,8 @@ template <int U, int RHS, int G, int REC>
 __device__ __forceinline__ bool step_rkck45(const Sys<U, G>& S, const DeviceProblem& P, Lane<U>& L,
                                             double T, double dt, double (&Yn)[U][UD], double (&E)[U][UD],
                                             Counters& cnt, bool& capped) {
-    Stages<U, G, 6> K;
-    if constexpr (U > 1) {
+    Stages<U, G, 6, stages_shared<U, RHS>()> K;
+    if constexpr (!stages_shared<U, RHS>()) {
 #pragma unroll
         for (int j = 0; j < 6; j++)
 #pragma unroll
@@ -2248,8 +2256,8 @@ __device__ __forceinline__ bool step_rkck45(const Sys<U, G>& S, const DeviceProb
 template <int U, int RHS, int G, int REC>
 __device__ __forceinline__ bool step_rk4(const Sys<U, G>& S, const DeviceProblem& P, Lane<U>& L,
                                          double T, double dt, double (&Yn)[U][UD], Counters& cnt, bool& capped) {
-    Stages<U, G, 4> K;
-    if constexpr (U > 1) {
+    Stages<U, G, 4, stages_shared<U, RHS>()> K;
+    if constexpr (!stages_shared<U, RHS>()) {
 #pragma unroll
         for (int j = 0; j < 4; j++)
 #pragma unroll
@@ -2748,7 +2756,7 @@ __global__ void __launch_bounds__(V > 20 ? 512 : V == 3 || V == 4 || V == 7 || V
         S.sPAR = S.xch + SM::XCH_DOUBLES;
         S.upsh = S.sPAR + NSPa + NSAa + NISAa;
     } else if constexpr (BAND) {
-        using SM = BandSmem<G>;
+        using SM = BandSmem<G, RHS == 10>;
         constexpr int NM = SM::NMAX;
         const int ND = SM::diagonals(P.band_width);
         double* base = smem + (size_t)slot * SM::doubles(P.band_width);
@@ -2864,8 +2872,9 @@ __global__ void __launch_bounds__(V > 20 ? 512 : V == 3 || V == 4 || V == 7 || V
         }
         if constexpr (BAND) {
             /* stage the system's band: Cb[d][i] = C[i][(i + d - bw) mod N] */
-            constexpr int NM = BandSmem<G>::NMAX;
-            const int ND = BandSmem<G>::diagonals(P.band_width);
+            using SM = BandSmem<G, RHS == 10>;
+            constexpr int NM = SM::NMAX;
+            const int ND = SM::diagonals(P.band_width);
             const int nd = ND < S.N ? ND : S.N;
             for (int idx = 32 * S.wis + lane; idx < nd * NM; idx += 32 * G) {
                 const int d = idx / NM, r = idx % NM;

@@ -4,5 +4,5 @@
 
 namespace bes {
 BES_KERNEL_VARIANT(1, 24, 2, 0, BES_SMEM_SHARED(1, 2, true))
-BES_KERNEL_VARIANT(1, 27, 2, 0, BES_SMEM_BAND(2))
+BES_KERNEL_VARIANT(1, 27, 2, 0, BES_SMEM_BAND(2, false))
 }  // namespace bes

@@ -4,5 +4,5 @@
 
 namespace bes {
 BES_KERNEL_VARIANT(1, 24, 4, 1, BES_SMEM_SHARED(1, 4, true))
-BES_KERNEL_VARIANT(1, 27, 4, 1, BES_SMEM_BAND(4))
+BES_KERNEL_VARIANT(1, 27, 4, 1, BES_SMEM_BAND(4, false))
 }  // namespace bes

@@ -6,6 +6,6 @@ namespace bes {
 BES_KERNEL_VARIANT(1, 0, 2, 0, BES_SMEM_WARP(1, 2))
 BES_KERNEL_VARIANT(1, 3, 2, 0, BES_SMEM_SHARED(1, 2, false))
 BES_KERNEL_VARIANT(1, 4, 2, 0, BES_SMEM_SHARED(1, 2, true))
-BES_KERNEL_VARIANT(1, 7, 2, 0, BES_SMEM_BAND(2))
-BES_KERNEL_VARIANT(1, 10, 2, 0, BES_SMEM_BAND(2))
+BES_KERNEL_VARIANT(1, 7, 2, 0, BES_SMEM_BAND(2, false))
+BES_KERNEL_VARIANT(1, 10, 2, 0, BES_SMEM_BAND(2, true))
 }  // namespace bes

@@ -52,7 +52,7 @@ inline size_t tmem_fit(size_t smem, int columns) {
 /* a team's warps, each with its own region */
 #define BES_SMEM_TEAM (size_t)warps * WarpSmem<1, 1, TEAM>::BYTES
 /* per-system band of the coupling matrix, sized by the run-time band width */
-#define BES_SMEM_BAND(G_) (size_t)(warps / (G_)) * (size_t)BandSmem<G_>::doubles(band) * 8
+#define BES_SMEM_BAND(G_, WIDE_) (size_t)(warps / (G_)) * (size_t)BandSmem<G_, WIDE_>::doubles(band) * 8
 /* one staged matrix per CTA plus per-system vectors */
 #define BES_SMEM_SHARED(U_, G_, SYM_)                                    \
     tmem_fit((size_t)SharedCSmem<U_, G_, SYM_>::C_BYTES +                \

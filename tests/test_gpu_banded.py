@@ -40,7 +40,7 @@ def test_banded_ragged_sizes_one_launch_per_class(gpu, oracle_lib):
 
 @pytest.mark.parametrize("rec", [0, 1])
 @pytest.mark.parametrize("n,bw", [(32, 12), (31, 15), (50, 9), (50, 30), (64, 20), (64, 40), (128, 4),
-                                  (128, 8), (101, 30), (128, 45)])
+                                  (128, 8), (101, 30), (128, 45), (128, 46), (127, 48)])
 def test_wide_bands_match_oracle(n, bw, rec, gpu, oracle_lib):
     """More diagonals than the operator keeps in registers, every remainder of the rest mod 4 (2 bw + 1 or n of
     them, eight in registers)."""

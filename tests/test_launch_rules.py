@@ -12,17 +12,21 @@ CSRC = ROOT / "bubbleensemble_implicitextension_b200" / "csrc"
 SMS = 148
 
 
-def run_rules(tmp_path, body, model=""):
-    """Output lines of `body`, C++ statements over namespace bes; `model`: lines that change the system definition.
-    The rules call no kernel, so the kernels' entry points stay unresolved."""
+def run_rules(tmp_path, body, model="", lib=None):
+    """Output of `body`, C++ statements over namespace bes; `model`: lines that change the system definition.
+    Linked with the library `lib` where the body asks what fits on an SM, else the kernels' entry points stay
+    unresolved: the rules alone call none."""
     (tmp_path / "model.cuh").write_text('#include "km_model.cuh"\n' + model)
     (tmp_path / "main.cu").write_text(
         '#include <cstdio>\n#include "bes_launch.h"\nint main() {\n    using namespace bes;\n' + body + "\n}\n")
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     exe = tmp_path / "rules"
+    link = ["-Xlinker", "--unresolved-symbols=ignore-all"]
+    if lib:
+        link = [str(lib), "-Xlinker", f"-rpath={lib.parent}"]
     res = subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-I", str(tmp_path),
                           "-I", str(CSRC), '-DBES_SYSTEM_DEFINITION="model.cuh"', str(CSRC / "bes_launch.cu"),
-                          str(tmp_path / "main.cu"), "-Xlinker", "--unresolved-symbols=ignore-all", "-o", str(exe)],
+                          str(tmp_path / "main.cu"), *link, "-o", str(exe)],
                          capture_output=True, text=True)
     assert res.returncode == 0, res.stderr[-3000:]
     out = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
@@ -45,3 +49,19 @@ def test_no_teams_for_models_with_shared_values(scope, tmp_path):
 
 def test_teams_for_models_with_unit_values_only(tmp_path):
     assert run_rules(tmp_path, TEAM_OF_EIGHT) == ["11/4", "15/4"]
+
+
+# most banded systems of 33-64 and of 65-128 units to a CTA of eight warps, by band width: what the band, the
+# operator, the vectors and the 21 unit parameters leave room for
+BAND_FITS = {2: {3: 4, 4: 4, 16: 4, 19: 4, 20: 3, 28: 3, 29: 2}, 4: {3: 2, 4: 2, 17: 2, 20: 2, 21: 1, 45: 1, 48: 1}}
+
+
+@pytest.mark.parametrize("rec", [0, 1])
+def test_bands_that_fit(rec, tmp_path, bes_lib):
+    widths = [(g, bw) for g, fits in BAND_FITS.items() for bw in fits]
+    body = "".join(f"""
+    std::printf("%d ", max_warps_per_block(class_variant({g // 2}, false, false, 0, false, {rec}, {bw})) / {g});"""
+                   for g, bw in widths)
+    from bubbleensemble_implicitextension_b200 import _build
+    got = [int(x) for x in run_rules(tmp_path, body, lib=_build.LIB)]
+    assert dict(zip(widths, got)) == {(g, bw): BAND_FITS[g][bw] for g, bw in widths}
