@@ -115,10 +115,19 @@ Variant class_variant(int cls, bool all32, bool shared, int warps_per_system, bo
         return Variant{1, !sym && sparse ? rhs + 7 : rhs, 1, rec};
     }
     const int width = cls == 1 ? 2 : 4;
-    if (!shared && band > 0) return Variant{1, wide ? 10 : dense ? 27 : 7, width, rec, band};   /* banded storage: one unit per lane */
+    /* sixteen warps an SM only where shared memory holds more than the eight of the other kernel */
+    auto denser = [&](Variant v) {
+        const Variant d{v.U, v.rhs + 20, v.G, v.rec, v.band};
+        return dense && max_warps_per_block(d) > max_warps_per_block(v) ? d : v;
+    };
+    if (!shared && band > 0) {   /* banded storage: one unit per lane */
+        const Variant v{1, wide ? 10 : 7, width, rec, band};
+        return wide ? v : denser(v);
+    }
     const int rhs = shared ? (symmetric ? 4 : 3) : 0;
     if (warps_per_system == 1) return Variant{width, rhs, 1, rec};
-    return Variant{1, rhs == 4 && dense ? 24 : rhs, width, rec};
+    const Variant v{1, rhs, width, rec};
+    return rhs == 4 ? denser(v) : v;
 }
 
 /* Can every warp of a team run the model's callbacks and come to the same bits?  Only while the callbacks
@@ -148,7 +157,9 @@ bool sparse_pays(int count, int total, int sm_count) { return count == total && 
 /* Do `count` systems of class cls (1: two warps each, 2: four) run the kernels compiled for sixteen
  * warps an SM?  As soon as there are more than the eight warps of 255 registers hold at once: the
  * 128-register kernels spill a little, but run twice the systems side by side (512 shared-geometry
- * systems of 128 bubbles 331 -> 291 ms, 512 rings of 128 307 -> 252 ms per pass). */
+ * systems of 128 bubbles 331 -> 291 ms, 512 rings of 128 307 -> 252 ms per pass).  Where shared memory
+ * holds no more of them, they only spill: class_variant leaves them out there, and for bands beyond the
+ * registers (512 systems of 128 units at CBW 8: 28.9 -> 18.2 ms without). */
 bool dense_pays(int cls, int count, int sm_count) { return count > (cls == 1 ? 4 : 2) * sm_count; }
 
 /* CTA shape of a launch of `count` systems: spread small ensembles over every

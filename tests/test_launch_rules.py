@@ -12,13 +12,13 @@ CSRC = ROOT / "bubbleensemble_implicitextension_b200" / "csrc"
 SMS = 148
 
 
-def run_rules(tmp_path, body, model="", lib=None):
+def run_rules(tmp_path, body, model="", lib=None, decl=""):
     """Output of `body`, C++ statements over namespace bes; `model`: lines that change the system definition.
     Linked with the library `lib` where the body asks what fits on an SM, else the kernels' entry points stay
     unresolved: the rules alone call none."""
     (tmp_path / "model.cuh").write_text('#include "km_model.cuh"\n' + model)
     (tmp_path / "main.cu").write_text(
-        '#include <cstdio>\n#include "bes_launch.h"\nint main() {\n    using namespace bes;\n' + body + "\n}\n")
+        '#include <cstdio>\n#include "bes_launch.h"\n' + decl + 'int main() {\n    using namespace bes;\n' + body + "\n}\n")
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     exe = tmp_path / "rules"
     link = ["-Xlinker", "--unresolved-symbols=ignore-all"]
@@ -65,3 +65,24 @@ def test_bands_that_fit(rec, tmp_path, bes_lib):
     from bubbleensemble_implicitextension_b200 import _build
     got = [int(x) for x in run_rules(tmp_path, body, lib=_build.LIB)]
     assert dict(zip(widths, got)) == {(g, bw): BAND_FITS[g][bw] for g, bw in widths}
+
+
+@pytest.mark.parametrize("parameters,variants", [(21, ["24/4", "27/4"]), (80, ["4/4", "7/4"])])
+def test_sixteen_warps_only_where_they_fit(parameters, variants, tmp_path):
+    """With 80 unit parameters shared memory holds two systems of 128 units an SM at most: eight warps.  The
+    layouts' sizes are those of the kernels' own macros."""
+    decl = """#include "bes_kernel_inst.cuh"
+namespace bes {
+template <> size_t cta_smem_t<1, 4, 4, 0>(int warps, int band) { return BES_SMEM_SHARED(1, 4, true); }
+template <> size_t cta_smem_t<1, 24, 4, 0>(int warps, int band) { return BES_SMEM_SHARED(1, 4, true); }
+template <> size_t cta_smem_t<1, 7, 4, 0>(int warps, int band) { return BES_SMEM_BAND(4, false); }
+template <> size_t cta_smem_t<1, 27, 4, 0>(int warps, int band) { return BES_SMEM_BAND(4, false); }
+}
+"""
+    body = f"""
+    const bool dense = dense_pays(2, 512, {SMS});
+    const Variant v[2] = {{class_variant(2, false, true, 0, true, 0, 0, false, dense),
+                          class_variant(2, false, false, 0, false, 0, 1, false, dense)}};
+    for (const Variant& x : v) std::printf("%d/%d ", x.rhs, x.G);"""
+    model = f"#undef BES_MODEL_NUP\n#define BES_MODEL_NUP {parameters}\n"
+    assert run_rules(tmp_path, body, model, decl=decl) == variants
