@@ -78,6 +78,14 @@ constexpr int XCH_BUF = 2 * 128 + 8;
  * values of one or two vectors, each run padded by one double2 so that the
  * runs a load reads at once start in different banks */
 constexpr int RED_RUN = 18, RED_BUF = 4 * RED_RUN;
+/* shared memory a CTA can have */
+constexpr int SMEM_MAX = 227 * 1024;
+/* stage derivatives of a system of NMAX units (one unit per lane) that go to shared memory beside
+ * `others` doubles, `systems` times in a CTA, if that fits: a model of many parameters or components
+ * may leave no room, and then they stay in registers */
+__host__ __device__ constexpr int stage_doubles(int nmax, long others, int systems = 1) {
+    return 8L * systems * ((others + 6 * UD * nmax + 31) / 32 * 32) <= SMEM_MAX ? 6 * UD * nmax : 0;
+}
 /* warps of a team: one system of up to 32 units on TEAM warps (RHS > 10: the variant RHS - 10) */
 constexpr int TEAM = 4;
 /* Shared-memory doubles per system (G warps, U units per lane, NMAX = 32 U G
@@ -101,12 +109,12 @@ struct WarpSmem {
     static constexpr int UP_DOUBLES = U == 1 ? NMAX * NUPa : 0; /* unit parameters (one unit per lane) */
     static constexpr int WT_DOUBLES = ONE && T == 1 ? NMAX * NMAX : 0;  /* each lane's column share of W */
     static constexpr int XT_DOUBLES = T > 1 ? 2 * T * 32 : 0;   /* a team's two exchange buffers (its first warp's are used) */
+    static constexpr int OTHERS = W_DOUBLES + WT_DOUBLES + VEC_DOUBLES + XCH_DOUBLES + RED_DOUBLES + SYS_DOUBLES +
+                                  UP_DOUBLES + XT_DOUBLES;
+    static constexpr int K_DOUBLES = U == 1 ? stage_doubles(NMAX, OTHERS, T > 1 ? T : 1) : 0;   /* stage derivatives */
     /* per-system stride rounded up to 256 bytes: every system's vectors stay
      * 16-byte aligned for the double2 broadcast loads */
-    static constexpr int K_DOUBLES = U == 1 ? 6 * UD * NMAX : 0;   /* stage derivatives (one unit per lane) */
-    static constexpr int DOUBLES =
-        (W_DOUBLES + WT_DOUBLES + VEC_DOUBLES + XCH_DOUBLES + RED_DOUBLES + SYS_DOUBLES + UP_DOUBLES + K_DOUBLES + XT_DOUBLES +
-         31) / 32 * 32;
+    static constexpr int DOUBLES = (OTHERS + K_DOUBLES + 31) / 32 * 32;
     static constexpr int BYTES = DOUBLES * 8;
     static_assert(DOUBLES % 2 == 0 && W_DOUBLES % 2 == 0 && NMAX % 2 == 0,
                   "broadcast vectors must start on 16-byte boundaries");
@@ -128,9 +136,9 @@ struct SharedCSmem {
     static constexpr int C_DOUBLES = TMEM ? 0 : NMAX * LDC;
     static constexpr int XCH_DOUBLES = G > 1 ? 2 * XCH_BUF + 8 : 0;
     static constexpr int UP_DOUBLES = U == 1 ? NMAX * NUPa : 0; /* unit parameters (one unit per lane) */
-    static constexpr int K_DOUBLES = U == 1 ? 6 * UD * NMAX : 0;    /* stage derivatives (one unit per lane) */
-    static constexpr int WARP_DOUBLES =
-        (5 * NMAX + XCH_DOUBLES + NSPa + NSAa + NISAa + UP_DOUBLES + K_DOUBLES + 31) / 32 * 32;
+    static constexpr int OTHERS = 5 * NMAX + XCH_DOUBLES + NSPa + NSAa + NISAa + UP_DOUBLES;
+    static constexpr int K_DOUBLES = U == 1 ? stage_doubles(NMAX, C_DOUBLES + OTHERS) : 0;   /* stage derivatives */
+    static constexpr int WARP_DOUBLES = (OTHERS + K_DOUBLES + 31) / 32 * 32;
     static constexpr int C_BYTES = C_DOUBLES * 8;
     static constexpr int WARP_BYTES = WARP_DOUBLES * 8;
     static_assert(C_DOUBLES % 2 == 0 && WARP_DOUBLES % 2 == 0, "16-byte alignment");
@@ -163,11 +171,11 @@ struct BandSmem {
     static constexpr int NMAX = 32 * G;
     static constexpr int XCH_DOUBLES = G > 1 ? 2 * XCH_BUF + 8 : 0;
     static constexpr int RED_DOUBLES = G == 1 ? 2 * RED_BUF : 0;   /* warp_sum32's buffers */
-    static constexpr int K_DOUBLES = WIDE ? 0 : 6 * UD * NMAX;   /* stage derivatives */
+    static constexpr int OTHERS = 6 * NMAX + XCH_DOUBLES + RED_DOUBLES + NSPa + NSAa + NISAa + NMAX * NUPa;
+    static constexpr int K_DOUBLES = WIDE ? 0 : stage_doubles(NMAX, 2 * (BAND_REGS - 1) * NMAX + OTHERS);   /* stage derivatives */
     __host__ __device__ static constexpr int diagonals(int bw) { return 2 * bw + 1 < NMAX ? 2 * bw + 1 : NMAX; }
     __host__ __device__ static constexpr int doubles(int bw) {
-        return (2 * diagonals(bw) * NMAX + 6 * NMAX + XCH_DOUBLES + RED_DOUBLES + NSPa + NSAa + NISAa + NMAX * NUPa +
-                K_DOUBLES + 31) / 32 * 32;
+        return (2 * diagonals(bw) * NMAX + OTHERS + K_DOUBLES + 31) / 32 * 32;
     }
 };
 
@@ -2142,9 +2150,17 @@ __device__ __forceinline__ double* upar_of(const Sys<U, G>& S, Lane<U>& L, int m
     else return L.up[m];
 }
 
+/* the shared-memory layout of a one-system-at-a-time variant */
+template <int U, int RHS, int G>
+using OwnSmem = WarpSmem<U, G, (RHS > 10 ? TEAM : RHS > 7 ? 0 : 1)>;
+
 /* are a variant's stage derivatives in shared memory */
-template <int U, int RHS>
-__device__ constexpr bool stages_shared() { return U == 1 && RHS != 10; }
+template <int U, int RHS, int G>
+__device__ constexpr bool stages_shared() {
+    if constexpr (RHS == 3 || RHS == 4) return SharedCSmem<U, G, RHS == 4>::K_DOUBLES > 0;
+    else if constexpr (RHS == 7 || RHS == 10) return BandSmem<G, RHS == 10>::K_DOUBLES > 0;
+    else return OwnSmem<U, RHS, G>::K_DOUBLES > 0;
+}
 
 /* The stage derivatives K_j of this lane's units: SHARED in shared memory (each
  * is written once and read a few times a step, while the BiCG needs the
@@ -2194,8 +2210,8 @@ template <int U, int RHS, int G, int REC>
 __device__ __forceinline__ bool step_rkck45(const Sys<U, G>& S, const DeviceProblem& P, Lane<U>& L,
                                             double T, double dt, double (&Yn)[U][UD], double (&E)[U][UD],
                                             Counters& cnt, bool& capped) {
-    Stages<U, G, 6, stages_shared<U, RHS>()> K;
-    if constexpr (!stages_shared<U, RHS>()) {
+    Stages<U, G, 6, stages_shared<U, RHS, G>()> K;
+    if constexpr (!stages_shared<U, RHS, G>()) {
 #pragma unroll
         for (int j = 0; j < 6; j++)
 #pragma unroll
@@ -2256,8 +2272,8 @@ __device__ __forceinline__ bool step_rkck45(const Sys<U, G>& S, const DeviceProb
 template <int U, int RHS, int G, int REC>
 __device__ __forceinline__ bool step_rk4(const Sys<U, G>& S, const DeviceProblem& P, Lane<U>& L,
                                          double T, double dt, double (&Yn)[U][UD], Counters& cnt, bool& capped) {
-    Stages<U, G, 4, stages_shared<U, RHS>()> K;
-    if constexpr (!stages_shared<U, RHS>()) {
+    Stages<U, G, 4, stages_shared<U, RHS, G>()> K;
+    if constexpr (!stages_shared<U, RHS, G>()) {
 #pragma unroll
         for (int j = 0; j < 4; j++)
 #pragma unroll
@@ -2772,7 +2788,7 @@ __global__ void __launch_bounds__(V > 20 ? 512 : V == 3 || V == 4 || V == 7 || V
         S.sPAR = S.xch + SM::XCH_DOUBLES + SM::RED_DOUBLES;
         S.upsh = S.sPAR + NSPa + NSAa + NISAa;
     } else {
-        using SM = WarpSmem<U, G, (RHS > 10 ? TEAM : RHS > 7 ? 0 : 1)>;
+        using SM = OwnSmem<U, RHS, G>;
         double* base = smem + (size_t)slot * SM::DOUBLES;
         if constexpr (RHS > 10) S.xt = base - (size_t)S.tw * SM::DOUBLES + SM::DOUBLES - SM::XT_DOUBLES;
         S.W = base;

@@ -79,7 +79,7 @@ int max_warps_per_block(Variant v) {
     /* the kernels' launch bounds: 256 threads with RHS 3 or G > 1, else 128 */
     const int cap = v.rhs > 20 ? 16 : (v.rhs == 3 || v.rhs == 4 || v.rhs == 7 || v.rhs == 10 || v.G > 1) ? 8 : 4;
     int w = 0;
-    while (w + v.G <= cap && cta_smem_bytes(v, w + v.G) <= 227 * 1024) w += v.G;
+    while (w + v.G <= cap && cta_smem_bytes(v, w + v.G) <= (size_t)SMEM_MAX) w += v.G;
     return w;
 }
 
@@ -134,14 +134,14 @@ Variant class_variant(int cls, bool all32, bool shared, int warps_per_system, bo
  * write nothing but their own unit's values: a global parameter would be written four times, and each warp
  * has its own copy of the system-scope values, on which the units of a system may race (plain stores, atomic
  * sums).  Nothing orders those alike in two warps, so the copies could differ, the warps decide differently,
- * and one wait at a team barrier for an exchange that the others never make. */
+ * and one wait at a team barrier for an exchange that the others never make.  The four warps' copies have to
+ * fit in shared memory, too. */
 constexpr bool TEAM_MODEL = BES_MODEL_NGP == 0 && BES_MODEL_NIGP == 0 && BES_MODEL_NSP == 0 && BES_MODEL_NSA == 0 &&
-                            BES_MODEL_NISA == 0;
+                            BES_MODEL_NISA == 0 && TEAM * WarpSmem<1, 1, TEAM>::BYTES <= SMEM_MAX;
 
 /* Does a launch of `total` systems run those of up to 32 units on teams of four warps (where TEAM_MODEL
- * allows them)?  Eight warps of
- * 255 registers are what an SM holds, and a team's warps repeat everything but the products, so a
- * system to an SM always gains (8 bubbles alone 33.0 -> 31.6 ms, 64 x 16 bubbles with RK4 17.4 -> 16.2),
+ * allows them)?  Eight warps of 255 registers are what an SM holds, and a team's warps repeat everything but
+ * the products, so a system to an SM always gains (8 bubbles alone 33.0 -> 31.6 ms, 64 x 16 bubbles with RK4 17.4 -> 16.2),
  * two only with the shared symmetric matrix (256 x 32: 331 -> 324 and 325 -> 289 ms of two draws; own
  * matrix 322 -> 326), and beside multi-warp systems none (384 uneven clouds: 92 -> 112 ms). */
 bool team_pays(int total, bool symmetric, int sm_count) {

@@ -47,6 +47,10 @@ def test_no_teams_for_models_with_shared_values(scope, tmp_path):
     assert run_rules(tmp_path, TEAM_OF_EIGHT, f"#undef BES_MODEL_{scope}\n#define BES_MODEL_{scope} 1\n") == ["1/1", "5/1"]
 
 
+def test_no_teams_for_models_too_large_for_four_copies(tmp_path):
+    assert run_rules(tmp_path, TEAM_OF_EIGHT, "#undef BES_MODEL_NUP\n#define BES_MODEL_NUP 200\n") == ["1/1", "5/1"]
+
+
 def test_teams_for_models_with_unit_values_only(tmp_path):
     assert run_rules(tmp_path, TEAM_OF_EIGHT) == ["11/4", "15/4"]
 
@@ -86,3 +90,17 @@ template <> size_t cta_smem_t<1, 27, 4, 0>(int warps, int band) { return BES_SME
     for (const Variant& x : v) std::printf("%d/%d ", x.rhs, x.G);"""
     model = f"#undef BES_MODEL_NUP\n#define BES_MODEL_NUP {parameters}\n"
     assert run_rules(tmp_path, body, model, decl=decl) == variants
+
+
+@pytest.mark.parametrize("components,parameters", [(2, 87), (6, 80), (12, 85)])
+def test_models_up_to_the_limit_of_shared_memory(components, parameters, tmp_path):
+    """128 units with a full matrix, their vectors and exchange buffers leave room for 87 unit parameters: whatever
+    else a kernel keeps in shared memory has to give way."""
+    body = """
+    std::printf("%d %d %d", WarpSmem<1, 4>::BYTES <= SMEM_MAX,
+                SharedCSmem<1, 4, false>::C_BYTES + SharedCSmem<1, 4, false>::WARP_BYTES <= SMEM_MAX,
+                BandSmem<4, true>::doubles(16) * 8 <= SMEM_MAX);"""
+    model = (f"#undef BES_MODEL_NUP\n#define BES_MODEL_NUP {parameters}\n"
+             f"#undef BES_MODEL_UD\n#define BES_MODEL_UD {components}\n")
+    decl = '#include "bes_kernel.cuh"\n'
+    assert run_rules(tmp_path, body, model, decl=decl) == ["1", "1", "1"]
