@@ -1111,7 +1111,7 @@ bes_status bes_solve_periods(bes_solver* h, int32_t n_periods, int32_t reset_at)
                 return fail(h, BES_ERR_ARGUMENT,
                             "bes_solve_periods: CouplingRowScale / CouplingColumnScale hold values other than 1, "
                             "which only the shared-matrix kernels apply: turn SharedCouplingMatrices on and give "
-                            "every system of a size class the same matrix (systems of more than 32 units)");
+                            "every system of a size class the same matrix (up to 32 units: one equal to its transpose)");
     if (!h->use_graph) {
         CUDA_TRY(h, cudaEventRecord(h->t0, h->stream));
         if ((st = enqueue_solve(h, P, h->stream, L, &h->last_launches))) return st;

@@ -2845,7 +2845,7 @@ __global__ void __launch_bounds__(V > 20 ? 512 : V == 3 || V == 4 || V == 7 || V
 #pragma unroll
                 for (int c = 0; c < NUP; c++) L.up[m][c] = v ? __ldg(P.upar + (int64_t)c * S.tot + g) : 0.0;
             }
-            if constexpr ((RHS >= 3 && RHS <= 7) || RHS > 14) {
+            if constexpr ((RHS >= 3 && RHS <= 6) || RHS > 14) {   /* the shared-matrix kernels */
                 L.ra[m] = v ? (P.coupling_row_scale ? __ldg(P.coupling_row_scale + g) : 1.0) : 0.0;
                 L.cb[m] = v ? (P.coupling_col_scale ? __ldg(P.coupling_col_scale + g) : 1.0) : 0.0;
             } else {

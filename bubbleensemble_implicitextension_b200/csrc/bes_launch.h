@@ -34,9 +34,9 @@ struct Variant {
     int band = 0;   /* band width of the banded variants (RHS 7, 10) */
 };
 
-/* does the variant read each system's own full matrix (no unit coupling factors applied) */
+/* does the variant read each system's own matrix, full or banded (no unit coupling factors applied) */
 inline bool own_matrix(const Variant& v) {
-    return v.rhs < 3 || v.rhs == 8 || v.rhs == 9 || v.rhs == 11 || v.rhs == 12;
+    return v.rhs < 3 || (v.rhs >= 7 && v.rhs <= 12) || v.rhs == 27;
 }
 /* is (U, RHS, G) one of the built variants */
 bool variant_exists(Variant v);

@@ -72,8 +72,10 @@ typedef int32_t bes_status;
                                               C_ij = a_i G_ij b_j, G the stored (shared) matrix; default 1.
                                               One geometry G = 1/d_ij serves systems with their own radii
                                               (a_i = R_i^-2, b_j = R_j^3).  Applied by the shared-matrix
-                                              kernels only (SharedCouplingMatrices, more than 32 units);
-                                              a solve with other launches and factors != 1 is an error. */
+                                              kernels only (SharedCouplingMatrices and one matrix per size
+                                              class; up to 32 units one equal to its transpose); a solve
+                                              with other launches, banded ones among them, and factors
+                                              != 1 is an error. */
 #define BES_POINCARE_SECTIONS 105          /* [sections][total_units] per-period analysis outputs (device -> host), */
 #define BES_PERIOD_NUMBER 106              /* [total_units] int32       see bes_set_period_analysis              */
 #define BES_MAXIMUM_ACCESSORY 107          /* [total_units]                                                       */

@@ -99,3 +99,18 @@ def test_unit_factors_need_a_shared_matrix(systems, gpu):
             ps.solve_periods(1, -1)
     finally:
         ps.close()
+
+
+@pytest.mark.parametrize("n,bw,systems", [(20, 2, 4), (50, 1, 4), (128, 1, 320), (128, 9, 4), (32, 9, 4)])
+def test_unit_factors_are_refused_with_banded_storage(n, bw, systems, gpu):
+    """Narrow and wide bands on one, two and four warps, and the kernel of many systems."""
+    from bubbleensemble_implicitextension_b200 import solver as S
+    ens = W.ring_ensemble(n_systems=systems, n_units=n, band_width=bw)
+    ps = ens.make_solver()
+    try:
+        ps.set_array(S.ListOfVariables.CouplingColumnScale, np.full(ens.total_units, 2.0))
+        ps.SynchroniseFromHostToDevice(S.ListOfVariables.All)
+        with pytest.raises(S.BesError, match="CouplingColumnScale"):
+            ps.solve_periods(1, -1)
+    finally:
+        ps.close()

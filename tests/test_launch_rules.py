@@ -104,3 +104,24 @@ def test_models_up_to_the_limit_of_shared_memory(components, parameters, tmp_pat
              f"#undef BES_MODEL_UD\n#define BES_MODEL_UD {components}\n")
     decl = '#include "bes_kernel.cuh"\n'
     assert run_rules(tmp_path, body, model, decl=decl) == ["1", "1", "1"]
+
+
+def test_which_variants_read_each_systems_own_matrix(tmp_path):
+    """Only the shared-matrix kernels apply unit coupling factors: every other variant, the banded ones of one, two
+    and four warps among them, counts as reading the system's own matrix, and factors are refused there."""
+    body = """
+    for (int cls = 0; cls < 3; cls++)
+        for (int band : {0, 1, 9})
+            for (int shared = 0; shared < 3; shared++)      /* 2: symmetric too */
+                for (int wps = 0; wps < 2; wps++)
+                    for (int rule = 0; rule < 4; rule++) {  /* none, team, dense, sparse */
+                        const Variant v = class_variant(cls, rule == 0, shared > 0, wps, shared == 2, 0, band,
+                                                        rule == 1, rule == 2, rule == 3);
+                        const bool applied = shared > 0 && (cls > 0 || shared == 2);
+                        if (own_matrix(v) == applied) std::printf("%d/%d/%d ", v.U, v.rhs, v.G);
+                    }
+    std::printf("done");"""
+    decl = "namespace bes {\n" + "".join(
+        f"template <> size_t cta_smem_t<1, {rhs}, {g}, 0>(int w, int) {{ return 1024 * w; }}\n"
+        for rhs in (4, 7, 24, 27) for g in (2, 4)) + "}\n"
+    assert run_rules(tmp_path, body, decl=decl) == ["done"]
