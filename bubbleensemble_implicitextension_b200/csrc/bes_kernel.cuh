@@ -74,10 +74,10 @@ constexpr unsigned FULL = 0xffffffffu;
 /* one group-exchange buffer: two values per unit of the largest group
  * (128 units) and one flag word per warp, padded to 16-byte multiples */
 constexpr int XCH_BUF = 2 * 128 + 8;
-/* one buffer of warp_sum32 / warp_sum32x2: the 16 even and the 16 odd units'
- * values of one or two vectors, each run padded by one double2 so that the
- * runs a load reads at once start in different banks */
-constexpr int RED_RUN = 18, RED_BUF = 4 * RED_RUN;
+/* one buffer of warp_sum32, or one vector split by parity: the 16 even and the 16
+ * odd units' values, each run padded by one double2 so that the two that a load
+ * reads at once start in different banks */
+constexpr int RED_RUN = 18, RED_BUF = 2 * RED_RUN;
 /* shared memory a CTA can have */
 constexpr int SMEM_MAX = 227 * 1024;
 /* stage derivatives of a system of NMAX units (one unit per lane) that go to shared memory beside
@@ -105,7 +105,7 @@ struct WarpSmem {
     static constexpr int VEC_DOUBLES = 6 * NMAX;
     static constexpr int XCH_DOUBLES = G > 1 ? 2 * XCH_BUF + 8 : 0; /* two buffers of two values per unit, vote words */
     static constexpr int SYS_DOUBLES = NSPa + NSAa + NISAa;  /* ints stored in double slots */
-    static constexpr int RED_DOUBLES = ONE ? 3 * RED_BUF : 0;   /* warp_sum32's buffers, two vectors by parity */
+    static constexpr int RED_DOUBLES = ONE ? 4 * RED_BUF : 0;   /* warp_sum32's buffers, two vectors by parity */
     static constexpr int UP_DOUBLES = U == 1 ? NMAX * NUPa : 0; /* unit parameters (one unit per lane) */
     static constexpr int WT_DOUBLES = ONE && T == 1 ? NMAX * NMAX : 0;  /* each lane's column share of W */
     static constexpr int XT_DOUBLES = T > 1 ? 2 * T * 32 : 0;   /* a team's two exchange buffers (its first warp's are used) */
@@ -310,31 +310,6 @@ __device__ __forceinline__ double warp_sum32(const Sys<1, 1>& S, double v) {
     return s + __shfl_xor_sync(FULL, s, 1);
 }
 
-/* The sums of two vectors at once, each as warp_sum32 forms it: a quarter of the
- * warp adds one parity of one vector, so both cost the loads and additions of
- * one and a second shuffle (a paired butterfly: 196 cycles and twenty shuffles). */
-__device__ __forceinline__ void warp_sum32x2(const Sys<1, 1>& S, double v, double w, double& sv, double& sw) {
-    double* buf = S.xch + (S.xsel & 1) * RED_BUF;
-    S.xsel++;
-    buf[par_slot(S.lane)] = v;
-    buf[2 * RED_RUN + par_slot(S.lane)] = w;
-    __syncwarp();
-    const double2* mine = reinterpret_cast<const double2*>(buf + (S.lane >> 3) * RED_RUN);
-    double a[16];
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-        const double2 t = mine[k];
-        a[2 * k] = t.x;
-        a[2 * k + 1] = t.y;
-    }
-    auto leaf = [&](int k) -> double { return a[k]; };
-    double s = TreeSum<1, 16>::run(0, leaf);
-    s = s + __shfl_xor_sync(FULL, s, 8);
-    const double o = __shfl_xor_sync(FULL, s, 16);
-    sv = S.lane & 16 ? o : s;
-    sw = S.lane & 16 ? s : o;
-}
-
 /* a[k][b]: value k of this lane's unit in block b = G m + wis, for all U G blocks */
 template <int U, int G, int K>
 __device__ __forceinline__ void grp_gather(const Sys<U, G>& S, const double (&v)[K][U], double (&a)[K][U * G]) {
@@ -516,7 +491,10 @@ __device__ __forceinline__ int grp_resolve_int(const Sys<U, G>& S, int before, i
 }
 
 /* Two sums over all 32U units of the warp, each in halving-tree order (the
- * shuffles of the two butterflies interleave); every lane gets both. */
+ * shuffles of the two butterflies interleave); every lane gets both.  One sum is
+ * shorter through shared memory (warp_sum32), two are not: 300 systems of 32
+ * units with their own matrices, 250 steps with REC 1, 5.94 ms so and 5.55 with
+ * the butterflies. */
 template <int U>
 __device__ __forceinline__ void warp_tree_sum2(const double (&v)[U], const double (&w)[U], double& sv, double& sw) {
     double a[U], b[U];
@@ -541,9 +519,7 @@ __device__ __forceinline__ void warp_tree_sum2(const double (&v)[U], const doubl
 template <int U, int G>
 __device__ __forceinline__ void grp_tree_sum2(const Sys<U, G>& S, const double (&v)[U], const double (&w)[U],
                                               double& sv, double& sw) {
-    if constexpr (U == 1 && G == 1) {
-        warp_sum32x2(S, v[0], w[0], sv, sw);
-    } else if constexpr (G == 1) {
+    if constexpr (G == 1) {
         warp_tree_sum2<U>(v, w, sv, sw);
     } else {
         double in[2][U], a[2][U * G];
@@ -639,9 +615,14 @@ __device__ __forceinline__ bool grp_read_max_below(const Sys<U, G>& S) {
  * and its instruction count.  Both quotients of either recurrence go on as
  * Markstein's and are proven at the end of the iteration, together with the
  * exit test, so the loop has one branch (a proof's comparison and branch on the
- * chain cost 60 cycles each, twice an iteration); an unproven one drops the
- * iteration, which is then done with IEEE divisions.  Returns the completed
- * iterations; sets capped when the cap ended the loop. */
+ * chain cost 60 cycles each, twice an iteration).  With an unproven one the
+ * update is dropped and done with IEEE divisions.  The iteration is repeated for
+ * that, but with REC 1, whose products do not need the quotients, a single warp
+ * repeats the update only: a second copy of the iteration beside the loop cost
+ * it registers (700 systems of 31 units 11.5 -> 10.7 ms without), while the
+ * kernels of 128 registers lose by keeping the products until the proof (1200
+ * systems of 64 units with a shared matrix: 13.3 ms, 13.8 so).  Returns the
+ * completed iterations; sets capped when the cap ended the loop. */
 template <int U, int G, int REC, class Put, class Mul>
 __device__ __forceinline__ int bicg_iterate(const Sys<U, G>& S, const DeviceProblem& P, const double (&b)[U],
                                             double (&r)[U], double (&x)[U], Put&& put, Mul&& mul, bool& capped) {
@@ -726,8 +707,23 @@ __device__ __forceinline__ int bicg_iterate(const Sys<U, G>& S, const DeviceProb
 #pragma unroll
         for (int m = 0; m < U; m++) { q[m] = 0.0; qt[m] = 0.0; }
         double sigma = 0.0, rho_prev = 1.0, y_prev = 1.0;   /* y_prev: reciprocal estimate of rho_prev */
-        double rho, sg, y1, pn[U], ptn[U], qn[U], qtn[U], xn[U], rn[U], rtn[U];
+        double rho, mu, sg, y1, pn[U], ptn[U], qn[U], qtn[U], xn[U], rn[U], rtn[U];
         bool small = false, proven = true, early = false;
+        /* the iterates pn .. rtn that the quotients lead to, and a single warp's exit test on them */
+        auto update = [&](double beta, double alpha) {
+#pragma unroll
+            for (int m = 0; m < U; m++) {
+                pn[m] = fma(beta, p[m], r[m]);
+                ptn[m] = fma(beta, pt[m], rt[m]);
+                qn[m] = fma(beta, q[m], w[m]);
+                qtn[m] = fma(beta, qt[m], wt[m]);
+                xn[m] = fma(alpha, pn[m], x[m]);
+                rn[m] = fma(-alpha, qn[m], r[m]);
+                rtn[m] = fma(-alpha, qtn[m], rt[m]);
+                ar[m] = fabs(rn[m]);
+            }
+            if constexpr (G == 1) small = grp_max_below<U, G>(S, ar, 1e-6);
+        };
         /* one iteration into pn .. rtn and sg: nothing is committed */
         auto iteration = [&](auto ieee) {
             if (G == 1 || done == 0) grp_sync(S);
@@ -740,7 +736,6 @@ __device__ __forceinline__ int bicg_iterate(const Sys<U, G>& S, const DeviceProb
                 early = done > 0 && !decltype(ieee)::value && grp_read_max_below<U, G>(S);
                 if (early) return;
             }
-            double mu;
 #pragma unroll
             for (int m = 0; m < U; m++) prod[m] = r[m] * rt[m];
             mul(r, rt, w, wt);
@@ -756,18 +751,7 @@ __device__ __forceinline__ int bicg_iterate(const Sys<U, G>& S, const DeviceProb
                                      ? math::div_ieee(rho, sg)
                                      : math::div_markstein(rho, sg, math::recip_estimate(sg), alpha_ok);   /* = rho / sigma */
             y1 = math::recip_estimate(rho);
-#pragma unroll
-            for (int m = 0; m < U; m++) {
-                pn[m] = fma(beta, p[m], r[m]);
-                ptn[m] = fma(beta, pt[m], rt[m]);
-                qn[m] = fma(beta, q[m], w[m]);
-                qtn[m] = fma(beta, qt[m], wt[m]);
-                xn[m] = fma(alpha, pn[m], x[m]);
-                rn[m] = fma(-alpha, qn[m], r[m]);
-                rtn[m] = fma(-alpha, qtn[m], rt[m]);
-                ar[m] = fabs(rn[m]);
-            }
-            if constexpr (G == 1) small = grp_max_below<U, G>(S, ar, 1e-6);
+            update(beta, alpha);
             proven = decltype(ieee)::value || __all_sync(FULL, beta_ok && alpha_ok);
             early = done == 0 && __all_sync(FULL, fabs(rho) < 1e-6);   /* the first rho test: the update is dropped */
         };
@@ -791,8 +775,13 @@ __device__ __forceinline__ int bicg_iterate(const Sys<U, G>& S, const DeviceProb
                 }
                 if (early) { exited = true; break; }
                 if (!proven) {
-                    iteration(Const<1>{});   /* the previous update's exit test is not repeated */
-                    if (early) { exited = true; break; }
+                    if constexpr (G == 1) {   /* the products, rho and mu stand */
+                        const double beta = done == 0 ? 0.0 : math::div_ieee(rho, rho_prev);
+                        sg = fma(-(beta * beta), sigma, mu);
+                        update(beta, math::div_ieee(rho, sg));
+                    } else {
+                        iteration(Const<1>{});   /* the previous update's exit test is not repeated */
+                    }
                 }
                 commit();
                 exited = small;
@@ -1702,22 +1691,34 @@ __device__ __forceinline__ int coupled_rhs_symquad(const Sys<1, G>& S, const Dev
 /* ---------------------------------------------------------------------------
  * Coupled right-hand side for N <= 32 when the launch shares one symmetric
  * matrix G (RHS = 5; 6 drops the N guards when every system has 32 units):
- * a lane keeps its share of G (two rows, two chains: 32 entries) in registers
- * for the whole system -- nothing is formed per right-hand side -- and both BiCG
- * products are row sums of those entries against posted vectors, with the unit
- * factors a, b as in coupled_rhs_sharedc<.., SYM = true> and the same arithmetic
- * order. */
+ * a lane's share of G (two rows, two chains: 32 entries) is staged in shared
+ * memory once per system, lane-consecutive, and taken into registers for a
+ * right-hand side -- nothing is formed -- and both BiCG products are row sums of
+ * those entries against posted vectors, with the unit factors a, b as in
+ * coupled_rhs_sharedc<.., SYM = true> and the same arithmetic order.  Held in
+ * registers for the whole system the share left too few of them outside the
+ * products: the compiler kept part of it in local memory, whose loads miss the
+ * small L1 that 230 KB of shared memory leave (300 systems of 31 units, 250
+ * steps: 7.7 -> 6.75 ms, with REC 1 8.7 -> 6.95). */
 template <int NFIX, int REC>
 __device__ __forceinline__ int coupled_rhs_regsym(const Sys<1>& S, const DeviceProblem& P, double T,
                                                   double (&Xs)[1][UD], double (&F)[1][UD], double (&ua)[1][NUAa],
                                                   int (&iua)[1][NIUAa], const double (&ra)[1], const double (&cb)[1],
-                                                  const double (&g)[32], bool& capped) {
+                                                  bool& capped) {
     const int N = NFIX ? NFIX : S.N;
     const int i = S.lane;
     const int h = i & 1;
     const bool valid = i < N;
     double xu = 0.0, rd = 0.0, x1 = 0.0;
     __syncwarp();
+    double g[32];   /* this lane's share of G */
+    const double2* share = reinterpret_cast<const double2*>(S.W) + i;
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+        const double2 t = share[32 * k];
+        g[2 * k] = t.x;
+        g[2 * k + 1] = t.y;
+    }
     if (valid) {
         double Fl[UD], cpt, cpf;
         CoupledSystems_PerBlock_OdeFunction<double>(S.sid, i, Fl, Xs[0], T, S.upsh + i * NUPa, S.sPAR, S.gPAR,
@@ -1824,7 +1825,7 @@ __device__ __forceinline__ void team_exchange(const Sys<1>& S, double partial, d
 template <bool SYM, int NFIX, int REC>
 __device__ __forceinline__ int coupled_rhs_team(const Sys<1>& S, const DeviceProblem& P, double T, double (&Xs)[1][UD],
                                                 double (&F)[1][UD], double (&ua)[1][NUAa], int (&iua)[1][NIUAa],
-                                                const double (&ra)[1], const double (&cb)[1], const double (&g)[32],
+                                                const double (&ra)[1], const double (&cb)[1], const double (&g)[16],
                                                 bool& capped) {
     constexpr int LDC = WarpSmem<1>::LDW;
     const int N = NFIX ? NFIX : S.N;
@@ -2100,7 +2101,7 @@ template <int U, int RHS, int G, int REC>
 __device__ __forceinline__ int rhs_eval(const Sys<U, G>& S, const DeviceProblem& P, double T, double (&Xs)[U][UD],
                                         double (&F)[U][UD], double (&up)[U][NUPa], double (&ua)[U][NUAa],
                                         int (&iua)[U][NIUAa], const double (&ra)[U], const double (&cb)[U],
-                                        const double (&grow)[32], bool& capped) {
+                                        const double (&grow)[16], bool& capped) {
     if constexpr (RHS == 0 && U == 1) {
         return coupled_rhs_quad<G, REC>(S, P, T, Xs, F, ua, iua, capped);
     } else if constexpr (RHS == 0) {
@@ -2113,7 +2114,7 @@ __device__ __forceinline__ int rhs_eval(const Sys<U, G>& S, const DeviceProblem&
         return coupled_rhs_team<(RHS > 14), RHS % 2 == 0 ? 32 : 0, REC>(S, P, T, Xs, F, ua, iua, ra, cb, grow, capped);
     } else if constexpr (RHS == 5 || RHS == 6) {
         static_assert(U == 1 && G == 1, "the register-resident operator needs one unit per lane");
-        return coupled_rhs_regsym<RHS == 6 ? 32 : 0, REC>(S, P, T, Xs, F, ua, iua, ra, cb, grow, capped);
+        return coupled_rhs_regsym<RHS == 6 ? 32 : 0, REC>(S, P, T, Xs, F, ua, iua, ra, cb, capped);
     } else if constexpr (RHS == 7 || RHS == 10) {
         static_assert(U == 1, "the banded operator runs one unit per lane");
         return coupled_rhs_band<G, RHS == 10, REC>(S, P, T, Xs, F, ua, iua, capped);
@@ -2132,7 +2133,7 @@ struct Lane {
     int iua[U][NIUAa];
     double ev_a[U][NEa], ev_n[U][NEa];
     double ra[U], cb[U];   /* coupling factors a_i, b_i of the shared-matrix kernels */
-    double grow[32];       /* this lane's share of the shared symmetric matrix (RHS 5, 6) */
+    double grow[16];       /* this lane's share of the shared symmetric matrix (teams) */
 };
 
 struct Counters {
@@ -2800,7 +2801,7 @@ __global__ void __launch_bounds__(V > 20 ? 512 : V == 3 || V == 4 || V == 7 || V
         S.vrd = S.vxu + SM::NMAX;
         S.xch = S.vrd + SM::NMAX;
         S.tpar = S.xch + 2 * RED_BUF;   /* U = G = 1 */
-        S.rdpar = S.tpar + 2 * RED_RUN;
+        S.rdpar = S.tpar + RED_BUF;
         S.flag = S.xch + 2 * XCH_BUF;
         S.sPAR = S.xch + SM::XCH_DOUBLES + SM::RED_DOUBLES;
         S.upsh = S.sPAR + SM::SYS_DOUBLES;
@@ -2879,11 +2880,13 @@ __global__ void __launch_bounds__(V > 20 ? 512 : V == 3 || V == 4 || V == 7 || V
             }
         }
         if constexpr (RHS == 5 || RHS == 6) {
-            /* rows 2r, 2r + 1 of the shared symmetric matrix at the columns 4t + 2h + e of lane 2r + h, zero-padded */
+            /* rows 2r, 2r + 1 of the shared symmetric matrix at the columns 4t + 2h + e for lane 2r + h, zero-padded,
+             * its entries k and k + 1 as one double2 among the lanes' */
 #pragma unroll
             for (int k = 0; k < 32; k++) {
                 const int row = (lane & ~1) + (k >> 4), j = 4 * ((k & 15) >> 1) + 2 * (lane & 1) + (k & 1);
-                L.grow[k] = (row < S.N && j < S.N) ? __ldg(S.C + row + (int64_t)j * S.N) : 0.0;
+                S.W[2 * (32 * (k >> 1) + lane) + (k & 1)] =
+                    (row < S.N && j < S.N) ? __ldg(S.C + row + (int64_t)j * S.N) : 0.0;
             }
         }
         if constexpr (BAND) {
