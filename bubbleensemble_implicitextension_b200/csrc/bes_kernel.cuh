@@ -621,11 +621,17 @@ __device__ __forceinline__ bool grp_read_max_below(const Sys<U, G>& S) {
  * repeats the update only: a second copy of the iteration beside the loop cost
  * it registers (700 systems of 31 units 11.5 -> 10.7 ms without), while the
  * kernels of 128 registers lose by keeping the products until the proof (1200
- * systems of 64 units with a shared matrix: 13.3 ms, 13.8 so).  Returns the
- * completed iterations; sets capped when the cap ended the loop. */
-template <int U, int G, int REC, class Put, class Mul>
+ * systems of 64 units with a shared matrix: 13.3 ms, 13.8 so).
+ * IN_PLACE: several units a lane have no registers for a second set of iterates
+ * (148 systems of 128 units on one warp, own matrices: 292 -> 205 ms without
+ * it), so each quotient is settled before it is used and the iterates are
+ * updated in place.  With a shared matrix REC 0 is faster with the second set
+ * all the same (239 ms, 250 in place).
+ * Returns the completed iterations; sets capped when the cap ended the loop. */
+template <int U, int G, int REC, bool IN_PLACE = false, class Put, class Mul>
 __device__ __forceinline__ int bicg_iterate(const Sys<U, G>& S, const DeviceProblem& P, const double (&b)[U],
                                             double (&r)[U], double (&x)[U], Put&& put, Mul&& mul, bool& capped) {
+    static_assert(!IN_PLACE || G == 1, "updates in place are for one warp");
     double rt[U], p[U], pt[U], ar[U];
     const int max_iter = P.bicg_max_iter;
 #pragma unroll
@@ -640,6 +646,37 @@ __device__ __forceinline__ int bicg_iterate(const Sys<U, G>& S, const DeviceProb
         if (max_iter < 1) return;
         if (__all_sync(FULL, fabs(rho1) < 1e-6)) { exited = true; return; }
         double rho2 = 1.0, y2 = 1.0;   /* y2: reciprocal estimate of rho2, formed an iteration early */
+        if constexpr (IN_PLACE) {
+            for (int it = 1; it <= max_iter; it++) {
+                const double beta = it == 1 ? 0.0 : math::div_known(rho1, rho2, y2);   /* = rho1 / rho2; p = r first */
+#pragma unroll
+                for (int m = 0; m < U; m++) {
+                    p[m] = fma(beta, p[m], r[m]);
+                    pt[m] = fma(beta, pt[m], rt[m]);
+                }
+                __syncwarp();
+                put(p, pt);
+                __syncwarp();
+                rho2 = rho1;
+                y2 = math::recip_estimate(rho2);
+                mul(p, pt, q, qt);
+#pragma unroll
+                for (int m = 0; m < U; m++) prod[m] = pt[m] * q[m];
+                const double sig = grp_tree_sum<U, G>(S, prod);
+                const double alpha = math::div_known(rho2, sig, math::recip_estimate(sig));   /* = rho / sigma */
+#pragma unroll
+                for (int m = 0; m < U; m++) {
+                    x[m] = fma(alpha, p[m], x[m]);
+                    r[m] = fma(-alpha, q[m], r[m]);
+                    rt[m] = fma(-alpha, qt[m], rt[m]);
+                    ar[m] = fabs(r[m]);
+                    prod[m] = r[m] * rt[m];
+                }
+                done++;
+                if (grp_sum_max_below<U, G>(S, ar, prod, 1e-6, rho1)) { exited = true; break; }
+            }
+            return;
+        }
         double pn[U], ptn[U], xn[U], rn[U], rtn[U], rho_next, y1;
         bool small, proven;
         int it = 0;   /* committed iterations of this solve (done counts a redone solve's too) */
@@ -707,6 +744,37 @@ __device__ __forceinline__ int bicg_iterate(const Sys<U, G>& S, const DeviceProb
 #pragma unroll
         for (int m = 0; m < U; m++) { q[m] = 0.0; qt[m] = 0.0; }
         double sigma = 0.0, rho_prev = 1.0, y_prev = 1.0;   /* y_prev: reciprocal estimate of rho_prev */
+        if constexpr (IN_PLACE) {
+            for (int it = 1; it <= max_iter; it++) {
+                __syncwarp();
+                put(r, rt);
+                __syncwarp();
+                mul(r, rt, w, wt);
+#pragma unroll
+                for (int m = 0; m < U; m++) { prod[m] = r[m] * rt[m]; rw[m] = rt[m] * w[m]; }
+                double rho, mu;
+                grp_tree_sum2<U, G>(S, prod, rw, rho, mu);
+                if (it == 1 && __all_sync(FULL, fabs(rho) < 1e-6)) { exited = true; break; }
+                const double beta = it == 1 ? 0.0 : math::div_known(rho, rho_prev, y_prev);   /* = rho / rho_prev */
+                sigma = fma(-(beta * beta), sigma, mu);
+                const double alpha = math::div_known(rho, sigma, math::recip_estimate(sigma));   /* = rho / sigma */
+                rho_prev = rho;
+                y_prev = math::recip_estimate(rho);
+#pragma unroll
+                for (int m = 0; m < U; m++) {
+                    p[m] = fma(beta, p[m], r[m]);
+                    pt[m] = fma(beta, pt[m], rt[m]);
+                    q[m] = fma(beta, q[m], w[m]);
+                    qt[m] = fma(beta, qt[m], wt[m]);
+                    x[m] = fma(alpha, p[m], x[m]);
+                    r[m] = fma(-alpha, q[m], r[m]);
+                    rt[m] = fma(-alpha, qt[m], rt[m]);
+                    ar[m] = fabs(r[m]);
+                }
+                done++;
+                if (grp_max_below<U, G>(S, ar, 1e-6)) { exited = true; break; }
+            }
+        }
         double rho, mu, sg, y1, pn[U], ptn[U], qn[U], qtn[U], xn[U], rn[U], rtn[U];
         bool small = false, proven = true, early = false;
         /* the iterates pn .. rtn that the quotients lead to, and a single warp's exit test on them */
@@ -766,7 +834,7 @@ __device__ __forceinline__ int bicg_iterate(const Sys<U, G>& S, const DeviceProb
             y_prev = y1;
             done++;
         };
-        if (max_iter >= 1) {
+        if (!IN_PLACE && max_iter >= 1) {
             for (;;) {
                 for (;;) {
                     iteration(Const<0>{});
@@ -1219,7 +1287,7 @@ __device__ __forceinline__ int coupled_rhs(const Sys<U, G>& S, const DeviceProbl
             }
         }
     };
-    const int done = bicg_iterate<U, G, REC>(S, P, bv, r, x, put, mul, capped);
+    const int done = bicg_iterate<U, G, REC, (U > 1)>(S, P, bv, r, x, put, mul, capped);
 #pragma unroll
     for (int m = 0; m < U; m++) F[m][IC] = x[m];
     return done;
@@ -1623,7 +1691,7 @@ __device__ __forceinline__ int coupled_rhs_sharedc(const Sys<U, G>& S, const Dev
             qt[m] = vld ? fma(x1[m], qts[m], vt[m]) : 0.0;
         }
     };
-    const int done = bicg_iterate<U, G, REC>(S, P, bv, r, x, put, mul, capped);
+    const int done = bicg_iterate<U, G, REC, (U > 1 && REC == 1)>(S, P, bv, r, x, put, mul, capped);
 #pragma unroll
     for (int m = 0; m < U; m++) F[m][IC] = x[m];
     return done;
