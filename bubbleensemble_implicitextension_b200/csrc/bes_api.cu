@@ -384,7 +384,8 @@ struct ClassLaunch {
 /* do the systems of up to 32 units run on teams */
 bool team_pays(const bes_solver* h) {
     return bes::team_pays(std::min(h->active, h->n_systems),
-                          h->shared_coupling && h->class_shared[0] && h->class_symmetric[0], h->sm_count);
+                          h->shared_coupling && h->class_shared[0] && h->class_symmetric[0], h->bicg_recurrence,
+                          h->sm_count);
 }
 
 bool sparse_pays(const bes_solver* h) {

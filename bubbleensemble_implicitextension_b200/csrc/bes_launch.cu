@@ -141,11 +141,13 @@ constexpr bool TEAM_MODEL = BES_MODEL_NGP == 0 && BES_MODEL_NIGP == 0 && BES_MOD
 
 /* Does a launch of `total` systems run those of up to 32 units on teams of four warps (where TEAM_MODEL
  * allows them)?  Eight warps of 255 registers are what an SM holds, and a team's warps repeat everything but
- * the products, so a system to an SM always gains (8 bubbles alone 33.0 -> 31.6 ms, 64 x 16 bubbles with RK4 17.4 -> 16.2),
- * two only with the shared symmetric matrix (256 x 32: 331 -> 324 and 325 -> 289 ms of two draws; own
- * matrix 322 -> 326), and beside multi-warp systems none (384 uneven clouds: 92 -> 112 ms). */
-bool team_pays(int total, bool symmetric, int sm_count) {
-    return TEAM_MODEL && total <= (symmetric ? 2 : 1) * sm_count;
+ * the products, so a system to an SM always gains (148 systems of 32 units, 250 steps: 5.3 -> 5.1 ms, with
+ * REC 1 5.6 -> 4.6).  Two gain only with the shared symmetric matrix and REC 1, whose iteration is the more
+ * product (256 x 32 to the end of a period, three draws: 353, 325, 321 -> 324, 293, 289 ms; with REC 0 350,
+ * 321, 318 -> 357, 322, 330; own matrix 322 -> 326), and beside multi-warp systems none (384 uneven clouds:
+ * 92 -> 112 ms). */
+bool team_pays(int total, bool symmetric, int rec, int sm_count) {
+    return TEAM_MODEL && total <= (symmetric && rec == 1 ? 2 : 1) * sm_count;
 }
 
 /* Does a launch of `total` systems, all of up to 32 units, keep the column share of W in tensor

@@ -60,8 +60,8 @@ bool sparse_pays(int count, int total, int sm_count);
 /* whether `count` systems of class cls > 0 run at sixteen warps an SM */
 bool dense_pays(int cls, int count, int sm_count);
 /* whether a launch of `total` systems runs those of up to 32 units on teams of four warps
- * (symmetric: they share one symmetric matrix) */
-bool team_pays(int total, bool symmetric, int sm_count);
+ * (symmetric: they share one symmetric matrix; rec: the BiCG recurrence) */
+bool team_pays(int total, bool symmetric, int rec, int sm_count);
 /* warps per CTA for `count` systems of variant v (requested > 0: that many,
  * clamped to what the variant allows and rounded down to a multiple of G) */
 int class_warps_per_block(Variant v, int count, int sm_count, int requested);

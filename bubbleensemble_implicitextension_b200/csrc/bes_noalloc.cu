@@ -154,7 +154,7 @@ extern "C" bes_status bes_solve_periods_noalloc(const bes_noalloc_problem* p, in
     for (int cls = 0; cls < 3; cls++) {
         if (count[cls] == 0) continue;
         var[cls] = bes::class_variant(cls, all32, false, 0, false, p->bicg_recurrence, 0,
-                                      bes::team_pays(count[0] + count[1] + count[2], false, sms));
+                                      bes::team_pays(count[0] + count[1] + count[2], false, p->bicg_recurrence, sms));
         const bes::Variant& v = var[cls];
         if (bes::max_warps_per_block(v) < v.G)
             return report(p, BES_ERR_CUDA, "bes_solve_periods_noalloc: kernel class %lld (%lld warps per system) does not fit in shared memory",

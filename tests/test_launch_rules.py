@@ -36,7 +36,7 @@ def run_rules(tmp_path, body, model="", lib=None, decl=""):
 
 TEAM_OF_EIGHT = f"""
     for (int sym = 0; sym < 2; sym++) {{
-        const Variant v = class_variant(0, false, sym, 0, sym, 0, 0, team_pays(8, sym, {SMS}));
+        const Variant v = class_variant(0, false, sym, 0, sym, 0, 0, team_pays(8, sym, 0, {SMS}));
         std::printf("%d/%d ", v.rhs, v.G);
     }}"""
 
@@ -53,6 +53,16 @@ def test_no_teams_for_models_too_large_for_four_copies(tmp_path):
 
 def test_teams_for_models_with_unit_values_only(tmp_path):
     assert run_rules(tmp_path, TEAM_OF_EIGHT) == ["11/4", "15/4"]
+
+
+def test_how_many_systems_run_on_teams(tmp_path):
+    """A system to an SM always; two with the shared symmetric matrix and the single-reduction recurrence."""
+    body = f"""
+    for (int rec = 0; rec < 2; rec++)
+        for (int sym = 0; sym < 2; sym++)
+            for (int total : {{{SMS}, {SMS + 1}, {2 * SMS}, {2 * SMS + 1}}})
+                std::printf("%d ", team_pays(total, sym, rec, {SMS}));"""
+    assert run_rules(tmp_path, body) == ["1", "0", "0", "0"] * 3 + ["1", "1", "1", "0"]
 
 
 # most banded systems of 33-64 and of 65-128 units to a CTA of eight warps, by band width: what the band, the
