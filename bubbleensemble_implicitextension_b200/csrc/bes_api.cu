@@ -1389,8 +1389,9 @@ bes_status bes_write_csv(bes_solver* h, int32_t kind, const char* path) {
 
 /* Launch-shape autotuner: for every non-empty size class, time each launch
  * shape the kernels allow (warps per system, then warps per CTA in powers of
- * two up to what shared memory and the launch bounds admit) on the device's
- * current inputs, from the same saved state each time, and keep the fastest.
+ * two up to what shared memory and the launch bounds admit; up to 32 units the
+ * latter only) on the device's current inputs, from the same saved state each
+ * time, and keep the fastest.
  * Every shape computes bit-identical results, so the choice changes speed
  * only.  The state, accessories, dense output and counters on the device are
  * restored afterwards; the host mirrors are not touched. */
@@ -1436,11 +1437,15 @@ bes_status bes_autotune(bes_solver* h, int32_t n_periods, int64_t step_cap, bes_
         if (h->class_count[cls] == 0) continue;
         float best = -1.0f;
         int best_wps = 0, best_wpb = 0;
-        const bool team = team_pays(h);
-        for (int wps = 0; wps <= (cls == 0 && !team ? 0 : 1) && !st; wps++) {
+        /* up to 32 units the choice between teams and one warp stays with team_pays (WarpsPerSystem 1 keeps
+         * it off): a capped run sees every system busy at once, where one warp each is ahead, and not the last
+         * long system alone on its SM, which sets the time of a whole period (256 x 32 with REC 1: 324 ms on teams,
+         * whose first 2000 steps take 48.1 ms, against 353 and 47.8 on one warp each) */
+        const int first_wps = cls == 0 && h->warps_per_system == 1 ? 1 : 0;
+        for (int wps = first_wps; wps <= (cls == 0 ? first_wps : 1) && !st; wps++) {
             const bes::Variant v = bes::class_variant(cls, h->class0_all32,
                                                       h->shared_coupling && h->class_shared[cls], wps,
-                                                      h->class_symmetric[cls], h->bicg_recurrence, h->cbw, team,
+                                                      h->class_symmetric[cls], h->bicg_recurrence, h->cbw, team_pays(h),
                                                       bes::dense_pays(cls, h->class_count[cls], h->sm_count),
                                                       sparse_pays(h));
             const int cap = bes::max_warps_per_block(v);

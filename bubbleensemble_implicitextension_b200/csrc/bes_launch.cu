@@ -141,8 +141,8 @@ constexpr bool TEAM_MODEL = BES_MODEL_NGP == 0 && BES_MODEL_NIGP == 0 && BES_MOD
 
 /* Does a launch of `total` systems run those of up to 32 units on teams of four warps (where TEAM_MODEL
  * allows them)?  Eight warps of 255 registers are what an SM holds, and a team's warps repeat everything but
- * the products, so a system to an SM always gains (148 systems of 32 units, 250 steps: 5.3 -> 5.1 ms, with
- * REC 1 5.6 -> 4.6).  Two gain only with the shared symmetric matrix and REC 1, whose iteration is the more
+ * the products, so a system to an SM always gains (148 systems of 32 units, 250 steps: 5.5 -> 5.1 ms, with
+ * REC 1 5.65 -> 4.7).  Two gain only with the shared symmetric matrix and REC 1, whose iteration is the more
  * product (256 x 32 to the end of a period, three draws: 353, 325, 321 -> 324, 293, 289 ms; with REC 0 350,
  * 321, 318 -> 357, 322, 330; own matrix 322 -> 326), and beside multi-warp systems none (384 uneven clouds:
  * 92 -> 112 ms). */

@@ -102,8 +102,10 @@ typedef int32_t bes_status;
 #define BES_OPT_USE_CUDA_GRAPH 103         /* 1 (default): bes_solve_periods captures its launches once into a
                                               CUDA graph and replays it; 0: direct launches */
 #define BES_OPT_WARPS_PER_SYSTEM 104       /* 0 (default): systems of 33-64 units run on 2 warps and of 65-128
-                                              units on 4 warps (one unit per lane); 1: one warp per system
-                                              (2 or 4 units per lane).  Results are bit-identical. */
+                                              units on 4 warps (one unit per lane), and launches of few systems
+                                              run those of up to 32 units on teams of 4 warps; 1: one warp per
+                                              system (2 or 4 units per lane above 32 units).  Results are
+                                              bit-identical. */
 #define BES_OPT_BICG_RECURRENCE 105        /* 0 (default): the reference's BiCG recurrence (Steppers.cuh:508-561:
                                               two reductions per iteration); 1: the single-reduction form of the
                                               same iterates (residual products first, rho = r.r~ and mu = r~.Ar
@@ -318,7 +320,7 @@ bes_status bes_write_csv(bes_solver* h, int32_t kind, const char* path);
  * BES_OPT_WARPS_PER_SYSTEM afterwards replaces the tuned choice. */
 typedef struct bes_autotune_result {
     int32_t warps_per_block[3];    /* per size class (N <= 32, <= 64, <= 128); 0 where the class is empty */
-    int32_t warps_per_system[3];   /* 0: 2 or 4 warps per system above 32 units, 1: one warp */
+    int32_t warps_per_system[3];   /* as BES_OPT_WARPS_PER_SYSTEM; up to 32 units that option's value */
     float ms[3];                   /* device time of the chosen shape */
     int32_t candidates;            /* shapes timed in all */
 } bes_autotune_result;

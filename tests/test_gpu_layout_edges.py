@@ -114,3 +114,20 @@ def test_unit_factors_are_refused_with_banded_storage(n, bw, systems, gpu):
             ps.solve_periods(1, -1)
     finally:
         ps.close()
+
+
+@pytest.mark.parametrize("wps", [0, 1])
+def test_autotuner_leaves_the_kernel_of_small_systems_to_the_rule(wps, gpu):
+    """A capped run is no measure of teams against one warp a system: only warps per CTA are tuned there (teams: 4
+    and 8 warps; one warp: 1, 2 and 4)."""
+    from bubbleensemble_implicitextension_b200 import solver as S
+    ens = _bounded(W.c1_ensemble(n_pa=2, n_f=2, n_units=32, factored=True), 50)
+    ps = ens.make_solver()
+    try:
+        ps.SolverOption(S.ListOfSolverOptions.WarpsPerSystem, wps)
+        ps.SynchroniseFromHostToDevice(S.ListOfVariables.All)
+        tuned = ps.autotune(n_periods=1, step_cap=20)
+        assert tuned["warps_per_system"][0] == wps
+        assert tuned["candidates"] == (3 if wps else 2)
+    finally:
+        ps.close()
