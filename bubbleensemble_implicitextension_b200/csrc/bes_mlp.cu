@@ -547,7 +547,7 @@ inline int blocks_for(int64_t n, int t) { return (int)((n + t - 1) / t); }
 
 struct bes_mlp {
     int device = 0;
-    int n_in = 0, width = 0, depth = 0, n_out = 0, max_batch = 0, n_layers = 0;
+    int n_in = 0, width = 0, depth = 0, n_out = 0, max_batch = 0, n_layers = 0, sm_count = 0;
     std::vector<int> fin, fout;
     std::vector<int64_t> w_off, b_off, wb_off; /* offsets in the parameter vector and in the BF16 weights */
     int64_t n_params = 0, n_wb = 0;
@@ -641,9 +641,8 @@ cudaError_t launch_rows(const NetView& v, const float* x, int batch, float* y, c
 
 /* rows a CTA: as many as still give every SM a tile (see mlp_rows) */
 template <bool TRAIN>
-cudaError_t rows_of(const NetView& v, const float* x, int batch, float* y, const float* target, float* err,
+cudaError_t rows_of(const NetView& v, int sms, const float* x, int batch, float* y, const float* target, float* err,
                     cudaStream_t s) {
-    const int sms = 148;   /* of a B200 */
     if (batch <= 4 * sms) return launch_rows<4, 1, TRAIN>(v, x, batch, y, target, err, s);
     if (batch <= 8 * sms) return launch_rows<4, 2, TRAIN>(v, x, batch, y, target, err, s);
     if (batch <= 16 * sms) return launch_rows<4, 4, TRAIN>(v, x, batch, y, target, err, s);
@@ -698,7 +697,11 @@ bes_status bes_mlp_create(const bes_mlp_config* c, bes_mlp** out) {
         h->wb_off.push_back(h->n_wb);
         h->n_wb += (int64_t)h->fin[l] * h->fout[l];
     }
-    if (cudaSetDevice(h->device) != cudaSuccess) { delete h; return BES_ERR_CUDA; }
+    if (cudaSetDevice(h->device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&h->sm_count, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess) {
+        delete h;
+        return BES_ERR_CUDA;
+    }
     /* host-side initialisation: uniform(-1, 1) * sqrt(6 / fan_in) (He-uniform), biases 0,
      * from a splitmix64 stream of the given seed */
     std::vector<float> w(h->n_params, 0.f);
@@ -821,7 +824,7 @@ bes_status bes_mlp_forward(bes_mlp* h, const float* x, int32_t batch, float* y, 
     if (!h || !x || !y || batch < 1 || batch > h->max_batch) return BES_ERR_ARGUMENT;
     MLP_TRY(h, cudaSetDevice(h->device));
     if (fused(h)) {
-        MLP_TRY(h, (rows_of<false>(view(h), x, batch, y, nullptr, nullptr, (cudaStream_t)stream)));
+        MLP_TRY(h, (rows_of<false>(view(h), h->sm_count, x, batch, y, nullptr, nullptr, (cudaStream_t)stream)));
         return BES_OK;
     }
     return forward(h, x, batch, y, (cudaStream_t)stream);
@@ -834,7 +837,7 @@ bes_status bes_mlp_backward(bes_mlp* h, const float* x, const float* target, int
     cudaStream_t s = (cudaStream_t)stream;
     if (fused(h)) {
         const NetView v = view(h);
-        MLP_TRY(h, (rows_of<true>(v, x, batch, nullptr, target, h->err, s)));
+        MLP_TRY(h, (rows_of<true>(v, h->sm_count, x, batch, nullptr, target, h->err, s)));
         GradPlan plan;
         std::memset(&plan, 0, sizeof plan);
         for (int l = 0; l < h->n_layers; l++) {
