@@ -27,8 +27,8 @@
  * the launch shares one matrix, it is staged once per CTA
  * instead; when that matrix is symmetric (a geometry 1/d with the radii as
  * unit factors), both products become row sums of the same entries -- read
- * once from tensor memory, or for N <= 32 held in registers for the whole
- * system.  Every scalar of the step control is uniform over the group
+ * once from tensor memory, or for N <= 32 held in registers for a right-hand
+ * side.  Every scalar of the step control is uniform over the group
  * and held in registers; a single-warp system needs no block barrier at all,
  * a multi-warp system one named barrier per reduction.
  *
@@ -989,14 +989,14 @@ __device__ __forceinline__ double quad_column_tree(const double* M, int col0, in
  * order of t, four columns each.  A chunk is loaded while the one before is
  * used; its latency is some 130 cycles, so chunks of eight doubles (40 cycles of
  * work) were slower than shared memory, and the loop is unrolled over all of
- * NMAX (guards on the chunks spilled registers).  The FP64 pipe is the bound now; shared memory's 128 bytes a clock were
- * (N = 128: 1540 of the 2070 cycles of a product).  Cycles per BiCG iteration of
- * a lone system on a B200: own matrix, N = 101: 3610 -> 2040, N = 48: 1780 ->
- * 1410; shared symmetric matrix, N = 128: 2900 -> 1960 (two on an SM: 4290 ->
- * 2660), N = 51: 1740 -> 1430. *
+ * NMAX (guards on the chunks spilled registers).  Shared memory's 128 bytes a
+ * clock were the bound before (N = 128: 1540 of the 2070 cycles of a product).
+ * Cycles per BiCG iteration of a lone system on a B200: own matrix, N = 101:
+ * 3610 -> 2040, N = 48: 1780 -> 1410; shared symmetric matrix, N = 128: 2900 ->
+ * 1960 (two on an SM: 4290 -> 2660), N = 51: 1740 -> 1430. */
 
-/* sums of this lane's row share against K posted vectors, entry j of vector k at v[K j + k];
- * the entries from N to the next multiple of 8 are zeros */
+/* sums of this lane's row share against K posted vectors, entry j of vector k at v[K j + k]; all NMAX
+ * columns are read, so the matrix and the vectors hold zeros from N to NMAX */
 template <int K, int NMAX>
 __device__ __forceinline__ void tmem_row_sums(uint32_t addr, int c, const double* v, double (&out)[K]) {
     double s[K][4];
@@ -1038,7 +1038,7 @@ __host__ __device__ constexpr int tree_leaf(int m, int T) {
     return t;
 }
 
-/* halving tree of this lane's column share against a posted vector, over the NMAX (zero-padded) rows */
+/* halving tree of this lane's column share against a posted vector, over all NMAX rows (zeros from N on) */
 template <int NMAX>
 __device__ __forceinline__ double tmem_column_tree(uint32_t addr, int c, const double* v) {
     constexpr int T = NMAX / 4, CH = T / 4;
@@ -1553,25 +1553,25 @@ __device__ __forceinline__ int coupled_rhs_sharedc(const Sys<U, G>& S, const Dev
         if constexpr (U == 1) {
             const double* const vec[1] = {reinterpret_cast<const double*>(v2)};
             quad_row_sums<LDC, 1>(S.W, row0, c, N, vec, out);
-            return;
-        }
-        double a0[U], a1[U], a2[U], a3[U];
+        } else {
+            double a0[U], a1[U], a2[U], a3[U];
 #pragma unroll
-        for (int m = 0; m < U; m++) { a0[m] = 0.0; a1[m] = 0.0; a2[m] = 0.0; a3[m] = 0.0; }
+            for (int m = 0; m < U; m++) { a0[m] = 0.0; a1[m] = 0.0; a2[m] = 0.0; a3[m] = 0.0; }
 #pragma unroll 4
-        for (int j = 0; j < NMAX; j += 4) {
-            const double2 va = v2[j / 2], vb = v2[j / 2 + 1];
+            for (int j = 0; j < NMAX; j += 4) {
+                const double2 va = v2[j / 2], vb = v2[j / 2 + 1];
 #pragma unroll
-            for (int m = 0; m < U; m++) {
-                const double* Crow = S.W + S.unit(m);
-                if (j < N) a0[m] = fma(Crow[j * LDC], va.x, a0[m]);
-                if (j + 1 < N) a1[m] = fma(Crow[(j + 1) * LDC], va.y, a1[m]);
-                if (j + 2 < N) a2[m] = fma(Crow[(j + 2) * LDC], vb.x, a2[m]);
-                if (j + 3 < N) a3[m] = fma(Crow[(j + 3) * LDC], vb.y, a3[m]);
+                for (int m = 0; m < U; m++) {
+                    const double* Crow = S.W + S.unit(m);
+                    if (j < N) a0[m] = fma(Crow[j * LDC], va.x, a0[m]);
+                    if (j + 1 < N) a1[m] = fma(Crow[(j + 1) * LDC], va.y, a1[m]);
+                    if (j + 2 < N) a2[m] = fma(Crow[(j + 2) * LDC], vb.x, a2[m]);
+                    if (j + 3 < N) a3[m] = fma(Crow[(j + 3) * LDC], vb.y, a3[m]);
+                }
             }
-        }
 #pragma unroll
-        for (int m = 0; m < U; m++) out[m] = (a0[m] + a1[m]) + (a2[m] + a3[m]);
+            for (int m = 0; m < U; m++) out[m] = (a0[m] + a1[m]) + (a2[m] + a3[m]);
+        }
     };
     /* the same row sums for two vectors at once: each matrix entry read from
      * shared memory once (the kernel is bound by shared-memory reads), the
@@ -1583,43 +1583,43 @@ __device__ __forceinline__ int coupled_rhs_sharedc(const Sys<U, G>& S, const Dev
             quad_row_sums<LDC, 2>(S.W, row0, c, N, vec, o);   /* the right-hand side's sums only */
             outv[0] = o[0];
             outw[0] = o[1];
-            return;
-        }
-        double a0[U], a1[U], a2[U], a3[U], b0[U], b1[U], b2[U], b3[U];
-#pragma unroll
-        for (int m = 0; m < U; m++) {
-            a0[m] = 0.0; a1[m] = 0.0; a2[m] = 0.0; a3[m] = 0.0;
-            b0[m] = 0.0; b1[m] = 0.0; b2[m] = 0.0; b3[m] = 0.0;
-        }
-#pragma unroll 2
-        for (int j = 0; j < NMAX; j += 4) {
-            const double2 va = v2[j / 2], vb = v2[j / 2 + 1];
-            const double2 wa = w2[j / 2], wb = w2[j / 2 + 1];
+        } else {
+            double a0[U], a1[U], a2[U], a3[U], b0[U], b1[U], b2[U], b3[U];
 #pragma unroll
             for (int m = 0; m < U; m++) {
-                const double* Crow = S.W + S.unit(m);
-                if (j < N) { const double c = Crow[j * LDC]; a0[m] = fma(c, va.x, a0[m]); b0[m] = fma(c, wa.x, b0[m]); }
-                if (j + 1 < N) {
-                    const double c = Crow[(j + 1) * LDC];
-                    a1[m] = fma(c, va.y, a1[m]);
-                    b1[m] = fma(c, wa.y, b1[m]);
-                }
-                if (j + 2 < N) {
-                    const double c = Crow[(j + 2) * LDC];
-                    a2[m] = fma(c, vb.x, a2[m]);
-                    b2[m] = fma(c, wb.x, b2[m]);
-                }
-                if (j + 3 < N) {
-                    const double c = Crow[(j + 3) * LDC];
-                    a3[m] = fma(c, vb.y, a3[m]);
-                    b3[m] = fma(c, wb.y, b3[m]);
+                a0[m] = 0.0; a1[m] = 0.0; a2[m] = 0.0; a3[m] = 0.0;
+                b0[m] = 0.0; b1[m] = 0.0; b2[m] = 0.0; b3[m] = 0.0;
+            }
+#pragma unroll 2
+            for (int j = 0; j < NMAX; j += 4) {
+                const double2 va = v2[j / 2], vb = v2[j / 2 + 1];
+                const double2 wa = w2[j / 2], wb = w2[j / 2 + 1];
+#pragma unroll
+                for (int m = 0; m < U; m++) {
+                    const double* Crow = S.W + S.unit(m);
+                    if (j < N) { const double c = Crow[j * LDC]; a0[m] = fma(c, va.x, a0[m]); b0[m] = fma(c, wa.x, b0[m]); }
+                    if (j + 1 < N) {
+                        const double c = Crow[(j + 1) * LDC];
+                        a1[m] = fma(c, va.y, a1[m]);
+                        b1[m] = fma(c, wa.y, b1[m]);
+                    }
+                    if (j + 2 < N) {
+                        const double c = Crow[(j + 2) * LDC];
+                        a2[m] = fma(c, vb.x, a2[m]);
+                        b2[m] = fma(c, wb.x, b2[m]);
+                    }
+                    if (j + 3 < N) {
+                        const double c = Crow[(j + 3) * LDC];
+                        a3[m] = fma(c, vb.y, a3[m]);
+                        b3[m] = fma(c, wb.y, b3[m]);
+                    }
                 }
             }
-        }
 #pragma unroll
-        for (int m = 0; m < U; m++) {
-            outv[m] = (a0[m] + a1[m]) + (a2[m] + a3[m]);
-            outw[m] = (b0[m] + b1[m]) + (b2[m] + b3[m]);
+            for (int m = 0; m < U; m++) {
+                outv[m] = (a0[m] + a1[m]) + (a2[m] + a3[m]);
+                outw[m] = (b0[m] + b1[m]) + (b2[m] + b3[m]);
+            }
         }
     };
     double bsum[U], asum[U];
@@ -1920,7 +1920,7 @@ __device__ __forceinline__ int coupled_rhs_team(const Sys<1>& S, const DevicePro
     const double2* vp2 = reinterpret_cast<const double2*>(S.vp) + h;
     const double2* tp2 = reinterpret_cast<const double2*>(S.tpar + h * RED_RUN);
     const int tslot = par_slot(i);
-    double w[16];   /* this lane's 16 entries of G or of W */
+    double w[16] = {};   /* this lane's 16 entries of G or of W */
     /* this warp's chains of row i of w against the vector posted at vp */
     auto row_part = [&]() -> double {
         double s[2] = {0.0, 0.0};
@@ -1944,8 +1944,6 @@ __device__ __forceinline__ int coupled_rhs_team(const Sys<1>& S, const DevicePro
         S.vcpt[i] = cp;
         S.rdpar[tslot] = rd;
         __syncwarp();
-#pragma unroll
-        for (int k = 0; k < 16; k++) w[k] = 0.0;
         const double* C = S.W;   /* C[i][j] at i + j * LDC, zero-padded */
         double bs[2] = {0.0, 0.0}, as[2] = {0.0, 0.0};
         if (!second) {
@@ -2744,18 +2742,21 @@ __device__ __forceinline__ void analysis_period_end(const Sys<U, G>& S, const De
 
 /* ---------------------------------------------------------------------------
  * The kernel: groups of G warps pull systems from the work counter.
- * RHS = 0: operator W in shared memory; RHS = 1 / 2: operator in registers
- * (U = 1, G = 1; 2 = every system of the launch has exactly 32 units);
- * RHS = 3: every system of the launch shares one coupling matrix, staged once
- * per CTA (up to 8 warps per CTA), RHS = 4 the same for a symmetric matrix
- * (both BiCG products as row sums from one read of each entry).  G > 1 runs
- * one unit per lane (U = 1) and
- * exchanges the group's values through shared memory and a named barrier per
- * system slot (barrier 0 is left to __syncthreads).  RHS 7 and 10 are the banded
- * operator of narrow and of wide bands.  RHS 8 and 9 are RHS 1 and 2
- * with the column share of W in tensor memory.  V > 20 is RHS V - 20 compiled
- * for sixteen warps an SM (128 registers a thread), V = RHS otherwise.  RHS > 10 runs the variant
- * RHS - 10 of a system of up to 32 units on a team of warps (coupled_rhs_team). */
+ * G > 1 runs one unit per lane (U = 1) and exchanges the group's values through
+ * shared memory and a named barrier per system slot (barrier 0 is left to
+ * __syncthreads).
+ * RHS = 0: operator W of the system's own matrix, in tensor memory (G > 1) or in
+ * shared memory (several units a lane on one warp); RHS = 1 / 2: U = 1, G = 1,
+ * half of W in registers, the column share in shared memory (2 = every system of
+ * the launch has exactly 32 units), RHS = 8 / 9 the same with the column share in
+ * tensor memory; RHS = 3: every system of the launch shares one coupling matrix,
+ * staged in shared memory once per CTA (up to 8 warps per CTA), RHS = 4 the same
+ * for a symmetric matrix (both BiCG products as row sums from one read of each
+ * entry), in tensor memory for U = 1; RHS = 5 / 6: as 1 / 2 for a shared
+ * symmetric matrix; RHS = 7 and 10: the banded operator of narrow and of wide
+ * bands; 10 < RHS < 17: the variant RHS - 10 of a system of up to 32 units on a
+ * team of warps (coupled_rhs_team).  V > 20 is RHS V - 20 compiled for sixteen
+ * warps an SM (128 registers a thread), V = RHS otherwise. */
 template <int U, int V, int G, int REC>
 __global__ void __launch_bounds__(V > 20 ? 512 : V == 3 || V == 4 || V == 7 || V >= 10 || G > 1 ? 256 : 128, 1)
     bes_ensemble_kernel(DeviceProblem P) {

@@ -76,7 +76,7 @@ size_t cta_smem_bytes(Variant v, int warps) {
 }
 
 int max_warps_per_block(Variant v) {
-    /* the kernels' launch bounds: 256 threads with RHS 3 or G > 1, else 128 */
+    /* the kernels' launch bounds: 512 threads for RHS > 20, 256 with a shared or banded matrix or G > 1, else 128 */
     const int cap = v.rhs > 20 ? 16 : (v.rhs == 3 || v.rhs == 4 || v.rhs == 7 || v.rhs == 10 || v.G > 1) ? 8 : 4;
     int w = 0;
     while (w + v.G <= cap && cta_smem_bytes(v, w + v.G) <= (size_t)SMEM_MAX) w += v.G;
@@ -95,13 +95,13 @@ cudaError_t launch(Variant v, const DeviceProblem& P, int grid, int warps, cudaS
     return e;
 }
 
-/* kernel variant of a units class: N <= 32 keeps the operator in registers
- * (rhs 2: every system has exactly 32 units); larger N runs one unit per lane
- * on 2 or 4 warps (or 2 or 4 units per lane on one warp) with W in shared
- * memory, or one staged copy of a matrix shared by the whole class when the
- * caller asked for shared coupling matrices (SharedCouplingMatrices); team asks
- * for four warps a system of up to 32 units (see team_pays).  With
- * banded coupling storage (band > 0) every class whose matrix is not staged
+/* kernel variant of a units class: N <= 32 keeps half of the operator in
+ * registers (rhs 2: every system has exactly 32 units); larger N runs one unit
+ * per lane on 2 or 4 warps with W in tensor memory (or 2 or 4 units per lane on
+ * one warp with W in shared memory), or one staged copy of a matrix shared by the
+ * whole class when the caller asked for shared coupling matrices
+ * (SharedCouplingMatrices).  team, dense and sparse are what team_pays, dense_pays
+ * and sparse_pays say of the launch.  With banded coupling storage (band > 0) every class whose matrix is not staged
  * as a shared symmetric (N <= 32) or shared (N > 32) matrix runs the banded
  * operator, one unit per lane on 1, 2 or 4 warps. */
 Variant class_variant(int cls, bool all32, bool shared, int warps_per_system, bool symmetric, int rec, int band,

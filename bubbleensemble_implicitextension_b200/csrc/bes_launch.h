@@ -3,18 +3,19 @@
  *
  * Variant (U, RHS, G): G warps per system with U units per lane (single warp:
  * U = 1, 2, 4 for N <= 32, 64, 128; multi-warp: U = 1 with G = 2, 4 for
- * N <= 64, 128).  RHS 0 keeps the operator in shared memory, RHS 1 keeps it
- * in registers (U = G = 1), RHS 2 is RHS 1 for launches whose systems all
- * have 32 units, RHS 3 stages one coupling matrix shared by the whole launch
- * per CTA (64 or 128 units), RHS 4 is RHS 3 for a symmetric shared matrix
- * (both BiCG products as row sums from one shared-memory read); RHS 5 / 6
- * (U = G = 1, N <= 32) keep a row of a shared symmetric matrix in registers
- * (6: every system has 32 units); RHS 7 (U = 1) keeps only the wrapping
- * band of banded coupling storage (CBW > 0), RHS 10 one of more than eight
- * diagonals; RHS 11, 12, 15, 16 with G = 4 are
+ * N <= 64, 128).  RHS 0 keeps the operator of the system's own matrix in tensor
+ * memory (G > 1) or shared memory (one warp, several units a lane); RHS 1 keeps
+ * half of it in registers and half in shared memory (U = G = 1), RHS 2 is RHS 1
+ * for launches whose systems all have 32 units, RHS 8 and 9 are RHS 1 and 2 with
+ * that half in tensor memory; RHS 3 stages one coupling matrix shared by the
+ * whole launch per CTA (64 or 128 units), RHS 4 is RHS 3 for a symmetric shared
+ * matrix (both BiCG products as row sums from one read, from tensor memory for
+ * U = 1); RHS 5 / 6 (U = G = 1, N <= 32) take a lane's share of a shared symmetric
+ * matrix into registers for a right-hand side (6: every system has 32 units);
+ * RHS 7 (U = 1) keeps only the wrapping band of banded coupling storage (CBW > 0),
+ * RHS 10 one of more than eight diagonals; RHS 11, 12, 15, 16 with G = 4 are
  * RHS 1, 2, 5, 6 on a team of four warps a system; RHS 24 and 27 are RHS 4 and 7
- * compiled for sixteen warps an SM; RHS 8 and 9 are RHS 1 and 2 with a share of
- * the operator in tensor memory.  Every variant exists with both BiCG
+ * compiled for sixteen warps an SM.  Every variant exists with both BiCG
  * recurrences (REC 0: the reference's; 1: the single-reduction form). */
 #ifndef BES_LAUNCH_H
 #define BES_LAUNCH_H
