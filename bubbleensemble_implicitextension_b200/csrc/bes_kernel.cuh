@@ -82,7 +82,7 @@ constexpr int RED_RUN = 18, RED_BUF = 2 * RED_RUN;
 constexpr int SMEM_MAX = 227 * 1024;
 /* stage derivatives of a system of NMAX units (one unit per lane) that go to shared memory beside
  * `others` doubles, `systems` times in a CTA, if that fits: a model of many parameters or components
- * may leave no room, and then they stay in registers */
+ * may leave no room, and then they are in local memory */
 __host__ __device__ constexpr int stage_doubles(int nmax, long others, int systems = 1) {
     return 8L * systems * ((others + 6 * UD * nmax + 31) / 32 * 32) <= SMEM_MAX ? 6 * UD * nmax : 0;
 }
@@ -2231,7 +2231,10 @@ __device__ constexpr bool stages_shared() {
 
 /* The stage derivatives K_j of this lane's units: SHARED in shared memory (each
  * is written once and read a few times a step, while the BiCG needs the
- * registers), else in registers. */
+ * registers).  Else, with one unit per lane, in local memory for the same reason
+ * (wide bands with REC 1 lack registers: 512 systems of 128 units, CBW 8, 100
+ * steps 15.9 ms in registers, 14.2 so; 148 of 60 units, CBW 4, 5.8 and 4.3); with
+ * several in registers. */
 template <int U, int G, int J, bool SHARED>
 struct Stages {
     double k[SHARED ? 1 : J][U][UD];
@@ -2239,6 +2242,9 @@ struct Stages {
         if constexpr (SHARED) {
 #pragma unroll
             for (int c = 0; c < UD; c++) S.ks[(st * UD + c) * 32 * G + S.unit(0)] = F[0][c];
+        } else if constexpr (U == 1) {
+#pragma unroll
+            for (int c = 0; c < UD; c++) k[st][0][c] = F[0][c];   /* st varies at run time: local memory */
         } else {
 #pragma unroll
             for (int j = 0; j < J; j++)

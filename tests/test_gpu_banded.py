@@ -7,6 +7,7 @@ the system (every column once, in band order)."""
 import numpy as np
 import pytest
 
+from bubbleensemble_implicitextension_b200 import solver as S
 from bubbleensemble_implicitextension_b200 import workloads as W
 from tests.helpers import assert_bitwise, run_gpu
 
@@ -48,4 +49,16 @@ def test_wide_bands_match_oracle(n, bw, rec, gpu, oracle_lib):
     ens.max_steps_per_period = 200
     got = run_gpu(ens, n_periods=1, reset_at=-1, bicg_recurrence=rec)
     want = oracle_lib.run(ens, n_periods=1, reset_at=-1, bicg_variant=rec)
+    assert_bitwise(got, want, KEYS)
+
+
+@pytest.mark.parametrize("rec", [0, 1])
+@pytest.mark.parametrize("n,bw", [(17, 5), (40, 6), (101, 9)])
+def test_wide_bands_rk4_match_oracle(n, bw, rec, gpu, oracle_lib):
+    """The fixed-step method keeps its stage derivatives as the adaptive one does."""
+    ens = W.ring_ensemble(n_systems=3, n_units=n, band_width=bw)
+    ens.dt0 = 2e-3
+    ens.max_steps_per_period = 200
+    got = run_gpu(ens, n_periods=1, reset_at=-1, algorithm=S.Algorithms.RK4, bicg_recurrence=rec)
+    want = oracle_lib.run(ens, n_periods=1, reset_at=-1, algorithm=0, bicg_variant=rec)
     assert_bitwise(got, want, KEYS)
